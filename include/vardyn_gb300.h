@@ -86,8 +86,9 @@ typedef struct vd_qg1l_schedule {
     int tc_group_fwd;    /* 32-column output tiles per CTA of the forward
                             tensor-core pass: 0 rule, or 1, 2, 4, 8 */
     int tc_group_inv;    /* the same for the inverse pass */
-    int fma_rows;        /* rows per CTA of the FMA pass: 0 rule, 16, 32 or
-                            64 (float32) */
+    int fma_rows;        /* rows per CTA of the float32 FMA pass: 0 rule, 16,
+                            32 or 64 (float64 plans accept 16 and 32 and keep
+                            their own rule) */
     int tridiag_rows;    /* rows per thread of the tridiagonal solve: 0 rule,
                             8, 16 or 32 (used when the field fits, else the
                             rule) */

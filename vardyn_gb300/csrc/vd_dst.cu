@@ -36,16 +36,6 @@ template <> struct Vec8<float> {
         r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
     }
 };
-template <> struct Vec8<double> {
-    static __device__ __forceinline__ void load(const double* p, double (&r)[8]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            double2 a = reinterpret_cast<const double2*>(p)[i];
-            r[2 * i] = a.x; r[2 * i + 1] = a.y;
-        }
-    }
-};
-
 struct GemmGeom {
     int n, ne, no, my, nx;
     long long fs;
@@ -214,6 +204,112 @@ dst_gemm_kernel(GemmGeom g, const T* __restrict__ W1, const T* __restrict__ W2,
                             out[o] = (mask[mi] == 3) ? ys[u] + add[o] : T(0);
                         }
                     }
+                }
+            }
+        }
+    }
+}
+
+// Dense form of the float64 pass. The part runs 2 FP64 FMAs a clock and SM, one
+// warp instruction per 64 clocks on each of an SM's four schedulers, so the
+// kernel is bound by the FP64 pipe as soon as every scheduler holds a warp:
+// operands are read straight from L1 / L2 (one W load per R FMAs), and the work
+// is cut finely enough to fill all 608 schedulers even for one 128^2 field.
+// A warp owns 32 output columns of one half (even-k or odd-k sums) of R rows;
+// a CTA's 8 warps are both halves x CWC column groups x 4/CWC row groups over
+// the butterflied rows in shared memory. Measured on one 128^2 field: the whole
+// solve 34 us, against 340 us with the 8 x 8 register tile of the float32 kernel
+// (8 CTAs of two warps a pass); 119 us on one 384^2 field.
+template <int R, int CWC, int MODE, int EPI>
+__global__ void __launch_bounds__(256)
+dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __restrict__ W2,
+                   const double* __restrict__ src, const double* __restrict__ sub, int sub_batches,
+                   double* __restrict__ spec, double* __restrict__ out, const double* __restrict__ add,
+                   int add_batches, const int8_t* __restrict__ mask)
+{
+    constexpr int RG = 4 / CWC, TR = R * RG, NC = 32 * CWC;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* As = reinterpret_cast<double*>(smem_raw);    // [ne][TR]
+    double* Bs = As + (size_t)g.ne * TR;                 // [no][TR]
+    const int n = g.n, ne = g.ne, no = g.no, my = g.my;
+    const int row0 = blockIdx.y * TR, c0 = blockIdx.x * NC;
+
+    for (int idx = threadIdx.x; idx < ne * TR; idx += 256) {
+        const int r = idx / ne, p = idx - r * ne;
+        const int row = row0 + r;
+        double a = 0.0, b = 0.0;
+        if (row < g.R) {
+            if (MODE == MODE_FWD) {
+                const int f = row / my;
+                const long long o = f * g.fs + (long long)(row - f * my + 1) * g.nx + 1;
+                const bool hs = sub != nullptr && f < sub_batches;
+                const double x1 = src[o + p] - (hs ? sub[o + p] : 0.0);
+                if (p < no) {
+                    const double x2 = src[o + n - 1 - p] - (hs ? sub[o + n - 1 - p] : 0.0);
+                    a = x1 + x2;
+                    b = x1 - x2;
+                } else {
+                    a = x1;   // middle point of an odd-length transform
+                }
+            } else {
+                const double* s = spec + (long long)row * g.lds;
+                a = s[p];
+                if (p < no) b = s[ne + p];
+            }
+        }
+        As[p * TR + r] = a;
+        if (p < no) Bs[p * TR + r] = b;
+    }
+    __syncthreads();
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int half = warp >> 2, cw = (warp & 3) % CWC, rg = (warp & 3) / CWC;
+    const int t = c0 + cw * 32 + lane;                   // < ldw: the tables' rows are zero-padded
+    const int K = half == 0 ? ne : no;
+    const double* __restrict__ W = (half == 0 ? W1 : W2) + t;
+    const double* __restrict__ X = (half == 0 ? As : Bs) + rg * R;
+    double acc[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) acc[i] = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) {
+        const double w = __ldg(W + (size_t)k * g.ldw);
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fma(X[k * TR + i], w, acc[i]);
+    }
+
+    if (MODE == MODE_FWD) {
+        if (t < K) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int row = row0 + rg * R + i;
+                if (row < g.R) spec[(long long)row * g.lds + (half == 0 ? 0 : ne) + t] = acc[i];
+            }
+        }
+    } else {
+        // y[p] = A + B, y[n-1-p] = A - B: the odd-half warps hand over B
+        __shared__ double ex[4][R][32];
+        if (half == 1) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) ex[warp & 3][i][lane] = acc[i];
+        }
+        __syncthreads();
+        if (half == 0 && t < ne) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int row = row0 + rg * R + i;
+                if (row >= g.R) break;
+                const int f = row / my, j = row - f * my + 1;
+                const long long base = f * g.fs + (long long)j * g.nx + 1;
+                const double B = t < no ? ex[warp][i][lane] : 0.0;
+                const double ys[2] = {acc[i] + B, acc[i] - B};
+                const int ps[2] = {t, n - 1 - t};
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (u == 1 && t >= no) break;
+                    const long long o = base + ps[u];
+                    if (EPI == EPI_H) out[o] = ys[u] + ((add != nullptr && f < add_batches) ? add[o] : 0.0);
+                    else out[o] = (mask[j * g.nx + 1 + ps[u]] == 3) ? ys[u] + add[o] : 0.0;
                 }
             }
         }
@@ -405,7 +501,8 @@ tridiag_global_kernel(T* __restrict__ spec, const T* __restrict__ trim, int my, 
 // FFT is a Stockham autosort (each stage reads v_r = x[j + r L/R], applies the
 // twiddles e^{-2 pi i k r / (Ns R)} with k = j mod Ns, takes the length-R DFT
 // and writes y[(j/Ns) Ns R + k + r Ns]; the output is in natural order) with
-// radix 4, 2, 3 and 5 stages, ping-ponging between two shared-memory buffers.
+// radix 4, 2, 3 and 5 stages and direct stages of other odd radices,
+// ping-ponging between two shared-memory buffers.
 // The orthonormal DST-I is its own inverse, so the inverse pass is the same
 // transform from the parity-split spectral rows to the field.
 // ---------------------------------------------------------------------------
@@ -509,6 +606,81 @@ __device__ __forceinline__ void fft_stage(const double2* __restrict__ in, double
     }
 }
 
+// A stage of any odd radix p >= 7 (a prime factor of n + 1), as a direct
+// length-p DFT by pairs: with t_q = v_q + v_{p-q}, d_q = v_q - v_{p-q},
+//   y_r, y_{p-r} = v_0 + sum_q cos(2 pi q r/p) t_q  -/+  i sum_q sin(2 pi q r/p) d_q.
+// A first pass writes t_q and d_q over v_q and v_{p-q} in place (with the
+// stage's twiddles); then one thread forms one output pair of one butterfly,
+// 4 FP64 FMAs per q. The pass is bound by the FP64 pipe (2 FMA a clock and
+// SM), not by the shared-memory reads of t and d.
+// FIRST (Ns = 1, the input still the odd extension z_{L-m} = -z_m): butterfly
+// T - j holds minus the reversed inputs of butterfly j, so its outputs are
+// -e^{2 pi i r/p} y_{p-r}: half of the butterflies need no sums.
+// Measured: 4 x 256^2 (n + 1 = 3 5 17) 28 us a pass (dense float32-style tile
+// 300 us), one 512^2 field (7 73) 110 us a solve, 291 us with dense products.
+template <bool FIRST>
+__device__ __forceinline__ void fft_stage_odd(double2* __restrict__ in, double2* __restrict__ out,
+                                              const double2* __restrict__ tw, int L, int Ns, int pp, int p)
+{
+    const int T = L / p, h = p >> 1;
+    const int tstep = FIRST ? 0 : L / (Ns * p);
+    const int nb = FIRST ? T / 2 + 1 : T;      // butterflies computed (L is even and p odd: T is even)
+    for (int idx = threadIdx.x; idx < pp * nb * h; idx += blockDim.x) {
+        const int bq = idx / nb, j = idx - bq * nb;
+        const int q = bq % h + 1;
+        double2* I = in + (long long)(bq / h) * L + j;
+        double2 a = I[q * T], b = I[(p - q) * T];
+        if (!FIRST) {
+            const int k = j % Ns;
+            a = cmul(a, __ldg(tw + (long long)k * q * tstep));
+            b = cmul(b, __ldg(tw + (long long)k * (p - q) * tstep));
+        }
+        I[q * T] = cadd(a, b);
+        I[(p - q) * T] = csub(a, b);
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < pp * nb * (h + 1); idx += blockDim.x) {
+        const int br = idx / nb, j = idx - br * nb;
+        const int r = br % (h + 1);
+        const double2* I = in + (long long)(br / (h + 1)) * L + j;
+        double2* O = out + (long long)(br / (h + 1)) * L;
+        double2 C = I[0], S = make_double2(0.0, 0.0);
+        if (r == 0) {
+            for (int q = 1; q <= h; ++q) C = cadd(C, I[q * T]);
+        } else {
+            int m = 0;
+            for (int q = 1; q <= h; ++q) {
+                m += r * T;                    // (q r mod p) T
+                if (m >= L) m -= L;
+                const double2 w = __ldg(tw + m);   // cos, -sin
+                const double2 t = I[q * T], d = I[(p - q) * T];
+                C.x = fma(w.x, t.x, C.x);
+                C.y = fma(w.x, t.y, C.y);
+                S.x = fma(w.y, d.x, S.x);
+                S.y = fma(w.y, d.y, S.y);
+            }
+        }
+        // S holds -sum sin d: y_r = C + i S, y_{p-r} = C - i S
+        const double2 yr = make_double2(C.x - S.y, C.y + S.x), yp = make_double2(C.x + S.y, C.y - S.x);
+        if (FIRST) {
+            O[j * p + r] = yr;
+            if (r) O[j * p + p - r] = yp;
+            if (j > 0 && j < T / 2) {
+                const double2 w = __ldg(tw + r * T);            // e^{-2 pi i r/p}
+                const double2 a = cmul(yp, make_double2(w.x, -w.y)), b = cmul(yr, w);
+                double2* M = O + (T - j) * p;
+                M[r] = make_double2(-a.x, -a.y);
+                if (r) M[p - r] = make_double2(-b.x, -b.y);
+            }
+        } else {
+            const int k = j % Ns;
+            const int base = (j / Ns) * Ns * p + k;
+            O[base + r * Ns] = yr;
+            if (r) O[base + (p - r) * Ns] = yp;
+        }
+    }
+}
+
 // One CTA: g.pp pairs of rows (2 g.pp consecutive rows of the R row list).
 template <int MODE, int EPI>
 __global__ void __launch_bounds__(256)
@@ -558,7 +730,11 @@ dst_fft_kernel(FftGeom g, const double2* __restrict__ tw, const double* __restri
             case 4: fft_stage<4>(b0, b1, tw, L, Ns, g.pp); break;
             case 2: fft_stage<2>(b0, b1, tw, L, Ns, g.pp); break;
             case 3: fft_stage<3>(b0, b1, tw, L, Ns, g.pp); break;
-            default: fft_stage<5>(b0, b1, tw, L, Ns, g.pp); break;
+            case 5: fft_stage<5>(b0, b1, tw, L, Ns, g.pp); break;
+            default:
+                if (Ns == 1) fft_stage_odd<true>(b0, b1, tw, L, Ns, g.pp, R);
+                else fft_stage_odd<false>(b0, b1, tw, L, Ns, g.pp, R);
+                break;
         }
         __syncthreads();
         double2* t = b0; b0 = b1; b1 = t;
@@ -601,6 +777,10 @@ size_t spec_bytes(const vd_qg1l_plan* p, int nf)
     return size_t(nf) * p->dst.my * p->dst.lds * elem_size(p->d.dtype);
 }
 
+// Measured cost of an FP64 instruction of the FFT form over one of the dense
+// form (index arithmetic, barriers between stages).
+constexpr double FFT_OVER_DENSE = 1.3;
+
 template <typename T>
 static int upload(const std::vector<double>& h, void** d)
 {
@@ -610,18 +790,43 @@ static int upload(const std::vector<double>& h, void** d)
     return VD_OK;
 }
 
-// FFT radices for L = 2(n+1) (radix 4 first, then 2, 3, 5); false when L has
-// another prime factor or its buffers do not fit shared memory.
+// FFT radices for L = 2(n+1): the odd primes above 5 first, largest first (the
+// first stage's odd symmetry halves its direct sums), then radix 4, 2, 3, 5.
+// False when the buffers do not fit shared memory or the dense form needs
+// fewer FP64 operations. Both forms are bound by the FP64 pipe, so the line is
+// drawn on FP64 instructions a row: ne^2 + no^2 FMAs dense; for the FFT, half of
+// L times the per-point cost of its stages (a row pair shares a transform).
+// Lengths that factor into 2, 3, 5 always take the FFT. Measured solves, FFT /
+// dense: n + 1 = 63 27 / 24 us, 127 50 / 34, 159 37 / 42, 191 (7 fields) 283 /
+// 140, 255 (4 fields) 69 / 152, 447 156 / 194, 1023 279 / 1839; the rule picks
+// the faster one of each.
 static bool fft_factor(int L, std::vector<int>& rad)
 {
     rad.clear();
     if (L < 4 || size_t(2) * L * sizeof(double2) > 200 * 1024) return false;
     int m = L;
-    while (m % 4 == 0) { rad.push_back(4); m /= 4; }
-    while (m % 2 == 0) { rad.push_back(2); m /= 2; }
-    while (m % 3 == 0) { rad.push_back(3); m /= 3; }
-    while (m % 5 == 0) { rad.push_back(5); m /= 5; }
-    return m == 1 && rad.size() <= 24;
+    std::vector<int> small;
+    while (m % 4 == 0) { small.push_back(4); m /= 4; }
+    while (m % 2 == 0) { small.push_back(2); m /= 2; }
+    while (m % 3 == 0) { small.push_back(3); m /= 3; }
+    while (m % 5 == 0) { small.push_back(5); m /= 5; }
+    for (int f = 7; m > 1; f += 2) {
+        if (f * f > m) f = m;
+        while (m % f == 0) { rad.push_back(f); m /= f; }
+    }
+    std::reverse(rad.begin(), rad.end());
+    const bool odd_primes = !rad.empty();
+    rad.insert(rad.end(), small.begin(), small.end());
+    if (rad.size() > 24) return false;
+    if (!odd_primes) return true;
+    double per = 0.0;
+    for (size_t i = 0; i < rad.size(); ++i) {
+        const int p = rad[i], h = p / 2;
+        if (p > 5) per += (i == 0 ? 2.0 * h * h / p + 4.0 : 4.0 * h * h / p + 6.0);
+        else per += p == 4 ? 7.0 : p == 2 ? 4.0 : p == 3 ? 8.0 : 12.0;
+    }
+    const double no = (L / 2 - 1) / 2, ne = (L / 2 - 1) - no;
+    return per * L / 2 * FFT_OVER_DENSE < ne * ne + no * no;
 }
 
 static int build_fft_tables(DSTTables& t)
@@ -732,6 +937,19 @@ static cudaError_t set_smem_attrs()
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, maxb);
 }
 
+template <int R, int CWC>
+static cudaError_t set_smem_dense64()
+{
+    const int maxb = 200 * 1024;   // plus the exchange tile in static shared memory
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, MODE_FWD, EPI_H>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, maxb))) return e;
+    if ((e = cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, MODE_INV, EPI_H>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, maxb))) return e;
+    return cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, MODE_INV, EPI_ADJQ>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, maxb);
+}
+
 // The y-direction tridiagonal solves of nf fields: 8 columns per CTA,
 // pieces of 16 rows (32 for fields of 1025-2048 rows; 8, in up to 32 warps,
 // as a schedule choice for fields of up to 1024 rows) in at most 16 warps;
@@ -780,8 +998,11 @@ static cudaError_t configure_kernels()
         if (!e) e = set_smem_attrs<float, 16>();
         if (!e) e = set_smem_attrs<float, 32>();
         if (!e) e = set_smem_attrs<float, 64>();
-        if (!e) e = set_smem_attrs<double, 16>();
-        if (!e) e = set_smem_attrs<double, 32>();
+        if (!e) e = set_smem_dense64<1, 2>();
+        if (!e) e = set_smem_dense64<2, 2>();
+        if (!e) e = set_smem_dense64<4, 2>();
+        if (!e) e = set_smem_dense64<2, 4>();
+        if (!e) e = set_smem_dense64<4, 4>();
         const int maxb = 227 * 1024;
         if (!e) e = cudaFuncSetAttribute(dst_fft_kernel<MODE_FWD, EPI_H>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, maxb);
@@ -816,6 +1037,50 @@ static int launch_pair(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs
     }
     VD_LAUNCH_CHECK();
     return VD_OK;
+}
+
+template <int R, int CWC>
+static int launch_dense64_rc(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs& a, double* spec,
+                             cudaStream_t st, bool fwd)
+{
+    const DSTTables& t = p->dst;
+    constexpr int TR = R * (4 / CWC), NC = 32 * CWC;
+    const size_t smem = (size_t)t.n * TR * sizeof(double);
+    const dim3 grid((t.ne + NC - 1) / NC, (g.R + TR - 1) / TR);
+    const double *Wo = (const double*)t.Wodd, *WoT = (const double*)t.WoddT, *We = (const double*)t.Weven;
+    if (fwd)
+        dst_dense64_kernel<R, CWC, MODE_FWD, EPI_H><<<grid, 256, smem, st>>>(
+            g, Wo, We, (const double*)a.src, (const double*)a.sub, a.sub_batches, spec, nullptr, nullptr, 0, nullptr);
+    else if (a.epi == EPI_H)
+        dst_dense64_kernel<R, CWC, MODE_INV, EPI_H><<<grid, 256, smem, st>>>(
+            g, WoT, We, nullptr, nullptr, 0, spec, (double*)a.out, (const double*)a.add, a.add_batches, p->d_mask);
+    else
+        dst_dense64_kernel<R, CWC, MODE_INV, EPI_ADJQ><<<grid, 256, smem, st>>>(
+            g, WoT, We, nullptr, nullptr, 0, spec, (double*)a.out, (const double*)a.add, a.add_batches, p->d_mask);
+    VD_LAUNCH_CHECK();
+    return VD_OK;
+}
+
+// Rows a warp: as many as leave about four warps to each of the 608 schedulers
+// (R FMAs share one W load); column groups a CTA: enough to cover the columns.
+static int launch_dense64(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs& a, double* spec,
+                          cudaStream_t st, bool fwd)
+{
+    const int cols = (p->dst.ne + 31) / 32;
+    const long long w1 = 2LL * cols * g.R;               // warps at one row each
+    const int R = w1 >= 4 * 608 * 4 ? 4 : w1 >= 2 * 608 * 4 ? 2 : 1;
+    if (cols == 1) {
+        if (R == 4) return launch_dense64_rc<4, 1>(p, g, a, spec, st, fwd);
+        if (R == 2) return launch_dense64_rc<2, 1>(p, g, a, spec, st, fwd);
+        return launch_dense64_rc<1, 1>(p, g, a, spec, st, fwd);
+    }
+    if (cols == 2 || R == 1) {
+        if (R == 4) return launch_dense64_rc<4, 2>(p, g, a, spec, st, fwd);
+        if (R == 2) return launch_dense64_rc<2, 2>(p, g, a, spec, st, fwd);
+        return launch_dense64_rc<1, 2>(p, g, a, spec, st, fwd);
+    }
+    if (R == 4) return launch_dense64_rc<4, 4>(p, g, a, spec, st, fwd);
+    return launch_dense64_rc<2, 4>(p, g, a, spec, st, fwd);
 }
 
 // The float64 FFT pass over g.R rows: pairs of rows per CTA chosen for about
@@ -855,21 +1120,36 @@ static int launch_fft(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs&
 
 // Rows per CTA: the largest tile that still gives about two waves of CTAs on
 // the 152 SMs and fits shared memory.
-template <typename T>
 static int pick_tr(const vd_qg1l_plan* p, int R)
 {
     const DSTTables& t = p->dst;
-    if (p->sched.fma_rows == 16 || p->sched.fma_rows == 32 || (p->sched.fma_rows == 64 && sizeof(T) == 4))
-        return p->sched.fma_rows;
+    if (p->sched.fma_rows) return p->sched.fma_rows;
     const int cand[3] = {64, 32, 16};
     for (int c : cand) {
-        if (sizeof(T) == 8 && c == 64) continue;
-        const size_t smem = (size_t(2) * t.kpad * c + size_t(std::max(2 * DST_KC * DST_NC, c * DST_NC))) * sizeof(T);
+        const size_t smem = (size_t(2) * t.kpad * c + size_t(std::max(2 * DST_KC * DST_NC, c * DST_NC))) * sizeof(float);
         if (smem > 200 * 1024) continue;
         const long long ctas = (long long)t.ncol_tiles * ((R + c - 1) / c);
         if (ctas >= 2 * 152) return c;
     }
     return 16;
+}
+
+// One x-direction pass: float32 on the tensor cores or CUDA-core FMA, float64
+// as FFT or dense products.
+template <typename T>
+static int dst_pass(const vd_qg1l_plan* p, int nf, const GemmGeom& g, const SolveArgs& a, T* spec, cudaStream_t st,
+                    bool fwd)
+{
+    if constexpr (sizeof(T) == 4) {
+        if (use_tc(p, nf)) return dst_pass_tc(p, nf, a, spec, fwd, st);
+        const int tr = pick_tr(p, g.R);
+        if (tr == 64) return launch_pair<T, 64>(p, g, a, spec, st, fwd);
+        if (tr == 32) return launch_pair<T, 32>(p, g, a, spec, st, fwd);
+        return launch_pair<T, 16>(p, g, a, spec, st, fwd);
+    } else {
+        if (p->dst.fft_L) return launch_fft(p, g, a, spec, st, fwd);
+        return launch_dense64(p, g, a, spec, st, fwd);
+    }
 }
 
 template <typename T>
@@ -882,21 +1162,10 @@ int helmholtz_solve(const vd_qg1l_plan* p, int nf, const SolveArgs& a, T* spec, 
     g.fs = (long long)p->d.ny * p->d.nx;
     g.R = nf * t.my;
     g.kpad = t.kpad; g.ldw = t.ldw; g.lds = t.lds;
-    const int tr = pick_tr<T>(p, g.R);
     int rc;
-    auto run = [&](bool fwd) -> int {
-        if constexpr (sizeof(T) == 4) {
-            if (use_tc(p, nf)) return dst_pass_tc(p, nf, a, (float*)spec, fwd, st);
-            if (tr == 64) return launch_pair<T, 64>(p, g, a, spec, st, fwd);
-        } else {
-            if (p->dst.fft_L) return launch_fft(p, g, a, (double*)spec, st, fwd);
-        }
-        if (tr == 32) return launch_pair<T, 32>(p, g, a, spec, st, fwd);
-        return launch_pair<T, 16>(p, g, a, spec, st, fwd);
-    };
-    if ((rc = run(true))) return rc;
+    if ((rc = dst_pass<T>(p, nf, g, a, spec, st, true))) return rc;
     if ((rc = launch_tridiag<T>(p, nf, spec, st))) return rc;
-    return run(false);
+    return dst_pass<T>(p, nf, g, a, spec, st, false);
 }
 
 template int helmholtz_solve<float>(const vd_qg1l_plan*, int, const SolveArgs&, float*, cudaStream_t);
@@ -921,15 +1190,7 @@ int dst_x_only(const vd_qg1l_plan* p, int nf, const T* field, T* spec, int inver
         a.src = nullptr;
         a.add = field; a.add_batches = nf; a.epi = EPI_ADJQ;
     }
-    const int tr = pick_tr<T>(p, g.R);
-    if constexpr (sizeof(T) == 4) {
-        if (use_tc(p, nf)) return dst_pass_tc(p, nf, a, (float*)spec, !inverse, st);
-        if (tr == 64) return launch_pair<T, 64>(p, g, a, spec, st, !inverse);
-    } else {
-        if (p->dst.fft_L) return launch_fft(p, g, a, (double*)spec, st, !inverse);
-    }
-    if (tr == 32) return launch_pair<T, 32>(p, g, a, spec, st, !inverse);
-    return launch_pair<T, 16>(p, g, a, spec, st, !inverse);
+    return dst_pass<T>(p, nf, g, a, spec, st, !inverse);
 }
 
 // The y-direction tridiagonal solve alone, in place on spectral rows.

@@ -83,15 +83,20 @@ typedef struct vd_qg1l_schedule {
                             VD_DST_AUTO, else CUDA-core FMA / float64 FFT);
                             1 CUDA-core FMA; 2 tensor cores (float32 plans
                             built with VD_DST_AUTO) */
-    int tc_group_fwd;    /* 32-column output tiles per CTA of the forward
-                            tensor-core pass: 0 rule, or 1, 2, 4, 8 */
+    int tc_group_fwd;    /* shape of a CTA of the forward tensor-core pass: 0
+                            rule; rows of a field x groups of 128 modes: 1
+                            32 x 1, 2 64 x 1, 4 128 x 1, 8 128 x 2. Also
+                            decides, with the rule, whether the pass solves
+                            the tridiagonal systems in its epilogue (the
+                            fields' row blocks, at most 8, then form a
+                            cluster) */
     int tc_group_inv;    /* the same for the inverse pass */
     int fma_rows;        /* rows per CTA of the float32 FMA pass: 0 rule, 16,
                             32 or 64 (float64 plans accept 16 and 32 and keep
                             their own rule) */
-    int tridiag_rows;    /* rows per thread of the tridiagonal solve: 0 rule,
-                            8, 16 or 32 (used when the field fits, else the
-                            rule) */
+    int tridiag_rows;    /* rows per thread of the separate tridiagonal
+                            solve: 0 rule, 8, 16 or 32 (used when the field
+                            fits, else the rule) */
     int tridiag_lean;    /* 1: the float32 16-row tridiagonal kernel capped at
                             80 registers (three CTAs per SM instead of two);
                             0 the standard kernel */

@@ -1163,6 +1163,11 @@ int helmholtz_solve(const vd_qg1l_plan* p, int nf, const SolveArgs& a, T* spec, 
     g.R = nf * t.my;
     g.kpad = t.kpad; g.ldw = t.ldw; g.lds = t.lds;
     int rc;
+    if constexpr (sizeof(T) == 4) {
+        bool done = false;
+        if (use_tc(p, nf) && (rc = dst_solve_tc(p, nf, a, spec, &done, st))) return rc;
+        if (done) return dst_pass<T>(p, nf, g, a, spec, st, false);
+    }
     if ((rc = dst_pass<T>(p, nf, g, a, spec, st, true))) return rc;
     if ((rc = launch_tridiag<T>(p, nf, spec, st))) return rc;
     return dst_pass<T>(p, nf, g, a, spec, st, false);

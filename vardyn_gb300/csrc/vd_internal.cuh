@@ -121,6 +121,9 @@ bool tc_fits(const vd_qg1l_plan* p, int nf);
 // Whether the tensor-core pass runs for nf fields under the plan's schedule.
 inline bool use_tc(const vd_qg1l_plan* p, int nf) { return p->dst.tc && tc_fits(p, nf) && p->sched.engine != 1; }
 int dst_pass_tc(const vd_qg1l_plan* p, int nf, const SolveArgs& a, float* spec, bool fwd, cudaStream_t st);
+// Forward pass with the tridiagonal solve in its epilogue (*done false, and
+// nothing launched, when the field is too tall for one cluster).
+int dst_solve_tc(const vd_qg1l_plan* p, int nf, const SolveArgs& a, float* spec, bool* done, cudaStream_t st);
 // Neumann spectral Helmholtz solve of nf [nx][ny] fields (dst may equal src).
 template <typename T>
 int neumann_solve(const vd_neumann_plan* p, int nf, const T* src, T* dst, cudaStream_t st);

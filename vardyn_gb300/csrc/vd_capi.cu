@@ -15,13 +15,15 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 size_t elem_size(int dtype) { return dtype == VD_F64 ? 8 : 4; }
 
 template <typename T>
-int advance_impl(const vd_qg1l_plan*, int, T*, int, int, int, const T*, const T*, T*, Arena&, cudaStream_t);
+int advance_impl(const vd_qg1l_plan*, int, T*, int, int, int, const T*, const T*, const int*, T*, Arena&,
+                 cudaStream_t);
 template <typename T>
-int forward_nostore(const vd_qg1l_plan*, int, T*, T*, int, const T*, const T*, T*, Arena&, cudaStream_t, bool);
+int forward_nostore(const vd_qg1l_plan*, int, const T*, T*, int, const T*, const T*, const int*, T*, T*, Arena&,
+                    cudaStream_t, bool, const T**);
 template <typename T>
 int advance_adj_impl(const vd_qg1l_plan*, int, const T*, int, int, int, T*, T*, Arena&, cudaStream_t);
 template <typename T>
-int init_state_impl(const vd_qg1l_plan*, int, int, const T*, const T*, T*, T*, T*, cudaStream_t);
+int init_state_impl(const vd_qg1l_plan*, int, int, const T*, const T*, T*, T*, T*, int*, cudaStream_t);
 template <typename T>
 int init_state_adj_impl(const vd_qg1l_plan*, int, const T*, const T*, T*, cudaStream_t);
 template <typename T>
@@ -194,9 +196,14 @@ extern "C" vd_status vd_qg1l_plan_create(vd_qg1l_plan** out, const vd_qg1l_desc*
     G.cy = 1.0 / (6 * d->dy);
     G.idx2 = 1.0 / (d->dx * d->dx);
     G.idy2 = 1.0 / (d->dy * d->dy);
+    G.gfx = G.gf * G.idx2;
+    G.gfy = G.gf * G.idy2;
     G.hasK = d->has_Kdiffus ? 1 : 0;
     G.Kx = d->has_Kdiffus ? d->Kdiffus / (d->dx * d->dx) : 0.0;
     G.Ky = d->has_Kdiffus ? d->Kdiffus / (d->dy * d->dy) : 0.0;
+    G.kd = QGConst<double>{G.gf, G.gfc2, G.cu, G.cv, G.cx, G.cy, G.idx2, G.idy2, G.gfx, G.gfy, G.Kx, G.Ky};
+    G.kf = QGConst<float>{(float)G.gf, (float)G.gfc2, (float)G.cu, (float)G.cv, (float)G.cx, (float)G.cy,
+                          (float)G.idx2, (float)G.idy2, (float)G.gfx, (float)G.gfy, (float)G.Kx, (float)G.Ky};
     G.mask = p->d_mask;
     G.beta = p->d_beta;
     G.fB = p->d_fB;
@@ -274,7 +281,7 @@ extern "C" size_t vd_qg1l_workspace_bytes(const vd_qg1l_plan* p, int B)
     const size_t adj = 2 * B * F + (adv_part > adj_part ? adv_part : adj_part) + 2 * B * F;
     size_t m = step > tgl ? step : tgl;
     m = m > adj ? m : adj;
-    return m + 64 * 256;
+    return m + 64 * 256 + B * sizeof(int);
 }
 
 static inline long long fb_elems(const vd_qg1l_plan* p, int B) { return (long long)B * p->geom.fs; }
@@ -284,9 +291,10 @@ extern "C" vd_status vd_qg1l_h2pv(const vd_qg1l_plan* p, int B, const void* h, c
     if (!p || B <= 0 || !h || !hb || !q) return VD_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     return p->d.dtype == VD_F32
-               ? init_state_impl<float>(p, B, B, (const float*)h, (const float*)hb, (float*)q, nullptr, nullptr, st)
+               ? init_state_impl<float>(p, B, B, (const float*)h, (const float*)hb, (float*)q, nullptr, nullptr, nullptr,
+                                       st)
                : init_state_impl<double>(p, B, B, (const double*)h, (const double*)hb, (double*)q, nullptr, nullptr,
-                                         st);
+                                         nullptr, st);
 }
 
 extern "C" vd_status vd_qg1l_h2uv(const vd_qg1l_plan* p, int B, const void* h, void* u, void* v, void* stream)
@@ -343,6 +351,13 @@ static int take_qlo(const vd_qg1l_plan* p, long long n, Arena& ws, T** qlo)
     return *qlo ? VD_OK : VD_ERR_WORKSPACE;
 }
 
+// Flags of windows whose background SSH is not all zeros (SolveArgs::bg_on).
+static int take_flags(int B, Arena& ws, int** on)
+{
+    *on = (int*)ws.take(B * sizeof(int));
+    return *on ? VD_OK : VD_ERR_WORKSPACE;
+}
+
 template <typename T>
 static int step_t(const vd_qg1l_plan* p, int B, const T* h0, const T* hb, int nstep, T* hout, T* traj, Arena& ws,
                   cudaStream_t st)
@@ -353,21 +368,22 @@ static int step_t(const vd_qg1l_plan* p, int B, const T* h0, const T* hb, int ns
     T* qlo;
     int rc;
     if ((rc = take_qlo<T>(p, fb, ws, &qlo))) return rc;
+    int* on;
+    if ((rc = take_flags(B, ws, &on))) return rc;
     if (traj) {
         T* h = traj;
         T* q = traj + fb;
         VD_CUDA_TRY(cudaMemcpyAsync(h, h0, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        if ((rc = init_state_impl<T>(p, B, B, h, hb, q, qb, qlo, st))) return rc;
-        if ((rc = advance_impl<T>(p, B, traj, nstep, 0, nstep, hb, qb, qlo, ws, st))) return rc;
+        if ((rc = init_state_impl<T>(p, B, B, h, hb, q, qb, qlo, on, st))) return rc;
+        if ((rc = advance_impl<T>(p, B, traj, nstep, 0, nstep, hb, qb, on, qlo, ws, st))) return rc;
         const T* hN = traj + (long long)nstep * p->nstage * 2 * fb;
         return finalize_impl<T>(p, B, hN, hb, nullptr, 0.0, nullptr, 1, hout, st);
     }
-    T* h = (T*)ws.take(fb * sizeof(T));
     T* q = (T*)ws.take(fb * sizeof(T));
-    if (!h || !q) return VD_ERR_WORKSPACE;
-    VD_CUDA_TRY(cudaMemcpyAsync(h, h0, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    if ((rc = init_state_impl<T>(p, B, B, h, hb, q, qb, qlo, st))) return rc;
-    if ((rc = forward_nostore<T>(p, B, h, q, nstep, hb, qb, qlo, ws, st, false))) return rc;
+    if (!q) return VD_ERR_WORKSPACE;
+    const T* h;
+    if ((rc = init_state_impl<T>(p, B, B, h0, hb, q, qb, qlo, on, st))) return rc;
+    if ((rc = forward_nostore<T>(p, B, h0, q, nstep, hb, qb, on, qlo, (T*)nullptr, ws, st, false, &h))) return rc;
     return finalize_impl<T>(p, B, h, hb, nullptr, 0.0, nullptr, 1, hout, st);
 }
 
@@ -396,11 +412,14 @@ static int step_tgl_t(const vd_qg1l_plan* p, int B, const T* dh0, const T* h0, c
     T* qlo;
     int rc;
     if ((rc = take_qlo<T>(p, 2 * fb, ws, &qlo))) return rc;
+    int* on;
+    if ((rc = take_flags(B, ws, &on))) return rc;
     VD_CUDA_TRY(cudaMemcpyAsync(h, h0, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
     VD_CUDA_TRY(cudaMemcpyAsync(h + fb, dh0, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    if ((rc = init_state_impl<T>(p, 2 * B, B, h, hb, q, qb, qlo, st))) return rc;
-    if ((rc = forward_nostore<T>(p, 2 * B, h, q, nstep, hb, qb, qlo, ws, st, true))) return rc;
-    return finalize_impl<T>(p, B, h + fb, nullptr, nullptr, 0.0, nullptr, 2, dhout, st);
+    if ((rc = init_state_impl<T>(p, 2 * B, B, h, hb, q, qb, qlo, on, st))) return rc;
+    const T* he;
+    if ((rc = forward_nostore<T>(p, 2 * B, h, q, nstep, hb, qb, on, qlo, h, ws, st, true, &he))) return rc;
+    return finalize_impl<T>(p, B, he + fb, nullptr, nullptr, 0.0, nullptr, 2, dhout, st);
 }
 
 extern "C" vd_status vd_qg1l_step_tgl(const vd_qg1l_plan* p, int B, const void* dh0, const void* h0,
@@ -432,10 +451,12 @@ static int step_adj_t(const vd_qg1l_plan* p, int B, const T* adh1, const T* h0, 
         if (!qb) return VD_ERR_WORKSPACE;
         T* qlo;
         if ((rc = take_qlo<T>(p, fb, ws, &qlo))) return rc;
+        int* on;
+        if ((rc = take_flags(B, ws, &on))) return rc;
         VD_CUDA_TRY(cudaMemcpyAsync(traj, h0, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        if ((rc = init_state_impl<T>(p, B, B, traj, hb, traj + fb, qb, qlo, st))) return rc;
+        if ((rc = init_state_impl<T>(p, B, B, traj, hb, traj + fb, qb, qlo, on, st))) return rc;
         Arena sub = ws;
-        if ((rc = advance_impl<T>(p, B, traj, nstep, 0, nstep, hb, qb, qlo, sub, st))) return rc;
+        if ((rc = advance_impl<T>(p, B, traj, nstep, 0, nstep, hb, qb, on, qlo, sub, st))) return rc;
     }
     if ((rc = copy_impl<T>(p, B, adh1, adh, 1, st))) return rc;
     if ((rc = zero_impl<T>(fb, adq, st))) return rc;
@@ -511,9 +532,9 @@ extern "C" vd_status vd_qg1l_init_state(const vd_qg1l_plan* p, int B, const void
     cudaStream_t st = (cudaStream_t)stream;
     return p->d.dtype == VD_F32
                ? init_state_impl<float>(p, B, B, (const float*)h, (const float*)hb, (float*)q, (float*)qb,
-                                        (float*)qlo, st)
+                                        (float*)qlo, nullptr, st)
                : init_state_impl<double>(p, B, B, (const double*)h, (const double*)hb, (double*)q, (double*)qb,
-                                         (double*)qlo, st);
+                                         (double*)qlo, nullptr, st);
 }
 
 extern "C" vd_status vd_qg1l_advance(const vd_qg1l_plan* p, int B, void* traj, int traj_steps, int first_step,
@@ -527,9 +548,9 @@ extern "C" vd_status vd_qg1l_advance(const vd_qg1l_plan* p, int B, void* traj, i
     cudaStream_t st = (cudaStream_t)stream;
     return p->d.dtype == VD_F32
                ? advance_impl<float>(p, B, (float*)traj, traj_steps, first_step, nstep, (const float*)hb,
-                                     (const float*)qb, (float*)qlo, ws, st)
+                                     (const float*)qb, nullptr, (float*)qlo, ws, st)
                : advance_impl<double>(p, B, (double*)traj, traj_steps, first_step, nstep, (const double*)hb,
-                                      (const double*)qb, (double*)qlo, ws, st);
+                                      (const double*)qb, nullptr, (double*)qlo, ws, st);
 }
 
 extern "C" vd_status vd_qg1l_advance_adj(const vd_qg1l_plan* p, int B, const void* traj, int traj_steps,

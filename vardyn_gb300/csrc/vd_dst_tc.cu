@@ -567,8 +567,8 @@ struct TcLoop {
 template <int RPW, int MG, bool FUSE>
 __global__ void __launch_bounds__(NTHREADS, 1)
 dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const float* __restrict__ src,
-                  const float* __restrict__ sub, int sub_batches, float* __restrict__ spec,
-                  const float* __restrict__ trim, float a)
+                  const float* __restrict__ sub, int sub_batches, const int* __restrict__ bg_on,
+                  float* __restrict__ spec, const float* __restrict__ trim, float a)
 {
     using Sh = TcShape<RPW, MG>;
     constexpr int RB = Sh::RB, PC = Sh::PC, NPC = Sh::NPC;
@@ -630,7 +630,7 @@ dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
         const uint32_t b_bytes = (uint32_t)wrows * KCH * 4;
         if constexpr (FUSE) {
             const unsigned first = (unsigned)((r0 + 1) * g.nx + 1), pitch = (unsigned)g.nx;
-            L.produce(src + o, sub != nullptr && f < sub_batches ? sub + o : nullptr,
+            L.produce(src + o, sub != nullptr && f < sub_batches && (!bg_on || bg_on[f]) ? sub + o : nullptr,
                       [&](int i) { return first + i * pitch; }, [](int) { return true; }, nv, g.n, lim, g.no, half,
                       bimg, tab.Ntot, b_bytes, side);
         } else {
@@ -640,7 +640,7 @@ dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
             for (int i = 0; i < RPW; ++i) {
                 const int r = min(r0 + i, nrows - 1), fi = r / g.my;
                 ro[i] = (unsigned)(fi * g.fs + (long long)(r - fi * g.my + 1) * g.nx + 1);
-                on |= (unsigned)(fi < sub_batches) << i;
+                on |= (unsigned)(sub != nullptr && fi < sub_batches && (!bg_on || bg_on[fi])) << i;
             }
             L.produce(src, on ? sub : nullptr, [&](int i) { return ro[i]; }, [&](int i) { return (on >> i & 1u) != 0; }, nv, g.n,
                       lim, g.no, half, bimg, tab.Ntot, b_bytes, side);
@@ -770,7 +770,7 @@ template <int RPW, int MG, int EPI>
 __global__ void __launch_bounds__(NTHREADS, 1)
 dst_tc_inv_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const float* __restrict__ spec,
                   float* __restrict__ out, const float* __restrict__ add, int add_batches,
-                  const int8_t* __restrict__ mask)
+                  const int* __restrict__ bg_on, const int8_t* __restrict__ mask)
 {
     using Sh = TcShape<RPW, MG>;
     constexpr int RB = Sh::RB, HR = RB / 2;
@@ -873,7 +873,7 @@ dst_tc_inv_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
             auto locate = [&](int r) {
                 const int f = (jb + r) / g.my, j = jb + r - f * g.my + 1;
                 return Row{f * g.fs + (long long)j * g.nx, mask + (long long)j * g.nx,
-                           add != nullptr && (EPI != EPI_H || f < add_batches)};
+                           add != nullptr && (EPI != EPI_H || (f < add_batches && (!bg_on || bg_on[f])))};
             };
             const float* stage = reinterpret_cast<const float*>(smem_raw) + ((L.sbase - smem_u32(smem_raw)) >> 2) + XFL;
             auto value = [&](const float x, float ad, int8_t mk) {
@@ -1182,9 +1182,9 @@ static int tc_launch_fwd(const vd_qg1l_plan* p, int nf, const SolveArgs& a, floa
         const float *src = (const float*)a.src, *sub = (const float*)a.sub, *trim = (const float*)t.trim;
         const float ta = (float)t.tri_a;
         return fuse ? cudaLaunchKernelEx(&cfg, dst_tc_fwd_kernel<R(), M(), true>, g, tab, (const float*)d->img, src,
-                                         sub, a.sub_batches, spec, trim, ta)
+                                         sub, a.sub_batches, a.bg_on, spec, trim, ta)
                     : cudaLaunchKernelEx(&cfg, dst_tc_fwd_kernel<R(), M(), false>, g, tab, (const float*)d->img, src,
-                                         sub, a.sub_batches, spec, trim, ta);
+                                         sub, a.sub_batches, a.bg_on, spec, trim, ta);
     });
     if (e != cudaSuccess) return VD_ERR_CUDA;
     VD_LAUNCH_CHECK();
@@ -1223,10 +1223,10 @@ static int tc_launch_inv(const vd_qg1l_plan* p, int nf, const SolveArgs& a, cons
         cfg.numAttrs = 1;
         return a.epi == EPI_H ? cudaLaunchKernelEx(&cfg, dst_tc_inv_kernel<R(), M(), EPI_H>, g, tab,
                                                    (const float*)d->img, spec, (float*)a.out, (const float*)a.add,
-                                                   a.add_batches, (const int8_t*)p->d_mask)
+                                                   a.add_batches, a.bg_on, (const int8_t*)p->d_mask)
                               : cudaLaunchKernelEx(&cfg, dst_tc_inv_kernel<R(), M(), EPI_ADJQ>, g, tab,
                                                    (const float*)d->img, spec, (float*)a.out, (const float*)a.add,
-                                                   a.add_batches, (const int8_t*)p->d_mask);
+                                                   a.add_batches, a.bg_on, (const int8_t*)p->d_mask);
     });
     if (e != cudaSuccess) return VD_ERR_CUDA;
     VD_LAUNCH_CHECK();

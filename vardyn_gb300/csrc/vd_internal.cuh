@@ -28,8 +28,17 @@ void count_launch();
 namespace vd {
 
 // ---------------------------------------------------------------------------
-// Grid constants passed to every QG kernel by value.
+// Grid constants passed to every QG kernel by value. The kernels take them from
+// the copy of their own type (qk): converting a double in a float32 kernel is an
+// FP64 instruction a thread, and this part's FP64 pipe (2 lanes a clock and SM)
+// then set the pace of the float32 stencils (the forward stage at 16 x 512^2:
+// 26.7 us with four such conversions for two points).
 // ---------------------------------------------------------------------------
+template <typename T>
+struct QGConst {
+    T gf, gfc2, cu, cv, cx, cy, idx2, idy2, gfx, gfy, Kx, Ky;
+};
+
 struct QGGeom {
     int ny, nx;
     long long fs;            // field stride = ny*nx
@@ -39,12 +48,19 @@ struct QGGeom {
     double cv;               //  g/f/(4 dx)
     double cx, cy;           // 1/(6 dx), 1/(6 dy)
     double idx2, idy2;       // 1/dx^2, 1/dy^2
+    double gfx, gfy;         // g/f/dx^2, g/f/dy^2
     double Kx, Ky;           // Kdiffus/dx^2, Kdiffus/dy^2 (0 when absent)
     int hasK;
+    QGConst<double> kd;      // the constants above, by type
+    QGConst<float> kf;
     const int8_t* mask;      // [ny][nx]
     const void* beta;        // T[ny][nx] or nullptr
     const void* fB;          // T[ny][nx] or nullptr
 };
+
+template <typename T> __host__ __device__ inline const QGConst<T>& qk(const QGGeom& G);
+template <> __host__ __device__ inline const QGConst<double>& qk<double>(const QGGeom& G) { return G.kd; }
+template <> __host__ __device__ inline const QGConst<float>& qk<float>(const QGGeom& G) { return G.kf; }
 
 // DST-I / tridiagonal tables of one grid (typed by the plan dtype).
 struct DSTTables {
@@ -84,6 +100,9 @@ struct SolveArgs {
     const void* add;     // EPI_H: hb (used for batches < add_batches); EPI_ADJQ: addend field
     int add_batches;
     int epi;
+    // per field f < sub_batches, nullable: 0 where the background is all zeros, so
+    // that sub and (EPI_H) add need not be read (the float32 tensor-core passes)
+    const int* bg_on = nullptr;
 };
 
 }  // namespace vd

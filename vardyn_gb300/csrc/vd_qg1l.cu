@@ -77,7 +77,7 @@ struct Vel {
     // from the SSH at rows j-1 (s), j, j+1 (n) and columns i-1 (w), i, i+1 (e)
     __device__ __forceinline__ void set(const QGGeom& G, T hs_w, T hs_c, T hs_e, T h_w, T h_e, T hn_w, T hn_c,
                                         T hn_e) {
-        const T cu = T(G.cu), cv = T(G.cv);
+        const T cu = qk<T>(G).cu, cv = qk<T>(G).cv;
         u0 = cu * (hn_w + hn_c - hs_c - hs_w);
         u1 = cu * (hn_c + hn_e - hs_e - hs_c);
         v0 = cv * (h_e + hs_e - hs_w - h_w);
@@ -101,11 +101,11 @@ __device__ __forceinline__ T tendency(const QGGeom& G, const Vel<T>& V, const Cr
     const T um = uT > T(0) ? T(0) : uT;
     const T vp = vT < T(0) ? T(0) : vT;
     const T vm = vT > T(0) ? T(0) : vT;
-    const T cx = T(G.cx), cy = T(G.cy);
+    const T cx = qk<T>(G).cx, cy = qk<T>(G).cy;
     T r = -up * cx * qa.Dpx() + um * cx * qa.Dmx() - vp * cy * qa.Dpy() + vm * cy * qa.Dmy();
     r -= beta * ((V.v0 + V.v1) / T(2));
     if (MAYK && G.hasK)
-        r += T(G.Kx) * (q.e1 + q.w1 - T(2) * q.c) + T(G.Ky) * (q.n1 + q.s1 - T(2) * q.c);
+        r += qk<T>(G).Kx * (q.e1 + q.w1 - T(2) * q.c) + qk<T>(G).Ky * (q.n1 + q.s1 - T(2) * q.c);
     return r;
 }
 
@@ -118,56 +118,119 @@ __device__ __forceinline__ T lap_helm(const QGGeom& G, const T* __restrict__ hc)
 {
     const int nx = G.nx;
     const T c = hc[0];
-    return T(G.gf) * ((hc[nx] + hc[-nx] - T(2) * c) * T(G.idy2) +
-                      (hc[1] + hc[-1] - T(2) * c) * T(G.idx2)) - T(G.gfc2) * c;
+    return qk<T>(G).gf * ((hc[nx] + hc[-nx] - T(2) * c) * qk<T>(G).idy2 +
+                      (hc[1] + hc[-1] - T(2) * c) * qk<T>(G).idx2) - qk<T>(G).gfc2 * c;
 }
 
+// float -> double and back by integer arithmetic: the conversions run on the
+// FP64 pipe (2 a clock and SM), integers on 64 lanes. Exact / rounded to nearest
+// even; anything but normal numbers and zeros takes the hardware conversion, in
+// a call: inlined it would be predicated, and a predicated-off FP64 instruction
+// still takes its issue slot.
+__device__ __noinline__ double f2d_slow(float x) { return (double)x; }
+__device__ __noinline__ float d2f_slow(double x) { return (float)x; }
+__device__ __forceinline__ double f2d(float x)
+{
+    const uint32_t b = __float_as_uint(x), e = b & 0x7f800000u;
+    if ((b << 1) != 0 && (e == 0 || e == 0x7f800000u)) return f2d_slow(x);
+    const uint32_t hi = (b & 0x80000000u) | ((b << 1) == 0 ? 0u : ((b & 0x7fffffffu) >> 3) + 0x38000000u);
+    return __hiloint2double((int)hi, (int)(b << 29));
+}
+__device__ __forceinline__ float d2f(double x)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    const uint32_t m = hi & 0x7fffffffu;
+    if (m < 0x38100000u || m >= 0x47e00000u) return d2f_slow(x);   // zero, below or above the normal floats, NaN
+    uint32_t r = ((m - 0x38000000u) << 3) | (lo >> 29);
+    const uint32_t rest = lo & 0x1fffffffu;
+    r += rest > 0x10000000u || (rest == 0x10000000u && (r & 1u));
+    return __uint_as_float((hi & 0x80000000u) | r);
+}
+
+// Finite and far from overflow through any of the stencils below.
+__device__ __forceinline__ bool tame(float x) { return (__float_as_uint(x) & 0x7fffffffu) < 0x5d000000u; }
+__device__ __forceinline__ bool tame(double x) { return ((uint32_t)__double2hiint(x) & 0x7fffffffu) < 0x5f000000u; }
+
+// Whether the Helmholtz stencil at hc is NaN, without its (FP64) instructions
+// where all five values are tame. The other form is a call: inlined, it would be
+// predicated and issued all the same.
 template <typename T>
-__device__ __forceinline__ double lap_helm_f64(const QGGeom& G, const T* __restrict__ hc)
+__device__ __noinline__ bool lap_is_nan_slow(const QGGeom& G, const T* __restrict__ hc)
+{
+    return isnan(lap_helm<T>(G, hc));
+}
+template <typename T>
+__device__ __forceinline__ bool lap_is_nan(const QGGeom& G, const T* __restrict__ hc)
 {
     const int nx = G.nx;
-    const double c = hc[0];
-    return G.gf * (((double)hc[nx] + (double)hc[-nx] - 2.0 * c) * G.idy2 +
-                   ((double)hc[1] + (double)hc[-1] - 2.0 * c) * G.idx2) - G.gfc2 * c;
+    if (tame(hc[0]) && tame(hc[nx]) && tame(hc[-nx]) && tame(hc[1]) && tame(hc[-1])) return false;
+    return lap_is_nan_slow<T>(G, hc);
+}
+
+// The stencil of a float32 SSH in float64: 7 FP64 instructions (exact
+// differences, then two products and the Helmholtz term).
+__device__ __forceinline__ double lap_helm_f64(const QGGeom& G, const float* __restrict__ hc)
+{
+    const int nx = G.nx;
+    const double c = f2d(hc[0]);
+    const double dy = fma(-2.0, c, f2d(hc[nx]) + f2d(hc[-nx]));
+    const double dx = fma(-2.0, c, f2d(hc[1]) + f2d(hc[-1]));
+    return fma(G.gfx, dx, fma(G.gfy, dy, -G.gfc2 * c));
+}
+
+__device__ __noinline__ double ring_pv_f64(const QGGeom& G, float hb) { return -G.gfc2 * f2d(hb); }
+__device__ __noinline__ bool lap_f64_is_nan_slow(const QGGeom& G, const float* __restrict__ hc)
+{
+    return isnan(lap_helm_f64(G, hc));
 }
 
 // With qlo != nullptr (float32 plans) the PV is evaluated in float64 from
-// the float32 SSH and returned as the pair q + qlo of the compensated state.
+// the float32 SSH and returned as the pair q + qlo of the compensated state; that
+// form is bound by the FP64 pipe, at 7 FP64 instructions a point (16 x 512^2:
+// 150 us with hardware conversions, a second stencil for the NaN guard and the
+// ring's product predicated, 66 us now).
+// on != nullptr: on[f] = 1 where field f of h holds anything but zeros.
 template <typename T>
 __global__ void k_h2pv(QGGeom G, int nf, int ntan0, const T* __restrict__ h,
-                       const T* __restrict__ hb, T* __restrict__ q, T* __restrict__ qlo)
+                       const T* __restrict__ hb, T* __restrict__ q, T* __restrict__ qlo, int* __restrict__ on)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int f = blockIdx.z;
+    if (on) {
+        const bool nz = i < G.nx && j < G.ny && h[f * G.fs + (long long)j * G.nx + i] != T(0);
+        if (__syncthreads_or(nz) && threadIdx.x + threadIdx.y == 0) on[f] = 1;
+    }
     if (i >= G.nx || j >= G.ny || f >= nf) return;
     const long long o = f * G.fs + (long long)j * G.nx + i;
     const int m = G.mask[j * G.nx + i];
-    if (qlo) {
-        double val = 0.0;
-        if (m == 3) {
-            val = lap_helm_f64<T>(G, h + o);
-            const double prim = f >= ntan0 ? lap_helm_f64<T>(G, h + o - ntan0 * G.fs) : val;
-            if (isnan(prim)) val = 0.0;
-        } else if (m != 0 && f < ntan0) {
-            val = -G.gfc2 * (double)hb[o];
+    if constexpr (sizeof(T) == 4) {
+        if (qlo) {
+            double val = 0.0;
+            if (m == 3) {
+                val = lap_helm_f64(G, h + o);
+                const float* hp = f >= ntan0 ? h + o - ntan0 * G.fs : h + o;
+                const bool fine = tame(hp[0]) && tame(hp[G.nx]) && tame(hp[-G.nx]) && tame(hp[1]) && tame(hp[-1]);
+                if (!fine && lap_f64_is_nan_slow(G, hp)) val = 0.0;
+            } else if (m != 0 && f < ntan0) {
+                val = ring_pv_f64(G, hb[o]);
+            }
+            const float hi = d2f(val);
+            q[o] = hi;
+            qlo[o] = d2f(val - f2d(hi));
+            return;
         }
-        const T hi = (T)val;
-        q[o] = hi;
-        qlo[o] = (T)(val - (double)hi);
-        return;
     }
     T val = T(0);
     if (m == 3) {
         val = lap_helm<T>(G, h + o);
         if (f >= ntan0) {
-            const T prim = lap_helm<T>(G, h + o - ntan0 * G.fs);
-            if (isnan(prim)) val = T(0);
+            if (lap_is_nan<T>(G, h + o - ntan0 * G.fs)) val = T(0);
         } else {
             val = guard0(val);
         }
     } else if (m != 0 && f < ntan0) {
-        val = -T(G.gfc2) * hb[o];
+        val = -qk<T>(G).gfc2 * hb[o];
     }
     q[o] = val;
 }
@@ -182,7 +245,7 @@ __global__ void k_h2pv_adj(QGGeom G, int nf, const T* __restrict__ h, const T* _
     const int f = blockIdx.z;
     if (i >= G.nx || j >= G.ny || f >= nf) return;
     const long long o = f * G.fs + (long long)j * G.nx + i;
-    const T gfy = T(G.gf) * T(G.idy2), gfx = T(G.gf) * T(G.idx2);
+    const T gfy = qk<T>(G).gf * qk<T>(G).idy2, gfx = qk<T>(G).gf * qk<T>(G).idx2;
     const int di[5] = {0, 1, -1, 0, 0};
     const int dj[5] = {0, 0, 0, 1, -1};
     T acc = T(0);
@@ -192,8 +255,8 @@ __global__ void k_h2pv_adj(QGGeom G, int nf, const T* __restrict__ h, const T* _
         if (jj < 0 || jj >= G.ny || ii < 0 || ii >= G.nx) continue;
         if (G.mask[jj * G.nx + ii] != 3) continue;
         const long long po = f * G.fs + (long long)jj * G.nx + ii;
-        if (isnan(lap_helm<T>(G, h + po))) continue;
-        const T coef = (k == 0) ? (-T(2) * gfy - T(2) * gfx - T(G.gfc2)) : (k < 3 ? gfx : gfy);
+        if (lap_is_nan<T>(G, h + po)) continue;
+        const T coef = (k == 0) ? (-T(2) * gfy - T(2) * gfx - qk<T>(G).gfc2) : (k < 3 ? gfx : gfy);
         acc += coef * adq[po];
     }
     adh[o] += acc;
@@ -355,12 +418,12 @@ __global__ void k_stage_tl(QGGeom G, int B, const T* __restrict__ hs, const T* _
             const T vp = vT < T(0) ? T(0) : vT, vm = vT > T(0) ? T(0) : vT;
             const T dup = uT < T(0) ? T(0) : duT, dum = uT > T(0) ? T(0) : duT;
             const T dvp = vT < T(0) ? T(0) : dvT, dvm = vT > T(0) ? T(0) : dvT;
-            const T cx = T(G.cx), cy = T(G.cy);
+            const T cx = qk<T>(G).cx, cy = qk<T>(G).cy;
             dr = -dup * cx * qa.Dpx() + dum * cx * qa.Dmx() - dvp * cy * qa.Dpy() + dvm * cy * qa.Dmy()
                  - up * cx * dq.Dpx() + um * cx * dq.Dmx() - vp * cy * dq.Dpy() + vm * cy * dq.Dmy();
             dr -= beta * ((dV.v0 + dV.v1) / T(2));
             if (G.hasK)
-                dr += T(G.Kx) * (dq.e1 + dq.w1 - T(2) * dq.c) + T(G.Ky) * (dq.n1 + dq.s1 - T(2) * dq.c);
+                dr += qk<T>(G).Kx * (dq.e1 + dq.w1 - T(2) * dq.c) + qk<T>(G).Ky * (dq.n1 + dq.s1 - T(2) * dq.c);
         }
     }
     if (qlo) {
@@ -688,7 +751,7 @@ k_adj_stage_fused(QGGeom G, int nf, const T* __restrict__ hs, const T* __restric
     // thread: their SSH and PV stencils overlap, so the pair reads 12 h and
     // 14 q values (each point alone 8 and 9) and then runs the single-point
     // arithmetic on each ----
-    const T cx = T(G.cx), cy = T(G.cy), cu = T(G.cu), cv = T(G.cv);
+    const T cx = qk<T>(G).cx, cy = qk<T>(G).cy, cu = qk<T>(G).cu, cv = qk<T>(G).cv;
 #pragma unroll
     for (int k = 0; k < NAL; ++k) {
         const int e = tid + 256 * k;
@@ -837,8 +900,8 @@ k_adj_stage_fused(QGGeom G, int nf, const T* __restrict__ hs, const T* __restric
                          - vp[u + 3] + vm[u]);
             if (hasK) {
                 const T lc = S.lk[Au][Bc];
-                aq += T(G.Kx) * (S.lk[Au][Bc - 1] + S.lk[Au][Bc + 1] - T(2) * lc)
-                    + T(G.Ky) * (S.lk[Au - 1][Bc] + S.lk[Au + 1][Bc] - T(2) * lc);
+                aq += qk<T>(G).Kx * (S.lk[Au][Bc - 1] + S.lk[Au][Bc + 1] - T(2) * lc)
+                    + qk<T>(G).Ky * (S.lk[Au - 1][Bc] + S.lk[Au + 1][Bc] - T(2) * lc);
             }
             const long long o = fo + (long long)j * G.nx + i;
             adq_out[o] = m3b[k][u] ? aq + accv[k][u] : T(0);
@@ -1060,9 +1123,9 @@ __global__ void k_h2uv(QGGeom G, int nf, const T* __restrict__ h, T* __restrict_
     const int nx = G.nx;
     T uu = T(0), vv = T(0);
     if (j >= 1 && j <= G.ny - 2 && i >= 1)
-        uu = T(G.cu) * (h[o + nx - 1] + h[o + nx] - h[o - nx] - h[o - nx - 1]);
+        uu = qk<T>(G).cu * (h[o + nx - 1] + h[o + nx] - h[o - nx] - h[o - nx - 1]);
     if (j >= 1 && i >= 1 && i <= G.nx - 2)
-        vv = T(G.cv) * (h[o + 1] + h[o - nx + 1] - h[o - nx - 1] - h[o - 1]);
+        vv = qk<T>(G).cv * (h[o + 1] + h[o - nx + 1] - h[o - nx - 1] - h[o - 1]);
     u[o] = guard0(uu);
     v[o] = guard0(vv);
 }
@@ -1123,7 +1186,8 @@ struct TrajView {
 // One forward step (stage loop) between explicit buffers.
 template <typename T>
 static int step_once(const vd_qg1l_plan* p, int nf, T* const* hsv, T* const* qsv, T* hnew, T* qnew,
-                     T* const* kbuf, const T* hb, const T* qb, T* spec, cudaStream_t st, bool tangent, T* qlo)
+                     T* const* kbuf, const T* hb, const T* qb, const int* bg_on, T* spec, cudaStream_t st,
+                     bool tangent, T* qlo)
 {
     const int S = p->nstage;
     const int B = tangent ? nf / 2 : nf;
@@ -1152,6 +1216,7 @@ static int step_once(const vd_qg1l_plan* p, int nf, T* const* hsv, T* const* qsv
         SolveArgs a;
         a.src = qo; a.sub = qb; a.sub_batches = B;
         a.out = ho; a.add = hb; a.add_batches = B; a.epi = EPI_H;
+        a.bg_on = bg_on;
         int rc = helmholtz_solve<T>(p, nf, a, spec, st);
         if (rc) return rc;
     }
@@ -1160,7 +1225,7 @@ static int step_once(const vd_qg1l_plan* p, int nf, T* const* hsv, T* const* qsv
 
 template <typename T>
 int advance_impl(const vd_qg1l_plan* p, int nf, T* traj, int traj_steps, int first, int nstep,
-                 const T* hb, const T* qb, T* qlo, Arena& ws, cudaStream_t st)
+                 const T* hb, const T* qb, const int* bg_on, T* qlo, Arena& ws, cudaStream_t st)
 {
     if (first < 0 || nstep < 0 || first + nstep > traj_steps) return VD_ERR_ARG;
     const int S = p->nstage;
@@ -1174,16 +1239,19 @@ int advance_impl(const vd_qg1l_plan* p, int nf, T* traj, int traj_steps, int fir
     for (int n = first; n < first + nstep; ++n) {
         T* hs[4]; T* qs[4];
         for (int s = 0; s < S; ++s) { hs[s] = tv.h(n, s); qs[s] = tv.q(n, s); }
-        int rc = step_once<T>(p, nf, hs, qs, tv.h(n + 1, 0), tv.q(n + 1, 0), kbuf, hb, qb, spec, st, false, qlo);
+        int rc = step_once<T>(p, nf, hs, qs, tv.h(n + 1, 0), tv.q(n + 1, 0), kbuf, hb, qb, bg_on, spec, st, false, qlo);
         if (rc) return rc;
     }
     return VD_OK;
 }
 
-// Forward without trajectory: ping-pong states in the workspace.
+// Forward without trajectory: ping-pong states in the workspace. The first step
+// reads the SSH from h0 (the wall ring of later states is never read); *h_end is
+// the final SSH (h0 itself for nstep = 0). q is overwritten, and so is `spare`
+// (nullable, may be h0: a state buffer taken otherwise).
 template <typename T>
-int forward_nostore(const vd_qg1l_plan* p, int nf, T* h, T* q, int nstep, const T* hb, const T* qb,
-                    T* qlo, Arena& ws, cudaStream_t st, bool tangent)
+int forward_nostore(const vd_qg1l_plan* p, int nf, const T* h0, T* q, int nstep, const T* hb, const T* qb,
+                    const int* bg_on, T* qlo, T* spare, Arena& ws, cudaStream_t st, bool tangent, const T** h_end)
 {
     const int S = p->nstage;
     const long long fb = (long long)nf * p->geom.fs;
@@ -1191,28 +1259,27 @@ int forward_nostore(const vd_qg1l_plan* p, int nf, T* h, T* q, int nstep, const 
     for (int s = 0; s < S; ++s)
         if (need_k(p, s) && !(kbuf[s] = (T*)ws.take(fb * sizeof(T)))) return VD_ERR_WORKSPACE;
     T* hs[4]; T* qs[4];
-    hs[0] = h; qs[0] = q;
     for (int s = 1; s < S; ++s) {
         hs[s] = (T*)ws.take(fb * sizeof(T));
         qs[s] = (T*)ws.take(fb * sizeof(T));
         if (!hs[s] || !qs[s]) return VD_ERR_WORKSPACE;
     }
-    T* h2 = (T*)ws.take(fb * sizeof(T));
+    T* hbuf[2] = {(T*)ws.take(fb * sizeof(T)), spare ? spare : (T*)ws.take(fb * sizeof(T))};
     T* q2 = (T*)ws.take(fb * sizeof(T));
     T* spec = (T*)ws.take(spec_bytes(p, nf));
-    if (!h2 || !q2 || !spec) return VD_ERR_WORKSPACE;
-    T* cur_h = h; T* cur_q = q; T* nxt_h = h2; T* nxt_q = q2;
+    if (!hbuf[0] || !hbuf[1] || !q2 || !spec) return VD_ERR_WORKSPACE;
+    const T* cur_h = h0;
+    T *cur_q = q, *nxt_q = q2;
     for (int n = 0; n < nstep; ++n) {
-        hs[0] = cur_h; qs[0] = cur_q;
-        int rc = step_once<T>(p, nf, hs, qs, nxt_h, nxt_q, kbuf, hb, qb, spec, st, tangent, qlo);
+        hs[0] = const_cast<T*>(cur_h);       // stage 0 only reads it
+        qs[0] = cur_q;
+        T* nxt_h = hbuf[n & 1];
+        int rc = step_once<T>(p, nf, hs, qs, nxt_h, nxt_q, kbuf, hb, qb, bg_on, spec, st, tangent, qlo);
         if (rc) return rc;
-        T* t1 = cur_h; cur_h = nxt_h; nxt_h = t1;
+        cur_h = nxt_h;
         T* t2 = cur_q; cur_q = nxt_q; nxt_q = t2;
     }
-    if (cur_h != h) {
-        VD_CUDA_TRY(cudaMemcpyAsync(h, cur_h, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        VD_CUDA_TRY(cudaMemcpyAsync(q, cur_q, fb * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    }
+    *h_end = cur_h;
     return VD_OK;
 }
 
@@ -1301,12 +1368,13 @@ int rk_stage_adj_impl(const vd_qg1l_plan* p, int nf, const T* hs, const T* qs, i
 
 template <typename T>
 int init_state_impl(const vd_qg1l_plan* p, int nf, int ntan0, const T* h, const T* hb, T* q, T* qb,
-                    T* qlo, cudaStream_t st)
+                    T* qlo, int* bg_on, cudaStream_t st)
 {
-    k_h2pv<T><<<pgrid(p, nf), kBlock, 0, st>>>(p->geom, nf, ntan0, h, hb, q, qlo);
+    k_h2pv<T><<<pgrid(p, nf), kBlock, 0, st>>>(p->geom, nf, ntan0, h, hb, q, qlo, (int*)nullptr);
     VD_LAUNCH_CHECK();
     if (qb) {
-        k_h2pv<T><<<pgrid(p, ntan0), kBlock, 0, st>>>(p->geom, ntan0, ntan0, hb, hb, qb, (T*)nullptr);
+        if (bg_on) VD_CUDA_TRY(cudaMemsetAsync(bg_on, 0, ntan0 * sizeof(int), st));
+        k_h2pv<T><<<pgrid(p, ntan0), kBlock, 0, st>>>(p->geom, ntan0, ntan0, hb, hb, qb, (T*)nullptr, bg_on);
         VD_LAUNCH_CHECK();
     }
     return VD_OK;
@@ -1376,13 +1444,13 @@ int rhs_impl(const vd_qg1l_plan* p, int nf, const T* u, const T* v, const T* q, 
                                   const double*, double, T*, T*, cudaStream_t);                           \
     template int rk_stage_adj_impl<T>(const vd_qg1l_plan*, int, const T*, const T*, int, const T* const*,  \
                                       const double*, int, const T* const*, T*, T*, cudaStream_t);         \
-    template int advance_impl<T>(const vd_qg1l_plan*, int, T*, int, int, int, const T*, const T*, T*,     \
-                                 Arena&, cudaStream_t);                                                   \
-    template int forward_nostore<T>(const vd_qg1l_plan*, int, T*, T*, int, const T*, const T*, T*,        \
-                                    Arena&, cudaStream_t, bool);                                          \
+    template int advance_impl<T>(const vd_qg1l_plan*, int, T*, int, int, int, const T*, const T*,         \
+                                 const int*, T*, Arena&, cudaStream_t);                                   \
+    template int forward_nostore<T>(const vd_qg1l_plan*, int, const T*, T*, int, const T*, const T*,      \
+                                    const int*, T*, T*, Arena&, cudaStream_t, bool, const T**);           \
     template int advance_adj_impl<T>(const vd_qg1l_plan*, int, const T*, int, int, int, T*, T*, Arena&,   \
                                      cudaStream_t);                                                       \
-    template int init_state_impl<T>(const vd_qg1l_plan*, int, int, const T*, const T*, T*, T*, T*,        \
+    template int init_state_impl<T>(const vd_qg1l_plan*, int, int, const T*, const T*, T*, T*, T*, int*,  \
                                     cudaStream_t);                                                        \
     template int init_state_adj_impl<T>(const vd_qg1l_plan*, int, const T*, const T*, T*, cudaStream_t);  \
     template int finalize_impl<T>(const vd_qg1l_plan*, int, const T*, const T*, const T*, double,         \

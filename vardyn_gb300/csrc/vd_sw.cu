@@ -18,10 +18,10 @@
 // The kernels are templates over the arithmetic type: T for the forward,
 // a one-direction dual number for the tangent-linear (jax.jvp of step,
 // sw.py:906-922). The adjoint (jax.vjp, 924-938) recomputes each step from
-// its stored start and runs hand-written transposes: per face the local
-// gradient of the WENO flux (a 6-direction dual number through the same
-// reconstruction code) is scattered with atomics, then a gather kernel
-// transposes the diagnostics. max(u, 0) takes derivative 1/2 at u = 0, the
+// its stored start and runs hand-written transposes, without atomics: a tile
+// kernel forms the local gradient of every face's WENO flux and gathers what
+// reaches its points (k_sw_tend_adj), then k_sw_diag_adj transposes the
+// diagnostics. max(u, 0) takes derivative 1/2 at u = 0, the
 // rule of jax's lax.max.
 #include "vd_internal.cuh"
 
@@ -269,9 +269,16 @@ __device__ __forceinline__ S weno_flux(const S* q, const S& vel, int bits, bool 
     return F;
 }
 
-// Reverse-mode gradients of the reconstructions (the same quotients as the
-// forward): wenoz4 of (q[1..4]) and wenoz6 of (q[0..5]) accumulate dR/dq
-// into g and return R.
+// a / b, where rb = 1 / b is at hand: a product in float64 (a division is 7 FP64
+// instructions, and 9 of them were a third of a face's gradient); in float32 the
+// forward's own quotient. The cells differ by little, so dR/dw is a difference of
+// nearly equal numbers: weights or an R rounded in another way than the forward's
+// move the float32 gradient by as much as its own error (3e-5).
+__device__ __forceinline__ double quo(double a, double, double rb) { return a * rb; }
+__device__ __forceinline__ float quo(float a, float b, float) { return qdiv(a, b); }
+
+// Reverse-mode gradients of the reconstructions: wenoz4 of (q[1..4]) and wenoz6
+// of (q[0..5]) accumulate dR/dq into g and return R.
 template <typename T>
 __device__ __forceinline__ T wenoz4_grad(const T* q, T* g)
 {
@@ -283,11 +290,11 @@ __device__ __forceinline__ T wenoz4_grad(const T* q, T* g)
     const T dd = b2 - b1;
     const T tau = sqrt(dd * dd + T(WENO_EPS * WENO_EPS));
     const T s1 = qdiv(T(1), b1 + T(WENO_EPS)), s2 = qdiv(T(1), b2 + T(WENO_EPS));
-    const T w1 = T(1.0 / 3.0) * (T(1) + qdiv(tau, b1 + T(WENO_EPS)));
-    const T w2 = T(2.0 / 3.0) * (T(1) + qdiv(tau, b2 + T(WENO_EPS)));
+    const T w1 = T(1.0 / 3.0) * (T(1) + quo(tau, b1 + T(WENO_EPS), s1));
+    const T w2 = T(2.0 / 3.0) * (T(1) + quo(tau, b2 + T(WENO_EPS), s2));
     const T W = w1 + w2;
-    const T R = qdiv(w1 * q1 + w2 * q2, W);
     const T iW = qdiv(T(1), W);
+    const T R = quo(w1 * q1 + w2 * q2, W, iW);
     const T aw1 = (q1 - R) * iW, aw2 = (q2 - R) * iW;       // dR/dw
     const T ar1 = w1 * iW, ar2 = w2 * iW;                    // dR/dq1, dR/dq2
     const T atau = aw1 * T(1.0 / 3.0) * s1 + aw2 * T(2.0 / 3.0) * s2;
@@ -317,19 +324,27 @@ __device__ __forceinline__ T wenoz6_grad(const T* q, T* g)
     const T dd = b1 - b3;
     const T tau = sqrt(dd * dd + T(WENO_EPS * WENO_EPS));
     const T s1 = qdiv(T(1), b1 + T(WENO_EPS)), s2 = qdiv(T(1), b2 + T(WENO_EPS)), s3 = qdiv(T(1), b3 + T(WENO_EPS));
-    const T w1 = T(0.1) * (T(1) + qdiv(tau, b1 + T(WENO_EPS)));
-    const T w2 = T(0.6) * (T(1) + qdiv(tau, b2 + T(WENO_EPS)));
-    const T w3 = T(0.3) * (T(1) + qdiv(tau, b3 + T(WENO_EPS)));
+    const T w1 = T(0.1) * (T(1) + quo(tau, b1 + T(WENO_EPS), s1));
+    const T w2 = T(0.6) * (T(1) + quo(tau, b2 + T(WENO_EPS), s2));
+    const T w3 = T(0.3) * (T(1) + quo(tau, b3 + T(WENO_EPS), s3));
     const T W = w1 + w2 + w3;
-    const T R = qdiv(w1 * r1 + w2 * r2 + w3 * r3, W);
     const T iW = qdiv(T(1), W);
+    const T R = quo(w1 * r1 + w2 * r2 + w3 * r3, W, iW);
     const T aw1 = (r1 - R) * iW, aw2 = (r2 - R) * iW, aw3 = (r3 - R) * iW;
     const T ar1 = w1 * iW, ar2 = w2 * iW, ar3 = w3 * iW;
-    const T atau = aw1 * T(0.1) * s1 + aw2 * T(0.6) * s2 + aw3 * T(0.3) * s3;
     const T dtau = qdiv(dd, tau);
-    const T ab1 = -aw1 * T(0.1) * tau * s1 * s1 + atau * dtau;
-    const T ab2 = -aw2 * T(0.6) * tau * s2 * s2;
-    const T ab3 = -aw3 * T(0.3) * tau * s3 * s3 - atau * dtau;
+    T ab1, ab2, ab3;
+    if constexpr (sizeof(T) == 4) {
+        const T atau = aw1 * T(0.1) * s1 + aw2 * T(0.6) * s2 + aw3 * T(0.3) * s3;
+        ab1 = -aw1 * T(0.1) * tau * s1 * s1 + atau * dtau;
+        ab2 = -aw2 * T(0.6) * tau * s2 * s2;
+        ab3 = -aw3 * T(0.3) * tau * s3 * s3 - atau * dtau;
+    } else {   // the same with the common products taken once (FP64 issue)
+        const T z1 = aw1 * T(0.1) * s1, z2 = aw2 * T(0.6) * s2, z3 = aw3 * T(0.3) * s3, at = (z1 + z2 + z3) * dtau;
+        ab1 = at - z1 * (tau * s1);
+        ab2 = -z2 * (tau * s2);
+        ab3 = -at - z3 * (tau * s3);
+    }
     const T c1 = T(2) * k1 * d1 * ab1, h1 = T(2) * k2 * f1 * ab1;
     const T c2 = T(2) * k1 * d2 * ab2, h2 = T(2) * k2 * f2 * ab2;
     const T c3 = T(2) * k1 * d3 * ab3, h3 = T(2) * k2 * f3 * ab3;
@@ -342,13 +357,12 @@ __device__ __forceinline__ T wenoz6_grad(const T* q, T* g)
     return R;
 }
 
-// Local gradient of the face flux: dF/dq[0..5], dF/dvel.
+// Cotangents of the face flux F for a cotangent a: a dF/dq[0..5] into s (0 where a
+// cell is not in the stencil, also for an infinite a) and dF/dvel.
 template <typename T>
-__device__ __forceinline__ void weno_flux_grad(const T* q, T vel, int bits, bool ok4, bool ok6, T* g, T& gv)
+__device__ __forceinline__ void weno_flux_adj(const T* q, T vel, int bits, bool ok4, bool ok6, T a, T* s, T& gv)
 {
-#pragma unroll
-    for (int k = 0; k < 6; ++k) g[k] = T(0);
-    if (vel == T(0)) {
+    if (vel == T(0)) {   // both directions, weight 1/2; no dependence on q
         const T P = recon<T>(q, bits, ok4, ok6, false), M = recon<T>(q, bits, ok4, ok6, true);
         gv = T(0.5) * (P + M);
         return;
@@ -368,8 +382,17 @@ __device__ __forceinline__ void weno_flux_grad(const T* q, T vel, int bits, bool
     }
     if ((bits & 2) && ok4) R = R + wenoz4_grad(qq, gg);
     if ((bits & 4) && ok6) R = R + wenoz6_grad(qq, gg);
+    const T c = a * vel;
+    if (c - c == T(0)) {
 #pragma unroll
-    for (int k = 0; k < 6; ++k) g[k] = vel * (rev ? gg[5 - k] : gg[k]);
+        for (int k = 0; k < 6; ++k) s[k] = c * (rev ? gg[5 - k] : gg[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const T gk = rev ? gg[5 - k] : gg[k];
+            s[k] = gk != T(0) ? c * gk : T(0);
+        }
+    }
     gv = R;
 }
 
@@ -449,6 +472,10 @@ struct WD {
     __device__ __forceinline__ WD at(long long o) const { return WD{p ? p + o : p, d ? d + o : d}; }
 };
 
+template <typename T>
+struct Fields {
+    T *u, *v, *h;
+};
 template <typename R> struct Tri { R u, v, h; };
 
 // A table value as the kernel's arithmetic type: the plain value, or for the
@@ -503,16 +530,26 @@ __global__ void k_sw_diag(Tab<T> t, Tri<R> x, W om, W kp, W ht)
                             vr * (vr * t.idyv2[wi])) * mh;
     // eta_l = sum_{m>=l} h_m / area; p_l = sum_{k<=l} g'_k eta_k (sw.py:705-706)
     S eta[MAXL], pacc = T(0) * h(0), acc{};
+    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-    for (int k = 0; k < MAXL; ++k) eta[k] = k < nl ? h((long long)k * sh + ui) : S{};
+        for (int k = 0; k < MAXL; ++k) eta[k] = k < nl ? h((long long)k * sh + ui) : S{};
 #pragma unroll
-    for (int k = MAXL - 1; k >= 0; --k) {
-        acc = eta[k] * iar + acc;
-        eta[k] = acc;
+        for (int k = MAXL - 1; k >= 0; --k) {
+            acc = eta[k] * iar + acc;
+            eta[k] = acc;
+        }
+#pragma unroll
+        for (int k = 0; k < MAXL; ++k)
+            if (k <= l) pacc = pacc + t.gp[k] * eta[k];
+    } else {   // an FP64 instruction of an absent layer costs its issue slot: loops over those there are
+#pragma unroll 1
+        for (int k = nl - 1; k >= 0; --k) {
+            acc = h((long long)k * sh + ui) * iar + acc;
+            eta[k] = acc;
+        }
+#pragma unroll 1
+        for (int k = 0; k <= l; ++k) pacc = pacc + t.gp[k] * eta[k];
     }
-#pragma unroll
-    for (int k = 0; k < MAXL; ++k)
-        if (k <= l) pacc = pacc + t.gp[k] * eta[k];
     kp.at(ob * t.sh)(ui, ke + pacc);
     const S hr = VD_TAB(S, t.href, t.d_href, (long long)l * t.sh + ui);
     if (t.linear) ht.at(ob * t.sh)(ui, hr + T(0) * hl);
@@ -863,50 +900,63 @@ __global__ void k_sw_scale(Tab<T> t, int nf, int mode, const T* u, const T* v, c
 
 // ------------------------------------------------------------------ adjoint kernels
 // Reverse of k_sw_update for one stage (elementwise): from the adjoint of the
-// stage output (adn, updated in place to the adjoint of the stage input's
-// direct path) build adk (adjoint of this stage's k) and accumulate the
-// adjoints of the earlier k's and of the sponge target.
+// stage output (an, updated in place to the adjoint of the stage input's
+// direct path) build ak (adjoint of this stage's k) and accumulate the
+// adjoints of the earlier k's and of the sponge target. FRESH: the sums a0 and a1
+// start here (stage 2 of a step) and are written instead of added to.
 template <typename T>
-__global__ void k_sw_update_adj(Tab<T> t, int stage, int nf, T* adn_u, T* adn_v, T* adn_h, T* adk_u, T* adk_v,
-                                T* adk_h, T* a0_u, T* a0_v, T* a0_h, T* a1_u, T* a1_v, T* a1_h, T* ab_u, T* ab_v,
-                                T* ab_h)
+struct UpdAdj {
+    int stage, fresh;
+    Fields<T> ak, a0, a1, ab;
+};
+
+template <typename T>
+__device__ __forceinline__ void upd_adj_point(const Tab<T>& t, int stage, bool fresh, T a, long long o, const T* gam,
+                                              int g, T* an, bool store, T* ak, T* a0, T* a1, T* ab)
+{
+    const T dt = t.dt;
+    T k;
+    if (stage == 2) {
+        k = (dt / T(12)) * T(8) * a;
+        const T c = -(dt / T(12)) * a;
+        a1[o] = fresh ? c : a1[o] + c;
+        a0[o] = fresh ? c : a0[o] + c;
+    } else if (stage == 1) {
+        k = a1[o] + (dt / T(4)) * a;
+        a0[o] += -(dt / T(4)) * T(3) * a;
+    } else {
+        k = a0[o] + dt * a;
+    }
+    ak[o] = k;
+    if (t.has_sponge) {
+        const T gk = gam[g];
+        an[o] = a - gk * k;
+        if (ab) ab[o] += gk * k;
+    } else if (store) {
+        an[o] = a;
+    }
+}
+
+template <typename T>
+__global__ void k_sw_update_adj(Tab<T> t, UpdAdj<T> n, int nf, Fields<T> ad)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y * blockDim.y + threadIdx.y;
     const int f = blockIdx.z;
     const int nx = t.nx, ny = t.ny;
     if (i > nx || j > ny || f >= nf) return;
-    const T dt = t.dt;
-    auto one = [&](long long o, T g, T* an, T* ak, T* a0, T* a1, T* ab) {
-        const T a = an[o];
-        T k;
-        if (stage == 2) {
-            k = (dt / T(12)) * T(8) * a;
-            a1[o] += -(dt / T(12)) * a;
-            a0[o] += -(dt / T(12)) * a;
-        } else if (stage == 1) {
-            k = a1[o] + (dt / T(4)) * a;
-            a0[o] += -(dt / T(4)) * T(3) * a;
-        } else {
-            k = a0[o] + dt * a;
-        }
-        ak[o] = k;
-        if (t.has_sponge) {
-            an[o] = a - g * k;
-            if (ab) ab[o] += g * k;
-        }
-    };
+    const int ui = i * ny + j, vi = i * (ny + 1) + j;
     if (j < ny) {
-        const long long k = (long long)i * ny + j;
-        one(f * t.su + k, t.has_sponge ? t.gu[k] : T(0), adn_u, adk_u, a0_u, a1_u, ab_u);
+        const long long o = f * t.su + ui;
+        upd_adj_point<T>(t, n.stage, n.fresh, ad.u[o], o, t.gu, ui, ad.u, false, n.ak.u, n.a0.u, n.a1.u, n.ab.u);
     }
     if (i < nx) {
-        const long long k = (long long)i * (ny + 1) + j;
-        one(f * t.sv + k, t.has_sponge ? t.gv[k] : T(0), adn_v, adk_v, a0_v, a1_v, ab_v);
+        const long long o = f * t.sv + vi;
+        upd_adj_point<T>(t, n.stage, n.fresh, ad.v[o], o, t.gv, vi, ad.v, false, n.ak.v, n.a0.v, n.a1.v, n.ab.v);
     }
     if (i < nx && j < ny) {
-        const long long k = (long long)i * ny + j;
-        one(f * t.sh + k, t.has_sponge ? t.gh[k] : T(0), adn_h, adk_h, a0_h, a1_h, ab_h);
+        const long long o = f * t.sh + ui;
+        upd_adj_point<T>(t, n.stage, n.fresh, ad.h[o], o, t.gh, ui, ad.h, false, n.ak.h, n.a0.h, n.a1.h, n.ab.h);
     }
 }
 
@@ -914,358 +964,376 @@ __global__ void k_sw_update_adj(Tab<T> t, int stage, int nf, T* adn_u, T* adn_v,
 // h_wind table cotangents and by the mass-consistent forcing adjoint.
 template <typename T> __device__ __forceinline__ void aadd(T* p, T v) { atomicAdd(p, v); }
 
-// Adjoint of k_sw_tend and of the divergence / diffusion part of
-// k_sw_update, in two passes with no atomics.
-//
-// Pass 1 (k_sw_tend_adj_src, one thread per point): every source point of
-// the forward tendency stores the cotangents it contributes, one value per
-// (source, term): at u faces the tendency cotangent a (KE + pressure, drag),
-// a * dF/dq_k of its vorticity WENO flux (k = 0..5), the V-average term, the
-// viscosity coefficient, aF * dF/dq_k of the thickness flux through the face
-// and the face's own flux-velocity term; the same at v faces; and the
-// thickness-diffusion coefficient at h points. Every index in range is
-// written (zeros where a point contributes nothing).
-// Pass 2 (k_sw_tend_adj_gather, one thread per target point): each target
-// sums, in a fixed order, the stored terms of the sources whose stencils
-// reach it (the inverse of each forward stencil, including the clamped
-// viscosity and diffusion neighbours at the edges). The sums are therefore
-// the same on every run. The H / h_wind table cotangents (only when
-// registered) still accumulate with atomics over the batch.
+// Adjoint of k_sw_tend and of the divergence / diffusion part of k_sw_update,
+// without atomics: one block owns a tile of ADJ_TI x ADJ_TJ targets of every kind
+// (vorticity, h, u, v) and forms, in four passes, the local gradients of the faces
+// whose stencils reach its targets: u faces' vorticity fluxes (reaching along y),
+// v faces' (along x), and the two thickness fluxes. A pass leaves a face's six
+// cotangents a * dF/dq_k and its velocity term in shared memory, then every target
+// sums those that reach it in a fixed order, so the sums are the same on every run.
+// A pass's halo is 5 faces along its own stencil alone: 20 % more faces than
+// targets at 24 x 32. The sums used to go through memory between two kernels (33
+// values a point written and read again, 620 MB a stage at 3 x 1024 x 768
+// float32): 206 + 169 us; here 245 us, bound by issue and by how many warps
+// cover the faces' loads: tiles of 16 rows with 3, 4 and 5 blocks an SM 322, 257 and
+// 253 us, 24 rows 303, 249 and 241 (48 registers, 10 of them spilled once). The
+// H / h_wind table cotangents (only when registered) accumulate with atomics over
+// the batch, each face in the block that owns it.
+#ifdef __CUDACC__
+constexpr int ADJ_NT = 256;
+#else
+constexpr int ADJ_NT = 1;   // host build: one thread runs a block's loops, pass by pass
+#endif
+constexpr int ADJ_TJ = 32;
+// float64 is bound by the FP64 pipe, where each halo face costs: 32 rows (17 % halo)
+// and 98 KB of shared memory a block (4.87 ms; 8 rows, 44 % halo, 5.77; the two
+// kernels 4.83); float32 24 rows and 38 KB
+template <typename T> constexpr int adj_ti = sizeof(T) == 4 ? 24 : 32;
+template <typename T> constexpr int adj_nf =   // faces of the largest pass
+    (adj_ti<T> + 5) * (ADJ_TJ + 1) > (adj_ti<T> + 1) * (ADJ_TJ + 5) ? (adj_ti<T> + 5) * (ADJ_TJ + 1)
+                                                                    : (adj_ti<T> + 1) * (ADJ_TJ + 5);
+template <typename T> constexpr int adj_smem =   // elements of shared memory
+    2 * (adj_ti<T> + 2) * (ADJ_TJ + 2) + (adj_ti<T> + 6) * (ADJ_TJ + 6) + 7 * adj_nf<T>;
 
 template <typename T>
-struct SwSrc {
-    T *ua, *uvm, *uc, *uf;   // [bl][su] u faces: a, V-average term, viscosity coefficient, own flux term
-    T *uw, *uh;              // [6][bl][su]: vorticity and thickness WENO terms
-    T *va, *vum, *vc, *vf;   // [bl][sv] v faces
-    T *vw, *vh;              // [6][bl][sv]
-    T *hd;                   // [bl][sh] thickness-diffusion coefficient
-    long long nu, nv;        // bl * su, bl * sv: stride of the six-term arrays
-};
-
-template <typename T>
-__global__ void k_sw_tend_adj_src(Tab<T> t, const T* u, const T* v, const T* h, const T* om, const T* ht,
-                                  const T* adk_u, const T* adk_v, const T* adk_h, SwSrc<T> S, const T* taux,
-                                  const T* tauy)
+__global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(Tab<T> t, const T* u, const T* v, const T* om, const T* ht,
+                                                        const T* adk_u, const T* adk_v, const T* adk_h, T* adom,
+                                                        T* adkp, T* adht, T* adu, T* adv, T* adh, const T* taux,
+                                                        const T* tauy)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    const int bl = blockIdx.z;
-    const int nx = t.nx, ny = t.ny, nl = t.nl, l = bl % nl;
-    if (i > nx || j > ny) return;
-    const long long ob = bl;
-    const T* hb = adk_h + ob * t.sh;
-    auto mh = [&](long long k) { return (t.fh[k] & 1) ? T(1) : T(0); };
-    // ---------------- u face (i, j)
-    if (j < ny) {
-        const long long ui = (long long)i * ny + j, so = ob * t.su + ui;
-        T a_s = T(0), vm_s = T(0), c_s = T(0), f_s = T(0), w_s[6], h_s[6];
+    constexpr int TI = adj_ti<T>, TJ = ADJ_TJ, RPT = TI * TJ / ADJ_NT;
+    constexpr int AC = TJ + 2, HC = TJ + 6;           // row lengths of the tiles of a and of the masked h cotangent
+    constexpr int CA = TJ + 5, CB = TJ + 1;           // row lengths of passes A (u faces, omega), B (v faces, omega)
+    constexpr int NF = adj_nf<T>;
+#ifdef __CUDACC__
+    extern __shared__ __align__(16) unsigned char adj_pool[];
+    T* const s_au = (T*)adj_pool;
+#else
+    T s_au[adj_smem<T>];
+#endif
+    T* const s_av = s_au + (TI + 2) * AC;
+    T* const s_hm = s_av + (TI + 2) * AC;
+    T(*const S)[NF] = (T(*)[NF])(s_hm + (TI + 6) * HC);
+    const int tid = threadIdx.x;
+    const int j0 = blockIdx.x * TJ, i0 = blockIdx.y * TI;
+    const int nx = t.nx, ny = t.ny, nl = t.nl, n1 = ny + 1;
+    const long long ob = blockIdx.z;
+    const int l = (int)(blockIdx.z % (unsigned)nl);
+    u += ob * t.su; adk_u += ob * t.su; adu += ob * t.su;
+    v += ob * t.sv; adk_v += ob * t.sv; adv += ob * t.sv;
+    om += ob * t.sw; adom += ob * t.sw;
+    ht += ob * t.sh; adk_h += ob * t.sh; adkp += ob * t.sh; adht += ob * t.sh; adh += ob * t.sh;
+
+    // ---- masked tendency cotangents of the interior u / v faces and of h around the tile (0 elsewhere)
+    for (int e = tid; e < (TI + 2) * AC; e += ADJ_NT) {
+        const int i = i0 - 1 + e / AC, j = j0 - 1 + e % AC;
+        T a = T(0), b = T(0);
+        if (i >= 1 && i <= nx - 1 && j >= 0 && j < ny) {
+            const int k = i * ny + j;
+            a = adk_u[k] * ((t.fu[k] & 1) ? T(1) : T(0));
+        }
+        if (i >= 0 && i < nx && j >= 1 && j <= ny - 1) {
+            const int k = i * n1 + j;
+            b = adk_v[k] * ((t.fv[k] & 1) ? T(1) : T(0));
+        }
+        s_au[e] = a;
+        s_av[e] = b;
+    }
+    for (int e = tid; e < (TI + 6) * HC; e += ADJ_NT) {
+        const int i = i0 - 3 + e / HC, j = j0 - 3 + e % HC;
+        T a = T(0);
+        if (i >= 0 && i < nx && j >= 0 && j < ny) {
+            const int k = i * ny + j;
+            a = adk_h[k] * ((t.fh[k] & 1) ? T(1) : T(0));
+        }
+        s_hm[e] = a;
+    }
+
+    // ---- pass A: vorticity fluxes of the u faces (i0 + r, j0 - 3 + c)
+    for (int e = tid; e < (TI + 1) * CA; e += ADJ_NT) {
+        const int i = i0 + e / CA, j = j0 - 3 + e % CA;
+        T ws[6], vm = T(0);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) w_s[k] = h_s[k] = T(0);
-        if (i >= 1 && i <= nx - 1) {
+        for (int k = 0; k < 6; ++k) ws[k] = T(0);
+        if (i >= 1 && i <= nx - 1 && j >= 0 && j < ny) {
+            const int ui = i * ny + j, vi = i * n1 + j;
             const int fl = t.fu[ui];
-            const T a = adk_u[so] * ((fl & 1) ? T(1) : T(0));
+            // (all loads before the branch on a: one wait instead of two)
+            const T a = adk_u[ui] * ((fl & 1) ? T(1) : T(0));
+            auto Vv = [&](int k) { return v[k] * t.idyv2[k]; };
+            const T Vm = T(0.25) * (Vv(vi + 1) + Vv(vi) + Vv(vi - n1 + 1) + Vv(vi - n1));
+            T q[6], gv;
+            ring6(q, R1<T>{om}, vi, 1, j - 2, ny);
             if (a != T(0)) {
-                const long long vb = ob * t.sv;
-                auto Vv = [&](int p, int c) {
-                    const long long k = (long long)p * (ny + 1) + c;
-                    return v[vb + k] * t.idyv2[k];
-                };
-                const T Vm = T(0.25) * (Vv(i, j + 1) + Vv(i, j) + Vv(i - 1, j + 1) + Vv(i - 1, j));
-                T q[6];
-                const long long wb = ob * t.sw + (long long)i * (ny + 1);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int jj = j - 2 + k;
-                    q[k] = (jj >= 0 && jj <= ny) ? om[wb + jj] : T(0);
-                }
-                T g[6], gv;
-                weno_flux_grad<T>(q, Vm, (fl >> 4) & 7, j >= 1 && j <= ny - 2, j >= 2 && j <= ny - 3, g, gv);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int jj = j - 2 + k;
-                    if (jj >= 0 && jj <= ny && g[k] != T(0)) w_s[k] = a * g[k];
-                }
-                vm_s = T(0.25) * a * (gv + t.fsu[ui]);
-                a_s = a;
+                weno_flux_adj<T>(q, Vm, (fl >> 4) & 7, j >= 1 && j <= ny - 2, j >= 2 && j <= ny - 3, a, ws, gv);
+                vm = T(0.25) * a * (gv + t.fsu[ui]);
                 // reference pressure gradient and wind factor (H / h_wind cotangents)
-                if (t.ad_dxp && t.hxy_dxp)
-                    aadd(&t.ad_dxp[(long long)l * (nx - 1) * ny + (long long)(i - 1) * ny + j], -a);
-                if (t.ad_wfu && l == 0) aadd(&t.ad_wfu[ui], a * (taux ? taux : t.taux)[(long long)(i - 1) * ny + j]);
-                if (t.visc > T(0)) c_s = t.visc * t.dxu[ui] * a;
-            }
-            // thickness flux through u face i: dt_h[c] = -div_x[c] * mask_h[c]
-            T aF = T(0);
-            if (i - 1 >= 1 && i - 1 <= nx - 2) aF -= mh((long long)(i - 1) * ny + j) * hb[(long long)(i - 1) * ny + j];
-            if (i >= 1 && i <= nx - 2) aF += mh(ui) * hb[ui];
-            if (aF != T(0)) {
-                const T iu2 = t.idxu2[ui];
-                const T Uf = u[so] * iu2;
-                T q[6];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int ii = i - 3 + k;
-                    q[k] = (ii >= 0 && ii < nx) ? ht[ob * t.sh + (long long)ii * ny + j] : T(0);
+                if (i < i0 + TI && j >= j0 && j < j0 + TJ) {
+                    if (t.ad_dxp && t.hxy_dxp) aadd(&t.ad_dxp[(long long)l * (nx - 1) * ny + ui - ny], -a);
+                    if (t.ad_wfu && l == 0) aadd(&t.ad_wfu[ui], a * (taux ? taux : t.taux)[ui - ny]);
                 }
-                T g[6], gv;
-                weno_flux_grad<T>(q, Uf, (fl >> 1) & 7, i >= 2 && i <= nx - 2, i >= 3 && i <= nx - 3, g, gv);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int ii = i - 3 + k;
-                    if (ii >= 0 && ii < nx && g[k] != T(0)) h_s[k] = aF * g[k];
-                }
-                f_s = aF * gv * iu2;
             }
         }
-        S.ua[so] = a_s;
-        S.uvm[so] = vm_s;
-        S.uc[so] = c_s;
-        S.uf[so] = f_s;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            S.uw[k * S.nu + so] = w_s[k];
-            S.uh[k * S.nu + so] = h_s[k];
+        for (int k = 0; k < 6; ++k) S[k][e] = ws[k];
+        S[6][e] = vm;
+    }
+    __syncthreads();
+    T a_om[RPT], a_h[RPT], a_u[RPT], a_v[RPT];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+        const int e = q * ADJ_NT + tid, ti = e / TJ, tj = e % TJ, i = i0 + ti, j = j0 + tj;
+        a_om[q] = a_h[q] = a_u[q] = a_v[q] = T(0);
+        // vorticity point (i, j): u face (i, j+2-k) reaches it with term k
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a_om[q] += S[k][ti * CA + tj + 5 - k];
+        const int o = ti * CA + tj + 3;
+        if (i < nx && j <= ny) {
+            // V-average of the u faces (i, j-1), (i, j), (i+1, j-1), (i+1, j)
+            const T iv2 = t.idyv2[i * n1 + j];
+            a_v[q] = (S[6][o - 1] + S[6][o] + S[6][o + CA - 1] + S[6][o + CA]) * iv2;
+        }
+        const int ea = (ti + 1) * AC + tj + 1, eh = (ti + 3) * HC + tj + 3;
+        if (i < nx && j < ny) {
+            // KE + pressure: u faces i (-a) and i+1 (+a), v faces j (-a) and j+1 (+a)
+            const int hi = i * ny + j;
+            adkp[hi] = (-s_au[ea] + s_au[ea + AC]) + (-s_av[ea] + s_av[ea + 1]);
+            if (t.diff > T(0)) {
+                // the diffusion stencil of cell (p, c): (p+-1, c), (p, c+-1) clamped to the grid, and (p, c)
+                auto D = [&](int e2, int k) { return s_hm[e2] * t.area[k]; };
+                const T ix2 = t.idx2h[hi], iy2 = t.idy2h[hi];
+                T w = -T(2) * ix2 - T(2) * iy2, s = T(0);
+                if (i >= 1) s += D(eh - HC, hi - ny) * t.idx2h[hi - ny];
+                else w += ix2;
+                if (i + 1 <= nx - 1) s += D(eh + HC, hi + ny) * t.idx2h[hi + ny];
+                else w += ix2;
+                if (j >= 1) s += D(eh - 1, hi - 1) * t.idy2h[hi - 1];
+                else w += iy2;
+                if (j + 1 <= ny - 1) s += D(eh + 1, hi + 1) * t.idy2h[hi + 1];
+                else w += iy2;
+                s += D(eh, hi) * w;
+                adh[hi] += t.diff * t.iarea[hi] * s;
+            }
         }
     }
-    // ---------------- v face (i, j)
-    if (i < nx) {
-        const long long vi = (long long)i * (ny + 1) + j, so = ob * t.sv + vi;
-        T a_s = T(0), um_s = T(0), c_s = T(0), f_s = T(0), w_s[6], h_s[6];
+    __syncthreads();
+
+    // ---- pass B: vorticity fluxes of the v faces (i0 - 3 + r, j0 + c)
+    for (int e = tid; e < (TI + 5) * CB; e += ADJ_NT) {
+        const int i = i0 - 3 + e / CB, j = j0 + e % CB;
+        T ws[6], um = T(0);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) w_s[k] = h_s[k] = T(0);
-        if (j >= 1 && j <= ny - 1) {
+        for (int k = 0; k < 6; ++k) ws[k] = T(0);
+        if (i >= 0 && i < nx && j >= 1 && j <= ny - 1) {
+            const int ui = i * ny + j, vi = i * n1 + j;
             const int fl = t.fv[vi];
-            const T a = adk_v[so] * ((fl & 1) ? T(1) : T(0));
+            const T a = adk_v[vi] * ((fl & 1) ? T(1) : T(0));
+            auto Uu = [&](int k) { return u[k] * t.idxu2[k]; };
+            const T Um = T(0.25) * (Uu(ui + ny) + Uu(ui + ny - 1) + Uu(ui) + Uu(ui - 1));
+            T q[6], gv;
+            ring6(q, R1<T>{om}, vi, n1, i - 2, nx);
             if (a != T(0)) {
-                const long long ub = ob * t.su;
-                auto Uu = [&](int p, int c) {
-                    const long long k = (long long)p * ny + c;
-                    return u[ub + k] * t.idxu2[k];
-                };
-                const T Um = T(0.25) * (Uu(i + 1, j) + Uu(i + 1, j - 1) + Uu(i, j) + Uu(i, j - 1));
-                T q[6];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int ii = i - 2 + k;
-                    q[k] = (ii >= 0 && ii <= nx) ? om[ob * t.sw + (long long)ii * (ny + 1) + j] : T(0);
+                weno_flux_adj<T>(q, Um, (fl >> 4) & 7, i >= 1 && i <= nx - 2, i >= 2 && i <= nx - 3, -a, ws, gv);
+                um = -T(0.25) * a * (gv + t.fsv[vi]);
+                if (i >= i0 && i < i0 + TI && j < j0 + TJ) {
+                    const int pk = i * (ny - 1) + j - 1;
+                    if (t.ad_dyp && t.hxy_dyp) aadd(&t.ad_dyp[(long long)l * nx * (ny - 1) + pk], -a);
+                    if (t.ad_wfv && l == 0) aadd(&t.ad_wfv[vi], a * (tauy ? tauy : t.tauy)[pk]);
                 }
-                T g[6], gv;
-                weno_flux_grad<T>(q, Um, (fl >> 4) & 7, i >= 1 && i <= nx - 2, i >= 2 && i <= nx - 3, g, gv);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int ii = i - 2 + k;
-                    if (ii >= 0 && ii <= nx && g[k] != T(0)) w_s[k] = -a * g[k];
-                }
-                um_s = -T(0.25) * a * (gv + t.fsv[vi]);
-                a_s = a;
-                if (t.ad_dyp && t.hxy_dyp)
-                    aadd(&t.ad_dyp[(long long)l * nx * (ny - 1) + (long long)i * (ny - 1) + j - 1], -a);
-                if (t.ad_wfv && l == 0) aadd(&t.ad_wfv[vi], a * (tauy ? tauy : t.tauy)[(long long)i * (ny - 1) + j - 1]);
-                if (t.visc > T(0)) c_s = t.visc * t.dyv[vi] * a;
             }
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) S[k][e] = ws[k];
+        S[6][e] = um;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+        const int e = q * ADJ_NT + tid, ti = e / TJ, tj = e % TJ, i = i0 + ti, j = j0 + tj;
+        // vorticity point (i, j): v face (i+2-k, j) reaches it with term k
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a_om[q] += S[k][(ti + 5 - k) * CB + tj];
+        if (i <= nx && j <= ny) adom[i * n1 + j] = a_om[q];
+        if (i <= nx && j < ny) {
+            // U-average of the v faces (i-1, j), (i-1, j+1), (i, j), (i, j+1)
+            const int o = (ti + 2) * CB + tj;
+            const T iu2 = t.idxu2[i * ny + j];
+            a_u[q] = (S[6][o] + S[6][o + 1] + S[6][o + CB] + S[6][o + CB + 1]) * iu2;
+        }
+    }
+    __syncthreads();
+
+    // ---- pass C: thickness fluxes of the u faces (i0 - 2 + r, j0 + c)
+    for (int e = tid; e < (TI + 5) * TJ; e += ADJ_NT) {
+        const int r = e / TJ, c = e % TJ, i = i0 - 2 + r, j = j0 + c;
+        T hs[6], f = T(0);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) hs[k] = T(0);
+        if (i >= 1 && i <= nx - 1 && j < ny) {
+            // dt_h[c] = -div_x[c] * mask_h[c], no x contribution in the first and last cells
             T aF = T(0);
-            const long long hj0 = (long long)i * ny + j - 1, hj1 = (long long)i * ny + j;
-            if (j - 1 >= 1 && j - 1 <= ny - 2) aF -= mh(hj0) * hb[hj0];
-            if (j >= 1 && j <= ny - 2) aF += mh(hj1) * hb[hj1];
+            if (i - 1 >= 1) aF -= s_hm[r * HC + c + 3];
+            if (i <= nx - 2) aF += s_hm[(r + 1) * HC + c + 3];
+            const int ui = i * ny + j, fl = t.fu[ui];
+            const T iu2 = t.idxu2[ui];
+            const T Uf = u[ui] * iu2;
+            T q[6], gv;
+            ring6(q, R1<T>{ht}, ui - ny, ny, i - 3, nx - 1);
             if (aF != T(0)) {
-                const T iv2 = t.idyv2[vi];
-                const T Vf = v[so] * iv2;
-                T q[6];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int jj = j - 3 + k;
-                    q[k] = (jj >= 0 && jj < ny) ? ht[ob * t.sh + (long long)i * ny + jj] : T(0);
-                }
-                T g[6], gv;
-                weno_flux_grad<T>(q, Vf, (fl >> 1) & 7, j >= 2 && j <= ny - 2, j >= 3 && j <= ny - 3, g, gv);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int jj = j - 3 + k;
-                    if (jj >= 0 && jj < ny && g[k] != T(0)) h_s[k] = aF * g[k];
-                }
-                f_s = aF * gv * iv2;
+                weno_flux_adj<T>(q, Uf, (fl >> 1) & 7, i >= 2 && i <= nx - 2, i >= 3 && i <= nx - 3, aF, hs, gv);
+                f = aF * gv * iu2;
             }
         }
-        S.va[so] = a_s;
-        S.vum[so] = um_s;
-        S.vc[so] = c_s;
-        S.vf[so] = f_s;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            S.vw[k * S.nv + so] = w_s[k];
-            S.vh[k * S.nv + so] = h_s[k];
+        for (int k = 0; k < 6; ++k) S[k][e] = hs[k];
+        S[6][e] = f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+        const int e = q * ADJ_NT + tid, ti = e / TJ, tj = e % TJ, i = i0 + ti, j = j0 + tj;
+        // h point (i, j): u face (i+3-k, j) reaches it with term k
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a_h[q] += S[k][(ti + 5 - k) * TJ + tj];
+        if (i <= nx && j < ny) {
+            const int ui = i * ny + j, ea = (ti + 1) * AC + tj + 1;
+            T s = a_u[q];
+            if (l == nl - 1) s += -t.drag * s_au[ea];
+            if (t.visc > T(0)) {
+                // viscosity stencil of u face (p, c): (p+-1, c), (p, c+-1) with c clamped, and (p, c);
+                // the faces p = 0 and nx, whose a is 0, contribute nothing
+                auto C = [&](int e2, int k) { return t.dxu[k] * s_au[e2]; };
+                const T ix2 = t.idxu2[ui], iy2 = t.idyu2[ui];
+                T w = -T(2) * ix2 - T(2) * iy2, c = T(0);
+                if (i >= 1) c += C(ea - AC, ui - ny) * t.idxu2[ui - ny];
+                if (i + 1 <= nx) c += C(ea + AC, ui + ny) * t.idxu2[ui + ny];
+                if (j >= 1) c += C(ea - 1, ui - 1) * t.idyu2[ui - 1];
+                else w += iy2;
+                if (j + 1 <= ny - 1) c += C(ea + 1, ui + 1) * t.idyu2[ui + 1];
+                else w += iy2;
+                c += C(ea, ui) * w;
+                s += t.visc * t.idxu[ui] * c;
+            }
+            s += S[6][(ti + 2) * TJ + tj];
+            adu[ui] += s;
         }
     }
-    // ---------------- thickness diffusion coefficient at h (i, j)
-    if (i < nx && j < ny) {
-        const long long hi = (long long)i * ny + j;
-        S.hd[ob * t.sh + hi] = t.diff > T(0) ? hb[hi] * mh(hi) * t.diff * t.area[hi] : T(0);
+    __syncthreads();
+
+    // ---- pass D: thickness fluxes of the v faces (i0 + r, j0 - 2 + c)
+    for (int e = tid; e < TI * CA; e += ADJ_NT) {
+        const int r = e / CA, c = e % CA, i = i0 + r, j = j0 - 2 + c;
+        T hs[6], f = T(0);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) hs[k] = T(0);
+        if (i < nx && j >= 1 && j <= ny - 1) {
+            T aF = T(0);
+            if (j - 1 >= 1) aF -= s_hm[(r + 3) * HC + c];
+            if (j <= ny - 2) aF += s_hm[(r + 3) * HC + c + 1];
+            const int vi = i * n1 + j, fl = t.fv[vi];
+            const T iv2 = t.idyv2[vi];
+            const T Vf = v[vi] * iv2;
+            T q[6], gv;
+            ring6(q, R1<T>{ht}, i * ny + j - 1, 1, j - 3, ny - 1);
+            if (aF != T(0)) {
+                weno_flux_adj<T>(q, Vf, (fl >> 1) & 7, j >= 2 && j <= ny - 2, j >= 3 && j <= ny - 3, aF, hs, gv);
+                f = aF * gv * iv2;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) S[k][e] = hs[k];
+        S[6][e] = f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+        const int e = q * ADJ_NT + tid, ti = e / TJ, tj = e % TJ, i = i0 + ti, j = j0 + tj;
+        // h point (i, j): v face (i, j+3-k) reaches it with term k
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a_h[q] += S[k][ti * CA + tj + 5 - k];
+        if (i < nx && j < ny) adht[i * ny + j] = a_h[q];
+        if (i < nx && j <= ny) {
+            const int vi = i * n1 + j, ea = (ti + 1) * AC + tj + 1;
+            T s = a_v[q];
+            if (l == nl - 1) s += -t.drag * s_av[ea];
+            if (t.visc > T(0)) {
+                // viscosity stencil of v face (p, c): (p+-1, c) with p clamped, (p, c+-1), and (p, c)
+                auto C = [&](int e2, int k) { return t.dyv[k] * s_av[e2]; };
+                const T ix2 = t.idxv2[vi], iy2 = t.idyv2[vi];
+                T w = -T(2) * ix2 - T(2) * iy2, c = T(0);
+                if (i >= 1) c += C(ea - AC, vi - n1) * t.idxv2[vi - n1];
+                else w += ix2;
+                if (i + 1 <= nx - 1) c += C(ea + AC, vi + n1) * t.idxv2[vi + n1];
+                else w += ix2;
+                if (j >= 1) c += C(ea - 1, vi - 1) * t.idyv2[vi - 1];
+                if (j + 1 <= ny) c += C(ea + 1, vi + 1) * t.idyv2[vi + 1];
+                c += C(ea, vi) * w;
+                s += t.visc * t.idyv[vi] * c;
+            }
+            s += S[6][ti * CA + tj + 2];
+            adv[vi] += s;
+        }
     }
 }
 
-// Pass 2: every target of the tendency adjoint sums the stored terms of its
-// sources. adom, adkp, adht are written (every index once); adu, adv, adh
-// are added to.
-template <typename T>
-__global__ void k_sw_tend_adj_gather(Tab<T> t, SwSrc<T> S, T* adom, T* adkp, T* adht, T* adu, T* adv, T* adh)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    const int bl = blockIdx.z;
-    const int nx = t.nx, ny = t.ny, nl = t.nl, l = bl % nl;
-    if (i > nx || j > ny) return;
-    const long long ob = bl;
-    // stored terms of u face (p, c) / v face (p, c); 0 outside the grid
-    auto U = [&](const T* A, int p, int c) {
-        return (p >= 0 && p <= nx && c >= 0 && c < ny) ? A[ob * t.su + (long long)p * ny + c] : T(0);
-    };
-    auto V = [&](const T* A, int p, int c) {
-        return (p >= 0 && p < nx && c >= 0 && c <= ny) ? A[ob * t.sv + (long long)p * (ny + 1) + c] : T(0);
-    };
-    // ---- vorticity point (i, j): u face (i, j+2-k) and v face (i+2-k, j) reach it with term k
-    {
-        T s = T(0);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) s += U(S.uw + k * S.nu, i, j + 2 - k);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) s += V(S.vw + k * S.nv, i + 2 - k, j);
-        adom[ob * t.sw + (long long)i * (ny + 1) + j] = s;
-    }
-    // ---- h point (i, j)
-    if (i < nx && j < ny) {
-        const long long hi = (long long)i * ny + j;
-        // KE + pressure: u faces i (-a) and i+1 (+a), v faces j (-a) and j+1 (+a)
-        adkp[ob * t.sh + hi] = (-U(S.ua, i, j) + U(S.ua, i + 1, j)) + (-V(S.va, i, j) + V(S.va, i, j + 1));
-        // thickness fluxes: u face (i+3-k, j) and v face (i, j+3-k) reach it with term k
-        T sh_ = T(0);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) sh_ += U(S.uh + k * S.nu, i + 3 - k, j);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) sh_ += V(S.vh + k * S.nv, i, j + 3 - k);
-        adht[ob * t.sh + hi] = sh_;
-        if (t.diff > T(0)) {
-            // the diffusion stencil of cell (p, c): (p+-1, c), (p, c+-1) clamped to the grid, and (p, c)
-            const T* D = S.hd + ob * t.sh;
-            const T ia = t.iarea[hi];
-            T s = T(0);
-            if (i >= 1) s += D[hi - ny] * t.idx2h[hi - ny] * ia;
-            if (i + 1 <= nx - 1) s += D[hi + ny] * t.idx2h[hi + ny] * ia;
-            if (j >= 1) s += D[hi - 1] * t.idy2h[hi - 1] * ia;
-            if (j + 1 <= ny - 1) s += D[hi + 1] * t.idy2h[hi + 1] * ia;
-            const T a0 = D[hi], ix2 = t.idx2h[hi], iy2 = t.idy2h[hi];
-            s += a0 * (-T(2) * ix2 - T(2) * iy2) * ia;
-            if (i == nx - 1) s += a0 * ix2 * ia;
-            if (i == 0) s += a0 * ix2 * ia;
-            if (j == ny - 1) s += a0 * iy2 * ia;
-            if (j == 0) s += a0 * iy2 * ia;
-            adh[ob * t.sh + hi] += s;
-        }
-    }
-    // ---- u face (i, j)
-    if (j < ny) {
-        const long long ui = (long long)i * ny + j;
-        const T iu2 = t.idxu2[ui];
-        // U-average of the v faces (i-1, j), (i-1, j+1), (i, j), (i, j+1)
-        T s = V(S.vum, i - 1, j) * iu2 + V(S.vum, i - 1, j + 1) * iu2 + V(S.vum, i, j) * iu2 +
-              V(S.vum, i, j + 1) * iu2;
-        const T a0 = U(S.ua, i, j);
-        if (l == nl - 1) s += -t.drag * a0;
-        if (t.visc > T(0)) {
-            // viscosity stencil of u face (p, c): (p+-1, c), (p, c+-1) with c clamped, and (p, c)
-            const T id = t.idxu[ui];
-            if (i >= 1) s += U(S.uc, i - 1, j) * t.idxu2[ui - ny] * id;
-            if (i + 1 <= nx) s += U(S.uc, i + 1, j) * t.idxu2[ui + ny] * id;
-            if (j >= 1) s += U(S.uc, i, j - 1) * t.idyu2[ui - 1] * id;
-            if (j + 1 <= ny - 1) s += U(S.uc, i, j + 1) * t.idyu2[ui + 1] * id;
-            const T c0 = U(S.uc, i, j), ix2 = t.idxu2[ui], iy2 = t.idyu2[ui];
-            s += c0 * (-T(2) * ix2 - T(2) * iy2) * id;
-            if (j == ny - 1) s += c0 * iy2 * id;
-            if (j == 0) s += c0 * iy2 * id;
-        }
-        s += U(S.uf, i, j);
-        adu[ob * t.su + ui] += s;
-    }
-    // ---- v face (i, j)
-    if (i < nx) {
-        const long long vi = (long long)i * (ny + 1) + j;
-        const T iv2 = t.idyv2[vi];
-        // V-average of the u faces (i, j-1), (i, j), (i+1, j-1), (i+1, j)
-        T s = U(S.uvm, i, j - 1) * iv2 + U(S.uvm, i, j) * iv2 + U(S.uvm, i + 1, j - 1) * iv2 +
-              U(S.uvm, i + 1, j) * iv2;
-        const T a0 = V(S.va, i, j);
-        if (l == nl - 1) s += -t.drag * a0;
-        if (t.visc > T(0)) {
-            // viscosity stencil of v face (p, c): (p+-1, c) with p clamped, (p, c+-1), and (p, c)
-            const T id = t.idyv[vi];
-            if (i >= 1) s += V(S.vc, i - 1, j) * t.idxv2[vi - (ny + 1)] * id;
-            if (i + 1 <= nx - 1) s += V(S.vc, i + 1, j) * t.idxv2[vi + (ny + 1)] * id;
-            if (j >= 1) s += V(S.vc, i, j - 1) * t.idyv2[vi - 1] * id;
-            if (j + 1 <= ny) s += V(S.vc, i, j + 1) * t.idyv2[vi + 1] * id;
-            const T c0 = V(S.vc, i, j), ix2 = t.idxv2[vi], iy2 = t.idyv2[vi];
-            s += c0 * (-T(2) * ix2 - T(2) * iy2) * id;
-            if (i == nx - 1) s += c0 * ix2 * id;
-            if (i == 0) s += c0 * ix2 * id;
-        }
-        s += V(S.vf, i, j);
-        adv[ob * t.sv + vi] += s;
-    }
-}
-
-// Adjoint of k_sw_diag (gather): adds into adu, adv, adh.
+// Adjoint of k_sw_diag (gather, one thread a point and layer): adds into ad, and
+// where n.stage >= 0 goes on with the reverse of that stage's combination, whose
+// input is this kernel's result at the point (a pass over ad, and its launch, less).
+// 3 x 1024 x 768 float32: 62 + 30 us as two kernels, here 51 us (a load latency a quantity).
 template <typename T>
 __global__ void k_sw_diag_adj(Tab<T> t, const T* u, const T* v, const T* h, const T* adom, const T* adkp,
-                              const T* adht, T* adu, T* adv, T* adh)
+                              const T* adht, Fields<T> ad, UpdAdj<T> n)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    const int b = blockIdx.z;
-    const int nx = t.nx, ny = t.ny, nl = t.nl;
+    const int nx = t.nx, ny = t.ny, nl = t.nl, n1 = ny + 1;
     if (i > nx || j > ny) return;
-    auto mh = [&](int p, int c) { return (t.fh[(long long)p * ny + c] & 1) ? T(1) : T(0); };
-    for (int l = 0; l < nl; ++l) {
-        const long long ob = (long long)(b * nl + l);
-        const T* AO = adom + ob * t.sw;
-        const T* AK = adkp + ob * t.sh;
-        if (j < ny) {   // u point: dy(u) at w (i, j) (+) and (i, j+1) (-); KE of cells i-1, i
-            const long long ui = (long long)i * ny + j, o = ob * t.su + ui;
-            T a = -t.wb[(long long)i * (ny + 1) + j] * AO[(long long)i * (ny + 1) + j] +
-                  t.wb[(long long)i * (ny + 1) + j + 1] * AO[(long long)i * (ny + 1) + j + 1];
-            T kk = T(0);
-            if (i >= 1) kk += mh(i - 1, j) * AK[(long long)(i - 1) * ny + j];
-            if (i < nx) kk += mh(i, j) * AK[(long long)i * ny + j];
-            a += T(0.5) * kk * u[o] * t.idxu2[ui];
-            adu[o] += a;
-        }
-        if (i < nx) {   // v point: dx(v) at w (i, j) (+) and (i+1, j) (-); KE of cells j-1, j
-            const long long vi = (long long)i * (ny + 1) + j, o = ob * t.sv + vi;
-            T a = t.wa[(long long)i * (ny + 1) + j] * AO[(long long)i * (ny + 1) + j] -
-                  t.wa[(long long)(i + 1) * (ny + 1) + j] * AO[(long long)(i + 1) * (ny + 1) + j];
-            T kk = T(0);
-            if (j >= 1) kk += mh(i, j - 1) * AK[(long long)i * ny + j - 1];
-            if (j < ny) kk += mh(i, j) * AK[(long long)i * ny + j];
-            a += T(0.5) * kk * v[o] * t.idyv2[vi];
-            adv[o] += a;
-        }
+    const long long ob = blockIdx.z;
+    const int l = (int)(blockIdx.z % (unsigned)nl);
+    const T* AO = adom + ob * t.sw;
+    const T* AK = adkp + ob * t.sh;
+    const int ui = i * ny + j, wi = i * n1 + j;
+    auto mh = [&](int k) { return (t.fh[k] & 1) ? T(1) : T(0); };
+    const bool next = n.stage >= 0;
+    if (j < ny) {   // u point: dy(u) at w (i, j) (+) and (i, j+1) (-); KE of cells i-1, i
+        const long long o = ob * t.su + ui;
+        T a = -t.wb[wi] * AO[wi] + t.wb[wi + 1] * AO[wi + 1];
+        T kk = T(0);
+        if (i >= 1) kk += mh(ui - ny) * AK[ui - ny];
+        if (i < nx) kk += mh(ui) * AK[ui];
+        a += T(0.5) * kk * u[o] * t.idxu2[ui];
+        a += ad.u[o];
+        if (next) upd_adj_point<T>(t, n.stage, n.fresh, a, o, t.gu, ui, ad.u, true, n.ak.u, n.a0.u, n.a1.u, n.ab.u);
+        else ad.u[o] = a;
+    }
+    if (i < nx) {   // v point: dx(v) at w (i, j) (+) and (i+1, j) (-); KE of cells j-1, j
+        const long long o = ob * t.sv + wi;
+        T a = t.wa[wi] * AO[wi] - t.wa[wi + n1] * AO[wi + n1];
+        T kk = T(0);
+        if (j >= 1) kk += mh(ui - 1) * AK[ui - 1];
+        if (j < ny) kk += mh(ui) * AK[ui];
+        a += T(0.5) * kk * v[o] * t.idyv2[wi];
+        a += ad.v[o];
+        if (next) upd_adj_point<T>(t, n.stage, n.fresh, a, o, t.gv, wi, ad.v, true, n.ak.v, n.a0.v, n.a1.v, n.ab.v);
+        else ad.v[o] = a;
     }
     if (i < nx && j < ny) {
-        const long long hi = (long long)i * ny + j;
-        const T ar = t.area[hi];
-        // pressure: p_l = sum_m h_m/area * G[min(l, m)]
-        T ap[MAXL];
-        for (int l = 0; l < nl; ++l) ap[l] = adkp[(long long)(b * nl + l) * t.sh + hi];
-        for (int m = 0; m < nl; ++m) {
-            const long long o = (long long)(b * nl + m) * t.sh + hi;
-            T a = T(0);
-            for (int l = 0; l < nl; ++l) a += ap[l] * t.G[l < m ? l : m];
-            a = a * t.iarea[hi];
-            T aref = adht[o];   // d h_tot / d h_ref (linear: h_tot = h_ref)
-            if (!t.linear) {
-                const T z = (t.href[(long long)m * t.sh + hi] + h[o] - t.hmin * ar) * t.sharp;
-                aref = adht[o] * sigmoid_v(z);
-                a += aref;
-            }
-            adh[o] += a;
-            if (t.ad_href) aadd(&t.ad_href[(long long)m * t.sh + hi], aref);
+        // pressure: p_k = sum_m h_m/area * G[min(k, m)]
+        const long long o = ob * t.sh + ui;
+        const T* ap = adkp + (ob - l) * t.sh + ui;
+        T a = T(0);
+        for (int k = 0; k < nl; ++k) a += ap[k * t.sh] * t.G[k < l ? k : l];
+        a = a * t.iarea[ui];
+        T aref = adht[o];   // d h_tot / d h_ref (linear: h_tot = h_ref)
+        if (!t.linear) {
+            const T z = (t.href[(long long)l * t.sh + ui] + h[o] - t.hmin * t.area[ui]) * t.sharp;
+            aref = aref * sigmoid_v(z);
+            a += aref;
         }
+        if (t.ad_href) aadd(&t.ad_href[(long long)l * t.sh + ui], aref);
+        a += ad.h[o];
+        if (next) upd_adj_point<T>(t, n.stage, n.fresh, a, o, t.gh, ui, ad.h, true, n.ak.h, n.a0.h, n.a1.h, n.ab.h);
+        else ad.h[o] = a;
     }
 }
 
@@ -1655,13 +1723,6 @@ __global__ void k_axpy(long long n, T a, const T* x, T* y)
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) y[k] += a * x[k];
 }
-template <typename T>
-__global__ void k_copy(long long n, const T* x, T* y)
-{
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) y[k] = x[k];
-}
-
 }  // namespace sw
 }  // namespace vd
 
@@ -2305,43 +2366,12 @@ static Sizes sizes(const vd_sw_plan* p)
 }
 
 template <typename T>
-struct Fields {
-    T *u, *v, *h;
-};
-
-template <typename T>
 static bool take_uvh(Arena& ws, const Sizes& s, int B, Fields<T>& f)
 {
     f.u = (T*)ws.take(sizeof(T) * s.su * B);
     f.v = (T*)ws.take(sizeof(T) * s.sv * B);
     f.h = (T*)ws.take(sizeof(T) * s.sh * B);
     return f.u && f.v && f.h;
-}
-
-// Per-source buffers of the two-pass tendency adjoint (16 values per u and v
-// face, one per h point, every field of the batch).
-template <typename T>
-static bool take_src(Arena& ws, const Sizes& s, int B, SwSrc<T>& S)
-{
-    const long long nu = s.su * B, nv = s.sv * B, nh = s.sh * B;
-    T* b = (T*)ws.take(sizeof(T) * (size_t)(16 * nu + 16 * nv + nh));
-    if (!b) return false;
-    S.nu = nu;
-    S.nv = nv;
-    S.ua = b; b += nu;
-    S.uvm = b; b += nu;
-    S.uc = b; b += nu;
-    S.uf = b; b += nu;
-    S.uw = b; b += 6 * nu;
-    S.uh = b; b += 6 * nu;
-    S.va = b; b += nv;
-    S.vum = b; b += nv;
-    S.vc = b; b += nv;
-    S.vf = b; b += nv;
-    S.vw = b; b += 6 * nv;
-    S.vh = b; b += 6 * nv;
-    S.hd = b;
-    return true;
 }
 
 struct Launch {
@@ -2353,6 +2383,23 @@ static Launch lgrid(const vd_sw_plan* p, int z)
     L.block = dim3(32, 8, 1);
     L.grid = dim3((unsigned)((p->ny + 1 + 31) / 32), (unsigned)((p->nx + 1 + 7) / 8), (unsigned)z);
     return L;
+}
+
+// blocks and attributes of k_sw_tend_adj
+template <typename T>
+static cudaError_t adj_attr()
+{
+    static vd::PerDeviceOnce once;
+    return once.run([] {
+        return cudaFuncSetAttribute(k_sw_tend_adj<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(sizeof(T) * adj_smem<T>));
+    });
+}
+template <typename T>
+static dim3 agrid(const vd_sw_plan* p, int z)
+{
+    return dim3((unsigned)((p->ny + 1 + ADJ_TJ - 1) / ADJ_TJ), (unsigned)((p->nx + 1 + adj_ti<T> - 1) / adj_ti<T>),
+                (unsigned)z);
 }
 
 // One RK3-SSP run of nstep steps in model space, forward (S = T) or
@@ -2480,7 +2527,8 @@ static int tend_tgl(vd_sw_plan* p, int B, Fields<T> cur, Fields<T> dcur, Work<T>
     return VD_OK;
 }
 
-// forward step loop
+// Forward step loop. With traj, the steps run from traj[n] to traj[n + 1] (x is
+// not touched); else x is advanced in place.
 template <typename T>
 static int run_fwd(vd_sw_plan* p, int B, Fields<T> x, int nstep, Fields<T> xb, Fields<T> F, int hasF, const T* taux,
                    const T* tauy, Work<T>& wk, Fields<T>* traj, cudaStream_t st)
@@ -2490,19 +2538,12 @@ static int run_fwd(vd_sw_plan* p, int B, Fields<T> x, int nstep, Fields<T> xb, F
     const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl);
     const int mc = p->d.forcing_momentum == 1;
     for (int n = 0; n < nstep; ++n) {
-        if (traj) {
-            k_copy<T><<<(unsigned)((s.su * B + 255) / 256), 256, 0, st>>>(s.su * B, x.u, traj[n].u);
-            VD_LAUNCH_CHECK();
-            k_copy<T><<<(unsigned)((s.sv * B + 255) / 256), 256, 0, st>>>(s.sv * B, x.v, traj[n].v);
-            VD_LAUNCH_CHECK();
-            k_copy<T><<<(unsigned)((s.sh * B + 255) / 256), 256, 0, st>>>(s.sh * B, x.h, traj[n].h);
-            VD_LAUNCH_CHECK();
-        }
-        Fields<T> cur = x;
+        const Fields<T> from = traj ? traj[n] : x, to = traj ? traj[n + 1] : x;
+        Fields<T> cur = from;
         for (int stg = 0; stg < 3; ++stg) {
             const int rc = tend_fwd<T>(p, B, cur, wk, taux, tauy, st);
             if (rc) return rc;
-            Fields<T> nxt = stg == 0 ? wk.x1 : (stg == 1 ? wk.x2 : (mc ? wk.x1 : x));
+            Fields<T> nxt = stg == 0 ? wk.x1 : (stg == 1 ? wk.x2 : (mc ? wk.x1 : to));
             StageArgs sa{stg, (stg == 2 && hasF && !mc) ? 1 : 0};
             Fields<T> ks = stg == 0 ? wk.k0 : wk.k1;
             k_sw_update<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, sa, rt(cur), r<T>(wk.tuvh.u), r<T>(wk.tuvh.v),
@@ -2512,7 +2553,7 @@ static int run_fwd(vd_sw_plan* p, int B, Fields<T> x, int nstep, Fields<T> xb, F
             cur = nxt;
         }
         if (mc) {
-            k_sw_force_mc<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(wk.x1), rt(F), wt(x));
+            k_sw_force_mc<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(wk.x1), rt(F), wt(to));
             VD_LAUNCH_CHECK();
         }
     }
@@ -2627,10 +2668,10 @@ extern "C" size_t vd_sw_workspace_bytes(const vd_sw_plan* p, int batch, int nste
     const long long bfn = bf_elems(p);
     const size_t wk = (esz == 8 ? work_bytes<double>(s, batch, bfn) : work_bytes<float>(s, batch, bfn));
     // inputs (x, xb, F), their tangents / adjoints, two work sets, adjoint
-    // accumulators, the per-source buffers of the tendency adjoint, and the
-    // per-step trajectory
+    // accumulators, the vorticity and thickness of a step's first two stages,
+    // and the per-step trajectory
     return 14 * F3 + 2 * wk + (size_t)nstep * F3 + esz * (s.sw + 2 * s.sh) * batch +
-           esz * (16 * s.su + 16 * s.sv + s.sh) * batch + 64 * 256;
+           2 * esz * (s.sw + s.sh) * batch + 64 * 256;
 }
 
 namespace {
@@ -2684,15 +2725,20 @@ static int sw_tgl_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
     return scale<T>(p, B, 1, din.x.u, din.x.v, din.x.h, (T*)du1, (T*)dv1, (T*)dh1, st);
 }
 
-// adjoint of one right-hand side at state x (model space): adk -> adx (+=)
+// adjoint of one right-hand side at state x (model space): adk -> adx (+=).
+// wk.om and wk.ht hold the state's vorticity and thickness (and wk.kp its KE +
+// pressure) where have_diag, else they are formed here. next: the reverse of the
+// stage combination that follows, or stage -1 for none.
 template <typename T>
-static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> adx, Work<T>& wk, T* adom, T* adkp,
-                   T* adht, const SwSrc<T>& src, const T* taux, const T* tauy, cudaStream_t st)
+static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> adx, const Work<T>& wk, bool have_diag,
+                   T* adom, T* adkp, T* adht, const UpdAdj<T>& next, const T* taux, const T* tauy, cudaStream_t st)
 {
     Tab<T>& t = tab<T>(p);
     const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl);
-    k_sw_diag<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(x), w(wk.om), w(wk.kp), w(wk.ht));
-    VD_LAUNCH_CHECK();
+    if (!have_diag) {
+        k_sw_diag<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(x), w(wk.om), w(wk.kp), w(wk.ht));
+        VD_LAUNCH_CHECK();
+    }
     Fields<T> ak = adk;
     if (p->bf) {
         // the filter's transpose first: it needs the pre-filter tendencies of
@@ -2712,12 +2758,11 @@ static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> a
         ak.u = wk.bau;
         ak.v = wk.bav;
     }
-    k_sw_tend_adj_src<T><<<Ll.grid, Ll.block, 0, st>>>(t, x.u, x.v, x.h, wk.om, wk.ht, ak.u, ak.v, ak.h, src,
-                                                        taux, tauy);
+    VD_CUDA_TRY(adj_attr<T>());
+    k_sw_tend_adj<T><<<agrid<T>(p, B * p->nl), ADJ_NT, sizeof(T) * adj_smem<T>, st>>>(t, x.u, x.v, wk.om, wk.ht, ak.u, ak.v, ak.h, adom,
+                                                                adkp, adht, adx.u, adx.v, adx.h, taux, tauy);
     VD_LAUNCH_CHECK();
-    k_sw_tend_adj_gather<T><<<Ll.grid, Ll.block, 0, st>>>(t, src, adom, adkp, adht, adx.u, adx.v, adx.h);
-    VD_LAUNCH_CHECK();
-    k_sw_diag_adj<T><<<Ld.grid, Ld.block, 0, st>>>(t, x.u, x.v, x.h, adom, adkp, adht, adx.u, adx.v, adx.h);
+    k_sw_diag_adj<T><<<Ll.grid, Ll.block, 0, st>>>(t, x.u, x.v, x.h, adom, adkp, adht, adx, next);
     VD_LAUNCH_CHECK();
     return VD_OK;
 }
@@ -2736,7 +2781,7 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
     Work<T> wk;
     if ((rc = take_work<T>(ws, s, B, wk, bf_elems(p)))) return rc;
     std::vector<Fields<T>> traj((size_t)(nstep > 0 ? nstep : 1));
-    for (int n = 0; n < nstep; ++n)
+    for (int n = 1; n < nstep; ++n)
         if (!take_uvh(ws, s, B, traj[n])) return VD_ERR_WORKSPACE;
     Fields<T> ad, adk, a0, a1, adb, adF, x1, x2;
     if (!take_uvh(ws, s, B, ad) || !take_uvh(ws, s, B, adk) || !take_uvh(ws, s, B, a0) || !take_uvh(ws, s, B, a1) ||
@@ -2745,16 +2790,22 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
     T* adom = (T*)ws.take(sizeof(T) * s.sw * B);
     T* adkp = (T*)ws.take(sizeof(T) * s.sh * B);
     T* adht = (T*)ws.take(sizeof(T) * s.sh * B);
-    SwSrc<T> src;
-    if (!adom || !adkp || !adht || !take_src(ws, s, B, src)) return VD_ERR_WORKSPACE;
-    // forward sweep storing the state at the start of every step
-    Fields<T> xr;
-    if (!take_uvh(ws, s, B, xr)) return VD_ERR_WORKSPACE;
-    VD_CUDA_TRY(cudaMemcpyAsync(xr.u, in.x.u, sizeof(T) * s.su * B, cudaMemcpyDeviceToDevice, st));
-    VD_CUDA_TRY(cudaMemcpyAsync(xr.v, in.x.v, sizeof(T) * s.sv * B, cudaMemcpyDeviceToDevice, st));
-    VD_CUDA_TRY(cudaMemcpyAsync(xr.h, in.x.h, sizeof(T) * s.sh * B, cudaMemcpyDeviceToDevice, st));
-    rc = run_fwd<T>(p, B, xr, nstep, in.xb, in.F, in.hasF, (const T*)taux, (const T*)tauy, wk, traj.data(), st);
-    if (rc) return rc;
+    // vorticity and thickness of the first two stages (the third's stay in wk)
+    T* som[2];
+    T* sht[2];
+    for (int k = 0; k < 2; ++k) {
+        som[k] = (T*)ws.take(sizeof(T) * s.sw * B);
+        sht[k] = (T*)ws.take(sizeof(T) * s.sh * B);
+    }
+    if (!adom || !adkp || !adht || !som[0] || !sht[0] || !som[1] || !sht[1]) return VD_ERR_WORKSPACE;
+    // forward sweep keeping the state at the start of every step (the last
+    // step's own result is not part of the adjoint)
+    traj[0] = in.x;
+    if (nstep > 1) {
+        rc = run_fwd<T>(p, B, in.x, nstep - 1, in.xb, in.F, in.hasF, (const T*)taux, (const T*)tauy, wk, traj.data(),
+                        st);
+        if (rc) return rc;
+    }
     // adjoint of the physical output -> model space
     if ((rc = scale<T>(p, B, 1, (const T*)adu1, (const T*)adv1, (const T*)adh1, ad.u, ad.v, ad.h, st))) return rc;
     if ((rc = zero(adb, s, B, st)) || (rc = zero(adF, s, B, st))) return rc;
@@ -2766,9 +2817,11 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
         Fields<T> stages[3] = {traj[n], x1, x2};
         {
             Fields<T> cur = traj[n];
-            const Launch Ld = lgrid(p, B);
             for (int stg = 0; stg < 2; ++stg) {
-                if ((rc = tend_fwd<T>(p, B, cur, wk, (const T*)taux, (const T*)tauy, st))) return rc;
+                Work<T> ws2 = wk;
+                ws2.om = som[stg];
+                ws2.ht = sht[stg];
+                if ((rc = tend_fwd<T>(p, B, cur, ws2, (const T*)taux, (const T*)tauy, st))) return rc;
                 Fields<T> nxt = stg == 0 ? x1 : x2;
                 StageArgs sa{stg, 0};
                 Fields<T> ks = stg == 0 ? wk.k0 : wk.k1;
@@ -2800,18 +2853,27 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
             k_sw_force_mc_adj<T><<<Ll.grid, Ll.block, 0, st>>>(t, wk.x1.u, wk.x1.v, wk.x1.h, in.F.h, ad.u, ad.v);
             VD_LAUNCH_CHECK();
         }
-        if ((rc = zero(a0, s, B, st)) || (rc = zero(a1, s, B, st))) return rc;
+        // the stages in reverse; the reverse of a stage's combination rides on the
+        // diagnostics' adjoint of the stage after it
+        auto upd = [&](int stage) { return UpdAdj<T>{stage, stage == 2, adk, a0, a1, adb}; };
+        k_sw_update_adj<T><<<Ll.grid, Ll.block, 0, st>>>(t, upd(2), B * p->nl, ad);
+        VD_LAUNCH_CHECK();
         for (int stg = 2; stg >= 0; --stg) {
-            k_sw_update_adj<T><<<Ll.grid, Ll.block, 0, st>>>(t, stg, B * p->nl, ad.u, ad.v, ad.h, adk.u, adk.v, adk.h,
-                                                             a0.u, a0.v, a0.h, a1.u, a1.v, a1.h, adb.u, adb.v, adb.h);
-            VD_LAUNCH_CHECK();
-            if ((rc = rhs_adj<T>(p, B, stages[stg], adk, ad, wk, adom, adkp, adht, src, (const T*)taux,
+            Work<T> ws2 = wk;
+            // (the mass-consistent form has rebuilt stage 2's diagnostics in wk as well)
+            if (stg < 2) {
+                ws2.om = som[stg];
+                ws2.ht = sht[stg];
+            }
+            // the filter's transpose forms the pre-filter tendencies again and reads KE + pressure
+            const bool have = (stg < 2 || mc) && !p->bf;
+            if ((rc = rhs_adj<T>(p, B, stages[stg], adk, ad, ws2, have, adom, adkp, adht, upd(stg - 1), (const T*)taux,
                                  (const T*)tauy, st)))
                 return rc;
         }
     }
-    // boundary fields that default to the initial state feed its adjoint
-    if (!in.hasb) {
+    // boundary fields that default to the initial state feed its adjoint (through the sponge)
+    if (!in.hasb && t.has_sponge) {
         if ((rc = addto(ad, T(1), adb, s, B, st))) return rc;
     }
     if ((rc = scale<T>(p, B, 0, ad.u, ad.v, ad.h, (T*)adu0, (T*)adv0, (T*)adh0, st))) return rc;
@@ -2955,10 +3017,9 @@ static int sw_rhs_adj_t(vd_sw_plan* p, int B, const void* u, const void* v, cons
     T* adom = (T*)ws.take(sizeof(T) * s.sw * B);
     T* adkp = (T*)ws.take(sizeof(T) * s.sh * B);
     T* adht = (T*)ws.take(sizeof(T) * s.sh * B);
-    SwSrc<T> src;
-    if (!adom || !adkp || !adht || !take_src(ws, s, B, src)) return VD_ERR_WORKSPACE;
+    if (!adom || !adkp || !adht) return VD_ERR_WORKSPACE;
     Fields<T> x{(T*)u, (T*)v, (T*)h}, ak{(T*)aku, (T*)akv, (T*)akh}, ad{(T*)adu, (T*)adv, (T*)adh};
-    return rhs_adj<T>(p, B, x, ak, ad, wk, adom, adkp, adht, src, nullptr, nullptr, st);
+    return rhs_adj<T>(p, B, x, ak, ad, wk, false, adom, adkp, adht, UpdAdj<T>{-1}, nullptr, nullptr, st);
 }
 
 // elementwise stage combination: k = rhs + sponge; stage 0/1 store k
@@ -3050,9 +3111,9 @@ template <typename T>
 static int sw_stage_adj_t(vd_sw_plan* p, int B, int stage, void* const* f, cudaStream_t st)
 {
     const Launch L = lgrid(p, B * p->nl);
-    k_sw_update_adj<T><<<L.grid, L.block, 0, st>>>(tab<T>(p), stage, B * p->nl, (T*)f[0], (T*)f[1], (T*)f[2],
-                                                   (T*)f[3], (T*)f[4], (T*)f[5], (T*)f[6], (T*)f[7], (T*)f[8],
-                                                   (T*)f[9], (T*)f[10], (T*)f[11], (T*)f[12], (T*)f[13], (T*)f[14]);
+    const UpdAdj<T> n{stage, 0, F3<T>(f[3], f[4], f[5]), F3<T>(f[6], f[7], f[8]), F3<T>(f[9], f[10], f[11]),
+                      F3<T>(f[12], f[13], f[14])};
+    k_sw_update_adj<T><<<L.grid, L.block, 0, st>>>(tab<T>(p), n, B * p->nl, F3<T>(f[0], f[1], f[2]));
     VD_LAUNCH_CHECK();
     return VD_OK;
 }

@@ -104,15 +104,15 @@ struct vd_mg_plan {
     int lc = 0;                          // first level run by the one-block coarse kernel (nlev: none)
     void* dev = nullptr;
     struct DLev {
-        const void *mask = nullptr, *cu = nullptr, *cv = nullptr, *factor = nullptr, *divr = nullptr,
-                   *divp = nullptr;
+        const void *mask = nullptr, *cu = nullptr, *cv = nullptr, *factor = nullptr, *g = nullptr, *mr = nullptr,
+                   *mp = nullptr;
     };
     std::vector<DLev> dl;
     const void* lam = nullptr;           // [nsys]
     const int32_t* bot_idx = nullptr;    // [nb] flat bottom cell index
     const void* bot_inv = nullptr;       // [nsys][nb][nb]
     // the bottom level's 6 niter_bottom damped sweeps as one linear map,
-    // f = N rhs (+ M f on a one-level grid): [nsys][N, M][input k][output m]
+    // f = N rhs (+ M f on a one-level grid): [nsys][N, M][output m][input k]
     const void* bot_sm = nullptr;
     // the whole solve as one CUDA graph on plan-owned rhs / solution buffers
     // (captured at the first solve with a given workspace, replayed after)
@@ -120,21 +120,26 @@ struct vd_mg_plan {
     cudaStream_t gstream = nullptr;      // capture stream
     cudaGraphExec_t gexec = nullptr;
     const void* gws = nullptr;           // workspace the graph was captured with
-    std::vector<size_t> ws_off;          // per level: f, rhs, tmp offsets (elements)
+    std::vector<size_t> ws_off;          // per level: f, rhs, tmp, scaled rhs offsets (elements)
     size_t ws_elems = 0;
 };
 
 namespace vd {
 
 // One level on the device. The edge coefficients are stored pre-scaled by
-// 1/d0^2 and 1/d1^2 and the Jacobi factor pre-multiplied by omega: the sweep
-// is then 7 FP64 instructions a cell (10 in the reference's grouping), the
-// rate that bounds it on this part (same operator, rounding order differs).
+// 1/d0^2 and 1/d1^2 and the Jacobi factor pre-multiplied by omega. In float64,
+// whose instruction rate bounds the sweeps, they are also stored times the factor
+// (g), and the level's right-hand side once times the factor (rr = factor rhs): a
+// sweep is then 5 FP64 instructions a cell instead of 7, for as many arrays. In
+// float32, bound by memory and launches, the shared coefficients are the fewer bytes.
 template <typename T>
 struct MgLev {
     int n0, n1;
     const T *mask, *cu, *cv, *factor, *lam;   // cu = c_u/d0^2, cv = c_v/d1^2, factor = omega mask/den
+    const T* g;                               // float64: [nsys][4][n0][n1], towards i+1, i-1, j+1, j-1
+    const T *mr, *mp;                         // mask / divisor of the restriction here, the prolongation to here
 };
+template <typename T> constexpr bool mg_scaled = sizeof(T) == 8;
 
 template <typename T>
 __device__ __forceinline__ T fat(const T* f, int n0, int n1, int i, int j)
@@ -142,68 +147,108 @@ __device__ __forceinline__ T fat(const T* f, int n0, int n1, int i, int j)
     return (i < 0 || j < 0 || i >= n0 || j >= n1) ? T(0) : f[(long long)i * n1 + j];
 }
 
-// Per-point arithmetic, shared by the level-wide kernels and the one-block
-// coarse-level kernel so that both give the same bits.
+// Per-point arithmetic, shared by the level-wide kernels, the tile kernels and the
+// one-block coarse-level kernel so that all give the same bits.
 
-// one damped Jacobi update at (i, j) (helmholtz_multigrid.py:86-98)
+// what a sweep reads of the right-hand side, at cell o of system b
 template <typename T>
-__device__ __forceinline__ T mg_sweep_pt(const MgLev<T>& L, const T* F, T rhs, T factor, int i, int j, T omega)
+__device__ __forceinline__ T mg_scaled_rhs(const MgLev<T>& L, T rhs, int b, long long o)
 {
-    const long long o = (long long)i * L.n1 + j;
-    const T cup = L.cu[(long long)(i + 1) * L.n1 + j], cui = L.cu[o];
-    const T cvp = L.cv[(long long)i * (L.n1 + 1) + j + 1], cvi = L.cv[(long long)i * (L.n1 + 1) + j];
-    const T s = cup * fat(F, L.n0, L.n1, i + 1, j) + cui * fat(F, L.n0, L.n1, i - 1, j) +
-                cvp * fat(F, L.n0, L.n1, i, j + 1) + cvi * fat(F, L.n0, L.n1, i, j - 1);
-    return factor * (s - rhs) + (T(1) - omega) * F[o];
+    if constexpr (mg_scaled<T>) return __ldg(L.factor + (long long)b * L.n0 * L.n1 + o) * rhs;
+    else return rhs;
+}
+
+// the first sweep from f = 0
+template <typename T>
+__device__ __forceinline__ T mg_first(const MgLev<T>& L, T rr, int b, long long o)
+{
+    if constexpr (mg_scaled<T>) return -rr;
+    else return __ldg(L.factor + (long long)b * L.n0 * L.n1 + o) * (T(0) - rr);
+}
+
+// one damped Jacobi update of cell (i, j) from its neighbours (helmholtz_multigrid.py:86-98)
+template <typename T>
+__device__ __forceinline__ T mg_update(const MgLev<T>& L, T fc, T fe, T fw, T fn, T fs, T rr, int b, int i, int j,
+                                       T omega)
+{
+    const long long n = (long long)L.n0 * L.n1, o = (long long)i * L.n1 + j;
+    if constexpr (mg_scaled<T>) {
+        const T* g = L.g + 4 * b * n + o;
+        const T s = (T(1) - omega) * fc - rr;
+        return __ldg(g) * fe + (__ldg(g + n) * fw + (__ldg(g + 2 * n) * fn + (__ldg(g + 3 * n) * fs + s)));
+    } else {
+        const T cup = L.cu[o + L.n1], cui = L.cu[o];
+        const T cvp = L.cv[o + i + 1], cvi = L.cv[o + i];
+        const T s = cup * fe + cui * fw + cvp * fn + cvi * fs;
+        return __ldg(L.factor + b * n + o) * (s - rr) + (T(1) - omega) * fc;
+    }
+}
+template <typename T>
+__device__ __forceinline__ T mg_sweep_pt(const MgLev<T>& L, const T* F, T rr, int b, int i, int j, T omega)
+{
+    return mg_update(L, F[(long long)i * L.n1 + j], fat(F, L.n0, L.n1, i + 1, j), fat(F, L.n0, L.n1, i - 1, j),
+                     fat(F, L.n0, L.n1, i, j + 1), fat(F, L.n0, L.n1, i, j - 1), rr, b, i, j, omega);
 }
 
 // rhs - mask (div(c grad f) - lambda f) at (i, j)  (helmholtz_multigrid.py:102-114)
 template <typename T>
-__device__ __forceinline__ T mg_residual_pt(const MgLev<T>& L, const T* F, T rhs, T lam, int i, int j)
+__device__ __forceinline__ T mg_resid(const MgLev<T>& L, T fc, T fe, T fw, T fn, T fs, T rhs, T lam, int i, int j)
 {
     const long long o = (long long)i * L.n1 + j;
-    const T fc = F[o];
-    const T cup = L.cu[(long long)(i + 1) * L.n1 + j], cui = L.cu[o];
-    const T cvp = L.cv[(long long)i * (L.n1 + 1) + j + 1], cvi = L.cv[(long long)i * (L.n1 + 1) + j];
-    const T hx = cup * (fat(F, L.n0, L.n1, i + 1, j) - fc) - cui * (fc - fat(F, L.n0, L.n1, i - 1, j));
-    const T hy = cvp * (fat(F, L.n0, L.n1, i, j + 1) - fc) - cvi * (fc - fat(F, L.n0, L.n1, i, j - 1));
-    const T Hf = (hx + hy - lam * fc) * L.mask[o];
-    return rhs - Hf;
+    const T cup = L.cu[o + L.n1], cui = L.cu[o];
+    const T cvp = L.cv[o + i + 1], cvi = L.cv[o + i];
+    // (one chain of FMAs: 10 FP64 instructions)
+    T h = cup * (fe - fc);
+    h = h - cui * (fc - fw);
+    h = h + cvp * (fn - fc);
+    h = h - cvi * (fc - fs);
+    h = h - lam * fc;
+    return rhs - h * L.mask[o];
+}
+template <typename T>
+__device__ __forceinline__ T mg_residual_pt(const MgLev<T>& L, const T* F, T rhs, T lam, int i, int j)
+{
+    return mg_resid(L, F[(long long)i * L.n1 + j], fat(F, L.n0, L.n1, i + 1, j), fat(F, L.n0, L.n1, i - 1, j),
+                    fat(F, L.n0, L.n1, i, j + 1), fat(F, L.n0, L.n1, i, j - 1), rhs, lam, i, j);
 }
 
-// (sum of the 2x2 fine cells) / div * mask_coarse at coarse (I, J)  (147-151)
+// (sum of the 2x2 fine cells) * (mask / div) at coarse (I, J)  (147-151)
 template <typename T>
-__device__ __forceinline__ T mg_restrict_pt(const T* fine, int n1c, int I, int J, const T* divr, const T* maskc)
+__device__ __forceinline__ T mg_restrict_pt(const T* fine, int n1c, int I, int J, const T* mr)
 {
     const int n1f = 2 * n1c;
     const T* F = fine + (long long)(2 * I) * n1f + 2 * J;
-    const long long o = (long long)I * n1c + J;
-    const T s = F[0] + F[n1f] + F[1] + F[n1f + 1];
-    return s / divr[o] * maskc[o];
+    return (F[0] + F[n1f] + F[1] + F[n1f + 1]) * mr[(long long)I * n1c + J];
 }
 
-// prolong(coarse) / div * mask_fine at fine (i, j)  (117-144)
+// f + prolong(coarse) * (mask / div) at a fine cell: 9-3-3-1 weights as two
+// interpolations of 3-1, along i then j  (117-144). c: its coarse cell, then the
+// coarse neighbours it leans on along i, along j and across
 template <typename T>
-__device__ __forceinline__ T mg_prolong_pt(const T* V, int n0c, int n1c, int i_f, int jf, const T* divp,
-                                           const T* maskf)
+__device__ __forceinline__ T mg_prolong4(T c, T ci, T cj, T cij, T mp, T f)
+{
+    return f + (T(3) * (T(3) * c + ci) + (T(3) * cj + cij)) * mp;
+}
+template <typename T>
+__device__ __forceinline__ T mg_prolong_pt(const T* V, int n0c, int n1c, int i_f, int jf, T mp, T f)
 {
     const int I = i_f >> 1, J = jf >> 1;
     const int di = (i_f & 1) ? 1 : -1, dj = (jf & 1) ? 1 : -1;
-    const T q = T(9) * fat(V, n0c, n1c, I, J) + T(3) * (fat(V, n0c, n1c, I, J + dj) + fat(V, n0c, n1c, I + di, J)) +
-                fat(V, n0c, n1c, I + di, J + dj);
-    const long long o = (long long)i_f * (2 * n1c) + jf;
-    return q / divp[o] * maskf[o];
+    return mg_prolong4(fat(V, n0c, n1c, I, J), fat(V, n0c, n1c, I + di, J), fat(V, n0c, n1c, I, J + dj),
+                       fat(V, n0c, n1c, I + di, J + dj), mp, f);
 }
 
+// One sweep of a level. FP64-issue bound in float64 at the large levels (1024 x 768:
+// 9.8 us, 7.9 at the pipe's rate; with 7 instructions a cell 13.0 us).
 template <typename T>
-__global__ void k_mg_sweep(MgLev<T> L, const T* __restrict__ f, const T* __restrict__ rhs, T* __restrict__ out,
+__global__ void k_mg_sweep(MgLev<T> L, const T* __restrict__ f, const T* __restrict__ rr, T* __restrict__ out,
                            T omega)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y, b = blockIdx.z;
     if (j >= L.n1) return;
     const long long fs = (long long)L.n0 * L.n1, o = (long long)i * L.n1 + j;
-    out[b * fs + o] = mg_sweep_pt(L, f + b * fs, rhs[b * fs + o], L.factor[b * fs + o], i, j, omega);
+    out[b * fs + o] = mg_sweep_pt(L, f + b * fs, rr[b * fs + o], b, i, j, omega);
 }
 
 template <typename T>
@@ -216,29 +261,187 @@ __global__ void k_mg_residual(MgLev<T> L, const T* __restrict__ f, const T* __re
     res[b * fs + o] = mg_residual_pt(L, f + b * fs, rhs[b * fs + o], L.lam[b], i, j);
 }
 
+// rr of a level (float64, the finest level's once a solve)
 template <typename T>
-__global__ void k_mg_restrict(int n0c, int n1c, const T* __restrict__ fine, const T* __restrict__ divr,
-                              const T* __restrict__ maskc, T* __restrict__ coarse)
+__global__ void k_mg_scale(MgLev<T> L, const T* __restrict__ rhs, T* __restrict__ rr)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.y, b = blockIdx.z;
+    if (j >= L.n1) return;
+    const long long fs = (long long)L.n0 * L.n1, o = (long long)i * L.n1 + j;
+    rr[b * fs + o] = mg_scaled_rhs(L, rhs[b * fs + o], b, o);
+}
+
+// What a level keeps of its right-hand side v at cell o: rhs, rr (float64) and,
+// where first is given, the result of the first sweep from f = 0.
+template <typename T>
+struct MgDown {
+    T *rhs, *rr, *first;
+};
+template <typename T>
+__device__ __forceinline__ void mg_put_rhs(const MgLev<T>& C, const MgDown<T>& d, T v, int b, long long o)
+{
+    const long long go = (long long)b * C.n0 * C.n1 + o;
+    d.rhs[go] = v;
+    const T rr = mg_scaled_rhs(C, v, b, o);
+    if constexpr (mg_scaled<T>) d.rr[go] = rr;
+    if (d.first) d.first[go] = mg_first(C, rr, b, o);
+}
+
+template <typename T>
+__global__ void k_mg_restrict(MgLev<T> C, const T* __restrict__ fine, MgDown<T> d)
+{
+    const int J = blockIdx.x * blockDim.x + threadIdx.x;
+    const int I = blockIdx.y, b = blockIdx.z;
+    if (J >= C.n1) return;
+    const long long fsc = (long long)C.n0 * C.n1;
+    mg_put_rhs(C, d, mg_restrict_pt(fine + b * 4 * fsc, C.n1, I, J, C.mr), b, (long long)I * C.n1 + J);
+}
+
+// Residual of level L restricted to level C, one thread a coarse cell (its four
+// residuals never leave registers). 1024 x 768 float64: 19.7 us (17 + 10 as two kernels
+// with a division), 16 at the FP64 rate.
+template <typename T>
+__global__ void k_mg_resid_restrict(MgLev<T> L, MgLev<T> C, const T* __restrict__ f, const T* __restrict__ rhs,
+                                    MgDown<T> d)
+{
+    const int J = blockIdx.x * blockDim.x + threadIdx.x;
+    const int I = blockIdx.y, b = blockIdx.z;
+    if (J >= C.n1) return;
+    const long long fs = (long long)L.n0 * L.n1;
+    f += b * fs;
+    rhs += b * fs;
+    T r[2][2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const int i = 2 * I + u, j = 2 * J + v;
+            r[u][v] = mg_residual_pt(L, f, rhs[(long long)i * L.n1 + j], L.lam[b], i, j);
+        }
+    const long long o = (long long)I * C.n1 + J;
+    mg_put_rhs(C, d, (r[0][0] + r[1][0] + r[0][1] + r[1][1]) * C.mr[o], b, o);
+}
+
+// Prolongation to level L of the coarse field V, one thread a coarse cell: its four
+// fine cells share their 3-1 interpolations along i (3.5 FP64 instructions a fine cell,
+// a division and 7 more when each fine cell was formed alone: 30 us at 1024 x 768, here
+// 8.4).
+template <typename T>
+__global__ void k_mg_prolong(MgLev<T> L, int n0c, int n1c, const T* __restrict__ V, T* __restrict__ fine, int add)
 {
     const int J = blockIdx.x * blockDim.x + threadIdx.x;
     const int I = blockIdx.y, b = blockIdx.z;
     if (J >= n1c) return;
-    const long long fsc = (long long)n0c * n1c;
-    coarse[b * fsc + (long long)I * n1c + J] = mg_restrict_pt(fine + b * 4 * fsc, n1c, I, J, divr, maskc);
+    V += b * (long long)n0c * n1c;
+    fine += b * (long long)L.n0 * L.n1;
+    T c[3][3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+#pragma unroll
+        for (int v = 0; v < 3; ++v) c[u][v] = fat(V, n0c, n1c, I + u - 1, J + v - 1);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const long long o = (long long)(2 * I + u) * L.n1 + 2 * J + v;
+            fine[o] = mg_prolong4(c[1][1], c[2 * u][1], c[1][2 * v], c[2 * u][2 * v], L.mp[o],
+                                  add ? fine[o] : T(0));
+        }
 }
 
-template <typename T>
-__global__ void k_mg_prolong(int n0c, int n1c, const T* __restrict__ coarse, const T* __restrict__ divp,
-                             const T* __restrict__ maskf, T* __restrict__ fine, int add)
+// Six sweeps of a level in one launch, over tiles of RO x CO cells with a halo that
+// shrinks by a cell a sweep; for the levels whose sweep is shorter than a launch.
+// DOWN: the pre-smoothing, from f or (ZERO) from f = 0, then the residual, restricted
+// to the coarser level C; in = f, out = the smoothed field, which goes to another
+// buffer since tiles read one another's cells. Up: in + prolonged correction V, then
+// the six sweeps.
+// A block is bound by its SM's FP64 rate (1.7 lanes a clock), so the tile is as small
+// as it takes to cover the SMs: the host picks the size by the sum of the active cells.
+template <int RO, int CO, int HALO>
+constexpr int mg_tile_work()   // warps' rounds of a block over its sweeps
 {
-    const int jf = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i_f = blockIdx.y, b = blockIdx.z;
-    const int n1f = 2 * n1c;
-    if (jf >= n1f) return;
-    const long long fsc = (long long)n0c * n1c, fsf = 4 * fsc;
-    const T v = mg_prolong_pt(coarse + b * fsc, n0c, n1c, i_f, jf, divp, maskf);
-    const long long o = (long long)i_f * n1f + jf;
-    fine[b * fsf + o] = add ? fine[b * fsf + o] + v : v;
+    int n = 0;
+    for (int h = HALO - 1; h >= HALO - 6; --h) n += ((RO + 2 * h) * (CO + 2 * h) + 31) / 32;
+    return n;
+}
+
+template <int RO, int CO> constexpr int mg_tile_nt = RO * CO >= 256 ? 512 : 256;   // threads
+
+template <typename T, int RO, int CO, bool DOWN, bool ZERO>
+__global__ void __launch_bounds__(mg_tile_nt<RO, CO>) k_mg_tile(MgLev<T> L, MgLev<T> C, const T* __restrict__ in,
+                                                 const T* __restrict__ V, const T* __restrict__ rhs,
+                                                 const T* __restrict__ rr, T* __restrict__ out, MgDown<T> d, T omega)
+{
+    constexpr int H = DOWN ? 7 : 6;                  // halo: the sweeps, and the residual's
+    constexpr int NT = mg_tile_nt<RO, CO>;
+    constexpr int RR = RO + 2 * H, CC = CO + 2 * H;
+    __shared__ T s[2][RR * CC];
+    const int b = blockIdx.z, tid = threadIdx.x;
+    const int i0 = (int)blockIdx.y * RO - H, j0 = (int)blockIdx.x * CO - H;
+    const long long fs = (long long)L.n0 * L.n1;
+    rr += b * fs;
+    rhs += b * fs;
+    auto inside = [&](int i, int j) { return i >= 0 && i < L.n0 && j >= 0 && j < L.n1; };
+    for (int e = tid; e < RR * CC; e += NT) {
+        const int r = e / CC, c = e % CC, i = i0 + r, j = j0 + c;
+        T x = T(0);
+        if (inside(i, j)) {
+            const long long o = (long long)i * L.n1 + j;
+            if constexpr (DOWN && ZERO) {
+                x = mg_first(L, rr[o], b, o);
+            } else {
+                x = in[b * fs + o];
+                if constexpr (!DOWN) {
+                    const long long fc = (long long)C.n0 * C.n1;
+                    x = mg_prolong_pt(V + b * fc, C.n0, C.n1, i, j, L.mp[o], x);
+                }
+            }
+        }
+        s[0][e] = x;
+        s[1][e] = T(0);   // cells outside the grid stay 0 in both
+    }
+    __syncthreads();
+    constexpr int FIRST = DOWN && ZERO ? 1 : 0;      // sweeps already done
+#pragma unroll
+    for (int k = FIRST; k < 6; ++k) {
+        const T* const src = s[(k - FIRST) & 1];
+        T* const dst = s[(k - FIRST + 1) & 1];
+        const int m = k + 1, W = CC - 2 * m, N = (RR - 2 * m) * W;
+        for (int e = tid; e < N; e += NT) {
+            const int r = e / W + m, c = e % W + m, i = i0 + r, j = j0 + c;
+            if (inside(i, j)) {
+                const T* q = src + r * CC + c;
+                dst[r * CC + c] = mg_update(L, q[0], q[CC], q[-CC], q[1], q[-1], rr[(long long)i * L.n1 + j], b, i, j,
+                                            omega);
+            }
+        }
+        __syncthreads();
+    }
+    const T* const res = s[(6 - FIRST) & 1];
+    for (int e = tid; e < RO * CO; e += NT) {
+        const int r = e / CO + H, c = e % CO + H, i = i0 + r, j = j0 + c;
+        if (inside(i, j)) out[b * fs + (long long)i * L.n1 + j] = res[r * CC + c];
+    }
+    if constexpr (DOWN) {
+        const T lam = L.lam[b];
+        for (int e = tid; e < RO * CO / 4; e += NT) {
+            const int R = e / (CO / 2), Cc = e % (CO / 2);
+            if (!inside(i0 + H + 2 * R, j0 + H + 2 * Cc)) continue;
+            T x[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const int r = H + 2 * R + u, c = H + 2 * Cc + v, i = i0 + r, j = j0 + c;
+                    const T* q = res + r * CC + c;
+                    x[u][v] = mg_resid(L, q[0], q[CC], q[-CC], q[1], q[-1], rhs[(long long)i * L.n1 + j], lam, i, j);
+                }
+            const int I = (int)blockIdx.y * (RO / 2) + R, J = (int)blockIdx.x * (CO / 2) + Cc;
+            const long long o = (long long)I * C.n1 + J;
+            mg_put_rhs(C, d, (x[0][0] + x[1][0] + x[0][1] + x[1][1]) * C.mr[o], b, o);
+        }
+    }
 }
 
 // bottom: f[b][idx[m]] = sum_l rhs[b][idx[l]] inv[b][l][m]  (341-346)
@@ -257,26 +460,25 @@ __global__ void k_mg_bottom(int nb, long long fs, const int32_t* __restrict__ id
 }
 
 // ---------------------------------------------------------------------------
-// Coarse levels in one block per system. Below a few thousand cells a level's
+// Coarse levels in one block (or one cluster of blocks) per system. Below a few thousand cells a level's
 // sweep is shorter than a kernel launch, and the bottom smoothing alone is
 // 6 x niter_bottom sweeps per V-cycle; this kernel runs everything from level
 // l0 down (the V-cycle, or the full-multigrid start) with the block's threads
-// striding over the level and __syncthreads() between phases. The solution,
+// striding over the level and a barrier between phases. The solution,
 // right-hand side and scratch of every level from l0 down live in shared
 // memory (level l0's come in from, and its solution goes back to, global
 // memory); the coefficients are read-only global tables; the arithmetic is
 // the per-point functions above.
 // ---------------------------------------------------------------------------
 constexpr int MG_MAXLEV = 16;
+constexpr long long MG_TILE_MAX = 65536;
 
 template <typename T>
 struct MgCoarseArgs {
-    int l0, nlev, niter_bottom, nb, fmg;
+    int l0, nlev, niter_bottom, nb, fmg, zero;   // zero: the V-cycle starts from f = 0
     T omega;
     MgLev<T> L[MG_MAXLEV];
-    const T* divr[MG_MAXLEV];   // restriction divisor of coarse level l
-    const T* divp[MG_MAXLEV];   // prolongation divisor of fine level l
-    int soff[MG_MAXLEV];        // shared-memory offset of level l: f, rhs, scratch (n0 n1 each)
+    int soff[MG_MAXLEV];        // shared-memory offset of level l: f, rhs, scratch, scaled rhs (n0 n1 each)
     T* f0;                      // level l0 solution (system-0 base): in (V-cycle) and out
     const T* rhs0;              // level l0 right-hand side (system-0 base)
     const int32_t* bot_idx;
@@ -286,7 +488,7 @@ struct MgCoarseArgs {
 
 template <typename T>
 struct MgcLevel {
-    T *f, *rhs, *tmp;
+    T *f, *rhs, *tmp, *rr;   // rr: what the sweeps read (mg_scaled_rhs)
     int n;
 };
 
@@ -298,147 +500,204 @@ __device__ __forceinline__ MgcLevel<T> mgc_level(const MgCoarseArgs<T>& A, T* sm
     v.f = sm + A.soff[l];
     v.rhs = v.f + v.n;
     v.tmp = v.rhs + v.n;
+    v.rr = mg_scaled<T> ? v.tmp + v.n : v.rhs;
     return v;
 }
 
-template <typename T>
-__device__ void mgc_smooth(const MgCoarseArgs<T>& A, T* sm, int l, int b, int times)
+// The threads of one system's coarse kernel: one block, or a cluster of blocks (CL)
+// that each hold every level in their own shared memory, take a share of the cells of
+// a phase, and store a result into all of the copies. A phase then reads locally and
+// ends at a cluster barrier instead of a block barrier.
+template <typename T, bool CL>
+struct McTeam {
+    int rank, nb;   // block of the cluster, blocks
+    __device__ __forceinline__ int first() const { return rank * (int)blockDim.x + (int)threadIdx.x; }
+    __device__ __forceinline__ int step() const { return nb * (int)blockDim.x; }
+    __device__ __forceinline__ void put(T* p, T v) const
+    {
+        if constexpr (CL) {
+            const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+            for (int r = 0; r < nb; ++r) {
+                uint32_t q;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(a), "r"(r));
+                if constexpr (sizeof(T) == 8)
+                    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(q), "d"(v) : "memory");
+                else
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(q), "f"(v) : "memory");
+            }
+        } else {
+            *p = v;
+        }
+    }
+    __device__ __forceinline__ void sync() const
+    {
+        if constexpr (CL) {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    }
+};
+
+template <typename T, bool CL>
+__device__ void mgc_smooth(const MgCoarseArgs<T>& A, const McTeam<T, CL>& tm, T* sm, int l, int b, int times)
 {
     const MgLev<T>& L = A.L[l];
     const MgcLevel<T> v = mgc_level(A, sm, l);
-    const T* fac = L.factor + (long long)b * v.n;
     for (int t = 0; t < times; ++t)
         for (int s = 0; s < 6; ++s) {
             const T* src = (s % 2 == 0) ? v.f : v.tmp;
             T* dst = (s % 2 == 0) ? v.tmp : v.f;
-            for (int o = threadIdx.x; o < v.n; o += blockDim.x) {
+            for (int o = tm.first(); o < v.n; o += tm.step()) {
                 const int i = o / L.n1, j = o - i * L.n1;
-                dst[o] = mg_sweep_pt(L, src, v.rhs[o], __ldg(fac + o), i, j, A.omega);
+                tm.put(dst + o, mg_sweep_pt(L, src, v.rr[o], b, i, j, A.omega));
             }
-            __syncthreads();
+            tm.sync();
         }
 }
 
-template <typename T>
-__device__ void mgc_bottom(const MgCoarseArgs<T>& A, T* sm, int b)
+template <typename T> __device__ __forceinline__ T mg_warp_sum(T x)
+{
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) x += __shfl_xor_sync(0xffffffffu, x, k);
+    return x;
+}
+
+template <typename T, bool CL>
+__device__ void mgc_bottom(const MgCoarseArgs<T>& A, const McTeam<T, CL>& tm, T* sm, int b)
 {
     const int l = A.nlev - 1;
+    const MgcLevel<T> v = mgc_level(A, sm, l);
     if (A.niter_bottom > 0 && A.bot_sm != nullptr) {
-        // f = N rhs (+ M f when the grid has one level; below it f is zero here)
-        const MgcLevel<T> v = mgc_level(A, sm, l);
+        // f = N rhs (+ M f when the grid has one level; below it f is zero here), a warp
+        // a cell: the rows of N and M are contiguous
         const long long n2 = (long long)v.n * v.n;
         const T* Nm = A.bot_sm + (long long)b * 2 * n2;
         const T* Mm = Nm + n2;
-        for (int m = threadIdx.x; m < v.n; m += blockDim.x) {
+        const int lane = threadIdx.x & 31;
+        for (int m = tm.first() >> 5; m < v.n; m += tm.step() >> 5) {
             T s = T(0);
-            for (int k = 0; k < v.n; ++k) s += __ldg(Nm + (long long)k * v.n + m) * v.rhs[k];
+            for (int k = lane; k < v.n; k += 32) s += __ldg(Nm + (long long)m * v.n + k) * v.rhs[k];
             if (A.nlev == 1)
-                for (int k = 0; k < v.n; ++k) s += __ldg(Mm + (long long)k * v.n + m) * v.f[k];
-            v.tmp[m] = s;
+                for (int k = lane; k < v.n; k += 32) s += __ldg(Mm + (long long)m * v.n + k) * v.f[k];
+            s = mg_warp_sum(s);
+            if (lane == 0) tm.put(v.tmp + m, s);
         }
-        __syncthreads();
-        for (int m = threadIdx.x; m < v.n; m += blockDim.x) v.f[m] = v.tmp[m];
-        __syncthreads();
+        tm.sync();
+        for (int m = threadIdx.x; m < v.n; m += blockDim.x) v.f[m] = v.tmp[m];   // every block its own copy
+        tm.sync();
         return;
     }
     if (A.niter_bottom > 0) {
-        mgc_smooth(A, sm, l, b, A.niter_bottom);
+        mgc_smooth(A, tm, sm, l, b, A.niter_bottom);
         return;
     }
-    const MgcLevel<T> v = mgc_level(A, sm, l);
     for (int o = threadIdx.x; o < v.n; o += blockDim.x) v.f[o] = T(0);
-    __syncthreads();
+    tm.sync();
     const T* P = A.bot_inv + (long long)b * A.nb * A.nb;
-    for (int m = threadIdx.x; m < A.nb; m += blockDim.x) {
+    for (int m = tm.first(); m < A.nb; m += tm.step()) {
         T s = T(0);
         for (int k = 0; k < A.nb; ++k) s += v.rhs[__ldg(A.bot_idx + k)] * __ldg(P + (long long)k * A.nb + m);
-        v.f[__ldg(A.bot_idx + m)] = s;
+        tm.put(v.f + __ldg(A.bot_idx + m), s);
     }
-    __syncthreads();
+    tm.sync();
 }
 
 // rhs of level lc from a fine-level field (shared memory)
-template <typename T>
-__device__ void mgc_restrict(const MgCoarseArgs<T>& A, T* sm, const T* fine, int lc)
+template <typename T, bool CL>
+__device__ void mgc_restrict(const MgCoarseArgs<T>& A, const McTeam<T, CL>& tm, T* sm, const T* fine, int lc, int b)
 {
     const MgLev<T>& C = A.L[lc];
     const MgcLevel<T> v = mgc_level(A, sm, lc);
-    for (int o = threadIdx.x; o < v.n; o += blockDim.x) {
+    for (int o = tm.first(); o < v.n; o += tm.step()) {
         const int I = o / C.n1, J = o - I * C.n1;
-        v.rhs[o] = mg_restrict_pt(fine, C.n1, I, J, A.divr[lc], C.mask);
+        const T x = mg_restrict_pt(fine, C.n1, I, J, C.mr);
+        tm.put(v.rhs + o, x);
+        if constexpr (mg_scaled<T>) tm.put(v.rr + o, mg_scaled_rhs(C, x, b, o));
     }
 }
 
-template <typename T>
-__device__ void mgc_prolong(const MgCoarseArgs<T>& A, T* sm, int l, bool add)
+template <typename T, bool CL>
+__device__ void mgc_prolong(const MgCoarseArgs<T>& A, const McTeam<T, CL>& tm, T* sm, int l, bool add)
 {
     const MgLev<T>& Fl = A.L[l];
     const MgLev<T>& C = A.L[l + 1];
     const MgcLevel<T> vf = mgc_level(A, sm, l), vc = mgc_level(A, sm, l + 1);
-    for (int o = threadIdx.x; o < vf.n; o += blockDim.x) {
+    for (int o = tm.first(); o < vf.n; o += tm.step()) {
         const int i = o / Fl.n1, j = o - i * Fl.n1;
-        const T x = mg_prolong_pt(vc.f, C.n0, C.n1, i, j, A.divp[l], Fl.mask);
-        vf.f[o] = add ? vf.f[o] + x : x;
+        tm.put(vf.f + o, mg_prolong_pt(vc.f, C.n0, C.n1, i, j, Fl.mp[o], add ? vf.f[o] : T(0)));
     }
-    __syncthreads();
+    tm.sync();
 }
 
-template <typename T>
-__device__ void mgc_vcycle(const MgCoarseArgs<T>& A, T* sm, int l0, int b)
+template <typename T, bool CL>
+__device__ void mgc_vcycle(const MgCoarseArgs<T>& A, const McTeam<T, CL>& tm, T* sm, int l0, int b)
 {
     const int last = A.nlev - 1;
     for (int l = l0; l < last; ++l) {
-        mgc_smooth(A, sm, l, b, 1);
+        mgc_smooth(A, tm, sm, l, b, 1);
         const MgLev<T>& L = A.L[l];
         const MgcLevel<T> v = mgc_level(A, sm, l);
-        for (int o = threadIdx.x; o < v.n; o += blockDim.x) {
+        for (int o = tm.first(); o < v.n; o += tm.step()) {
             const int i = o / L.n1, j = o - i * L.n1;
-            v.tmp[o] = mg_residual_pt(L, v.f, v.rhs[o], L.lam[b], i, j);
+            tm.put(v.tmp + o, mg_residual_pt(L, v.f, v.rhs[o], L.lam[b], i, j));
         }
-        __syncthreads();
-        mgc_restrict(A, sm, v.tmp, l + 1);
+        tm.sync();
+        mgc_restrict(A, tm, sm, v.tmp, l + 1, b);
         const MgcLevel<T> c = mgc_level(A, sm, l + 1);
         for (int o = threadIdx.x; o < c.n; o += blockDim.x) c.f[o] = T(0);
-        __syncthreads();
+        tm.sync();
     }
-    mgc_bottom(A, sm, b);
+    mgc_bottom(A, tm, sm, b);
     for (int l = last - 1; l >= l0; --l) {
-        mgc_prolong(A, sm, l, true);
-        mgc_smooth(A, sm, l, b, 1);
+        mgc_prolong(A, tm, sm, l, true);
+        mgc_smooth(A, tm, sm, l, b, 1);
     }
 }
 
-template <typename T>
+template <typename T, bool CL>
 __global__ void __launch_bounds__(1024) k_mg_coarse(MgCoarseArgs<T> A)
 {
     extern __shared__ __align__(16) unsigned char mg_smem[];
     T* sm = reinterpret_cast<T*>(mg_smem);
-    const int b = blockIdx.x;
+    McTeam<T, CL> tm;
+    tm.rank = 0;
+    tm.nb = 1;
+    if constexpr (CL) {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(tm.rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(tm.nb));
+    }
+    const int b = blockIdx.x / tm.nb;
     const MgcLevel<T> v0 = mgc_level(A, sm, A.l0);
     const long long g0 = (long long)b * v0.n;
+    // (every block reads the whole level into its copy; the barrier also says that
+    // every block of the cluster has started, before the first store into it)
     for (int o = threadIdx.x; o < v0.n; o += blockDim.x) {
         v0.rhs[o] = A.rhs0[g0 + o];
-        if (!A.fmg) v0.f[o] = A.f0[g0 + o];
+        if constexpr (mg_scaled<T>) v0.rr[o] = mg_scaled_rhs(A.L[A.l0], v0.rhs[o], b, o);
+        if (!A.fmg) v0.f[o] = A.zero ? T(0) : A.f0[g0 + o];
     }
-    __syncthreads();
+    tm.sync();
     if (!A.fmg) {
-        mgc_vcycle(A, sm, A.l0, b);
+        mgc_vcycle(A, tm, sm, A.l0, b);
     } else {
         const int last = A.nlev - 1;
         for (int l = A.l0 + 1; l <= last; ++l) {
-            mgc_restrict(A, sm, mgc_level(A, sm, l - 1).rhs, l);
-            __syncthreads();
+            mgc_restrict(A, tm, sm, mgc_level(A, sm, l - 1).rhs, l, b);
+            tm.sync();
         }
         const MgcLevel<T> vb = mgc_level(A, sm, last);
         for (int o = threadIdx.x; o < vb.n; o += blockDim.x) vb.f[o] = T(0);
-        __syncthreads();
-        mgc_bottom(A, sm, b);
+        tm.sync();
+        mgc_bottom(A, tm, sm, b);
         for (int l = last - 1; l >= A.l0; --l) {
-            mgc_prolong(A, sm, l, false);
-            mgc_vcycle(A, sm, l, b);
+            mgc_prolong(A, tm, sm, l, false);
+            mgc_vcycle(A, tm, sm, l, b);
         }
     }
-    for (int o = threadIdx.x; o < v0.n; o += blockDim.x) A.f0[g0 + o] = v0.f[o];
+    // (the last phase's barrier: no block stores into another any more)
+    for (int o = tm.first(); o < v0.n; o += tm.step()) A.f0[g0 + o] = v0.f[o];
 }
 
 template <typename T>
@@ -451,6 +710,8 @@ __global__ void k_mg_zero(long long n, T* __restrict__ x)
 }  // namespace vd
 
 namespace {
+
+constexpr int MG_COARSE_CL = 256;   // threads of a clustered block (512: 6.26 ms a solve for 6.16)
 
 template <typename T>
 struct MgRun {
@@ -468,12 +729,31 @@ struct MgRun {
         L.cu = (const T*)D.cu;
         L.cv = (const T*)D.cv;
         L.factor = (const T*)D.factor;
+        L.g = (const T*)D.g;
+        L.mr = (const T*)D.mr;
+        L.mp = (const T*)D.mp;
         L.lam = (const T*)p->lam;
         return L;
     }
-    T* buf(int l, int which) const { return ws + p->ws_off[3 * l + which]; }
+    T* buf(int l, int which) const { return ws + p->ws_off[4 * l + which]; }
+    // what the sweeps of level l read for the right-hand side rhs
+    const T* scaled(int l, const T* rhs) const { return vd::mg_scaled<T> ? buf(l, 3) : rhs; }
+    vd::MgDown<T> down(int l) const
+    {
+        vd::MgDown<T> d;
+        d.rhs = buf(l, 1);
+        d.rr = vd::mg_scaled<T> ? buf(l, 3) : nullptr;
+        d.first = (l < p->lc && !tiled(l)) ? buf(l, 2) : nullptr;
+        return d;
+    }
     long long nel(int l) const { return (long long)p->nsys * p->lv[l].n0 * p->lv[l].n1; }
     dim3 grid(int n0, int n1) const { return dim3((unsigned)((n1 + 127) / 128), (unsigned)n0, (unsigned)p->nsys); }
+
+    // Levels whose six sweeps run as one tile kernel: those of at most MG_TILE_MAX cells
+    // (all systems), where a sweep is shorter than its launch; above, the halo's extra
+    // FP64 work costs more than the launches. A 1024 x 768 float64 solve with the line at
+    // 0, 4096, 16384, 65536 and 262144 cells: 6.61, 6.40, 6.25, 6.16 and 6.45 ms.
+    bool tiled(int l) const { return l < p->nlev - 1 && l < p->lc && nel(l) <= vd::MG_TILE_MAX; }
 
     int zero(T* x, long long n) const
     {
@@ -481,22 +761,55 @@ struct MgRun {
         VD_LAUNCH_CHECK();
         return VD_OK;
     }
-    // `times` smooths of 6 damped sweeps, ping-pong through the level's tmp buffer
-    int smooth(int l, T* f, const T* rhs, int times) const
+    // `times` smooths of 6 damped sweeps, ping-pong through the level's tmp buffer;
+    // started: the first sweep is in tmp already (from f = 0)
+    int smooth(int l, T* f, const T* rhs, int times, bool started = false) const
     {
         const vd::MgLev<T> L = lev(l);
         T* tmp = buf(l, 2);
+        const T* rr = scaled(l, rhs);
         const dim3 g = grid(L.n0, L.n1);
-        for (int t = 0; t < times; ++t)
-            for (int s = 0; s < 6; ++s) {
-                const T* src = (s % 2 == 0) ? f : tmp;
-                T* dst = (s % 2 == 0) ? tmp : f;
-                vd::k_mg_sweep<T><<<g, 128, 0, st>>>(L, src, rhs, dst, T(p->omega));
-                VD_LAUNCH_CHECK();
-            }
+        for (int s = started ? 1 : 0; s < 6 * times; ++s) {
+            const T* src = (s % 2 == 0) ? f : tmp;
+            T* dst = (s % 2 == 0) ? tmp : f;
+            vd::k_mg_sweep<T><<<g, 128, 0, st>>>(L, src, rr, dst, T(p->omega));
+            VD_LAUNCH_CHECK();
+        }
         return VD_OK;
     }
-    int bottom(T* f, const T* rhs) const
+    template <int RO, int CO>
+    int tile(int l, bool dn, bool started, const T* in, const T* V, const T* rhs, T* out) const
+    {
+        const vd::MgLev<T> L = lev(l), C = lev(l + 1);
+        const dim3 g((unsigned)((L.n1 + CO - 1) / CO), (unsigned)((L.n0 + RO - 1) / RO), (unsigned)p->nsys);
+        const int nt = vd::mg_tile_nt<RO, CO>;
+        const T w = T(p->omega);
+        const T* rr = scaled(l, rhs);
+        const vd::MgDown<T> d = down(l + 1);
+        if (!dn) vd::k_mg_tile<T, RO, CO, false, false><<<g, nt, 0, st>>>(L, C, in, V, rhs, rr, out, d, w);
+        else if (started) vd::k_mg_tile<T, RO, CO, true, true><<<g, nt, 0, st>>>(L, C, in, V, rhs, rr, out, d, w);
+        else vd::k_mg_tile<T, RO, CO, true, false><<<g, nt, 0, st>>>(L, C, in, V, rhs, rr, out, d, w);
+        VD_LAUNCH_CHECK();
+        return VD_OK;
+    }
+    // the tile that keeps the busiest SM shortest: work of a block x blocks an SM
+    int tile_any(int l, bool dn, bool started, const T* in, const T* V, const T* rhs, T* out) const
+    {
+        auto cost = [&](int ro, int co, int work) {
+            const long long nb = (long long)((p->lv[l].n0 + ro - 1) / ro) * ((p->lv[l].n1 + co - 1) / co) * p->nsys;
+            return ((nb + 151) / 152) * work;
+        };
+        const long long c0 = cost(8, 8, vd::mg_tile_work<8, 8, 6>()), c1 = cost(8, 16, vd::mg_tile_work<8, 16, 6>()),
+                        c2 = cost(16, 16, vd::mg_tile_work<16, 16, 6>()),
+                        c3 = cost(16, 32, vd::mg_tile_work<16, 32, 6>());
+        const long long m = std::min(std::min(c0, c1), std::min(c2, c3));
+        if (c3 == m) return tile<16, 32>(l, dn, started, in, V, rhs, out);
+        if (c2 == m) return tile<16, 16>(l, dn, started, in, V, rhs, out);
+        if (c1 == m) return tile<8, 16>(l, dn, started, in, V, rhs, out);
+        return tile<8, 8>(l, dn, started, in, V, rhs, out);
+    }
+    // started: f starts from zero (and its first sweep is in tmp)
+    int bottom(T* f, const T* rhs, bool started) const
     {
         const int l = p->nlev - 1;
         if (p->niter_bottom <= 0) {
@@ -510,52 +823,75 @@ struct MgRun {
             }
             return VD_OK;
         }
-        return smooth(l, f, rhs, p->niter_bottom);
+        return smooth(l, f, rhs, p->niter_bottom, started);
     }
     // levels >= l0 in one block per system (p->lc <= l0): a V-cycle on (f, rhs)
-    // at l0, or (fmg) the full-multigrid start from the restricted rhs at l0
-    int coarse(T* f, const T* rhs, int l0, bool fmg) const
+    // at l0 (from f = 0 where zero_f), or (fmg) the full-multigrid start from the
+    // restricted rhs at l0
+    int coarse(T* f, const T* rhs, int l0, bool fmg, bool zero_f) const
     {
         vd::MgCoarseArgs<T> A;
         A.l0 = l0; A.nlev = p->nlev; A.niter_bottom = p->niter_bottom; A.nb = p->nb; A.fmg = fmg ? 1 : 0;
+        A.zero = zero_f ? 1 : 0;
         A.omega = T(p->omega);
         int off = 0;
         for (int l = 0; l < p->nlev; ++l) {
             A.L[l] = lev(l);
-            A.divr[l] = (const T*)p->dl[l].divr;
-            A.divp[l] = (const T*)p->dl[l].divp;
             A.soff[l] = off;
-            if (l >= l0) off += 3 * p->lv[l].n0 * p->lv[l].n1;
+            if (l >= l0) off += (vd::mg_scaled<T> ? 4 : 3) * p->lv[l].n0 * p->lv[l].n1;
         }
         A.f0 = f;
         A.rhs0 = rhs;
         A.bot_idx = p->bot_idx;
         A.bot_inv = (const T*)p->bot_inv;
         A.bot_sm = (const T*)p->bot_sm;
-        vd::k_mg_coarse<T><<<(unsigned)p->nsys, 1024, (size_t)off * sizeof(T), st>>>(A);
+        const size_t smem = (size_t)off * sizeof(T);
+        // blocks a system: one in float32 (a phase is shorter than a cluster barrier);
+        // in float64, where one SM's FP64 rate is the bound, a cluster of up to 8 while
+        // the systems' clusters fit the GPU at once (15 of 8). Levels of 768 and 192 cells:
+        // 43.5 us a V-cycle with one block, 31.8 with 8, now bound by the barriers
+        int nc = 1;
+        if (vd::mg_scaled<T>)
+            while (nc < 8 && (long long)p->nsys * 2 * nc <= 120) nc *= 2;
+        if (nc == 1) {
+            vd::k_mg_coarse<T, false><<<(unsigned)p->nsys, 1024, smem, st>>>(A);
+        } else if constexpr (vd::mg_scaled<T>) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(p->nsys * nc));
+            cfg.blockDim = dim3(MG_COARSE_CL);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = (unsigned)nc;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            VD_CUDA_TRY(cudaLaunchKernelEx(&cfg, vd::k_mg_coarse<T, true>, A));
+        }
         VD_LAUNCH_CHECK();
         return VD_OK;
     }
-    int vcycle(T* f, const T* rhs, int l) const
+    // one V-cycle on (f, rhs) at level l. started: from f = 0, with the first sweep
+    // in tmp where the level's sweeps are single launches
+    int vcycle(T* f, const T* rhs, int l, bool started) const
     {
-        if (l >= p->lc) return coarse(f, rhs, l, false);
-        if (l == p->nlev - 1) return bottom(f, rhs);
+        if (l >= p->lc) return coarse(f, rhs, l, false, started);
+        if (l == p->nlev - 1) return bottom(f, rhs, started);
         int rc;
-        if ((rc = smooth(l, f, rhs, 1))) return rc;
-        const vd::MgLev<T> L = lev(l);
-        T* res = buf(l, 2);
-        vd::k_mg_residual<T><<<grid(L.n0, L.n1), 128, 0, st>>>(L, f, rhs, res);
-        VD_LAUNCH_CHECK();
-        const int n0c = p->lv[l + 1].n0, n1c = p->lv[l + 1].n1;
+        const vd::MgLev<T> L = lev(l), C = lev(l + 1);
         T* rcz = buf(l + 1, 1);
         T* ec = buf(l + 1, 0);
-        vd::k_mg_restrict<T><<<grid(n0c, n1c), 128, 0, st>>>(n0c, n1c, res, (const T*)p->dl[l + 1].divr,
-                                                              (const T*)p->dl[l + 1].mask, rcz);
+        if (tiled(l)) {
+            if ((rc = tile_any(l, true, started, f, nullptr, rhs, buf(l, 2)))) return rc;
+            if ((rc = vcycle(ec, rcz, l + 1, true))) return rc;
+            return tile_any(l, false, false, buf(l, 2), ec, rhs, f);
+        }
+        if ((rc = smooth(l, f, rhs, 1, started))) return rc;
+        vd::k_mg_resid_restrict<T><<<grid(C.n0, C.n1), 128, 0, st>>>(L, C, f, rhs, down(l + 1));
         VD_LAUNCH_CHECK();
-        if ((rc = zero(ec, nel(l + 1)))) return rc;
-        if ((rc = vcycle(ec, rcz, l + 1))) return rc;
-        vd::k_mg_prolong<T><<<grid(L.n0, L.n1), 128, 0, st>>>(n0c, n1c, ec, (const T*)p->dl[l].divp,
-                                                              (const T*)p->dl[l].mask, f, 1);
+        if ((rc = vcycle(ec, rcz, l + 1, true))) return rc;
+        vd::k_mg_prolong<T><<<grid(C.n0, C.n1), 128, 0, st>>>(L, C.n0, C.n1, ec, f, 1);
         VD_LAUNCH_CHECK();
         return smooth(l, f, rhs, 1);
     }
@@ -564,51 +900,41 @@ struct MgRun {
     {
         const int n = p->nlev;
         int rc;
+        if (vd::mg_scaled<T>) {
+            vd::k_mg_scale<T><<<grid(p->n0, p->n1), 128, 0, st>>>(lev(0), rhs, buf(0, 3));
+            VD_LAUNCH_CHECK();
+        }
         if (n == 1) {
             if ((rc = zero(out, nel(0)))) return rc;
-            if ((rc = bottom(out, rhs))) return rc;
-        } else if (p->lc < n) {
-            // host levels down to lc, then the coarse kernel's full-multigrid start
-            const int lc = p->lc;
-            for (int i = 1; i <= lc; ++i) {
-                const T* src = (i == 1) ? rhs : buf(i - 1, 1);
-                vd::k_mg_restrict<T><<<grid(p->lv[i].n0, p->lv[i].n1), 128, 0, st>>>(
-                    p->lv[i].n0, p->lv[i].n1, src, (const T*)p->dl[i].divr, (const T*)p->dl[i].mask, buf(i, 1));
-                VD_LAUNCH_CHECK();
-            }
-            if ((rc = coarse(lc == 0 ? out : buf(lc, 0), lc == 0 ? rhs : buf(lc, 1), lc, true))) return rc;
-            for (int L = lc - 1; L >= 0; --L) {
-                T* fL = (L == 0) ? out : buf(L, 0);
-                const T* rL = (L == 0) ? rhs : buf(L, 1);
-                vd::k_mg_prolong<T><<<grid(p->lv[L].n0, p->lv[L].n1), 128, 0, st>>>(
-                    p->lv[L + 1].n0, p->lv[L + 1].n1, buf(L + 1, 0), (const T*)p->dl[L].divp,
-                    (const T*)p->dl[L].mask, fL, 0);
-                VD_LAUNCH_CHECK();
-                if ((rc = vcycle(fL, rL, L))) return rc;
-            }
+            if ((rc = bottom(out, rhs, false))) return rc;
         } else {
-            for (int i = 1; i < n; ++i) {
-                const T* src = (i == 1) ? rhs : buf(i - 1, 1);
+            // right-hand sides down to the coarse kernel's first level or the bottom,
+            // the start there, and a V-cycle on every level up
+            const int lb = p->lc < n ? p->lc : n - 1;
+            for (int i = 1; i <= lb; ++i) {
                 vd::k_mg_restrict<T><<<grid(p->lv[i].n0, p->lv[i].n1), 128, 0, st>>>(
-                    p->lv[i].n0, p->lv[i].n1, src, (const T*)p->dl[i].divr, (const T*)p->dl[i].mask, buf(i, 1));
+                    lev(i), (i == 1) ? rhs : buf(i - 1, 1), down(i));
                 VD_LAUNCH_CHECK();
             }
-            T* fb = buf(n - 1, 0);
-            if ((rc = zero(fb, nel(n - 1)))) return rc;
-            if ((rc = bottom(fb, buf(n - 1, 1)))) return rc;
-            for (int i = 2; i <= n; ++i) {
-                const int L = n - i;
+            T* fb = lb == 0 ? out : buf(lb, 0);
+            const T* rb = lb == 0 ? rhs : buf(lb, 1);
+            if (p->lc < n) {
+                if ((rc = coarse(fb, rb, lb, true, false))) return rc;
+            } else {
+                if ((rc = zero(fb, nel(lb)))) return rc;
+                if ((rc = bottom(fb, rb, false))) return rc;
+            }
+            for (int L = lb - 1; L >= 0; --L) {
                 T* fL = (L == 0) ? out : buf(L, 0);
                 const T* rL = (L == 0) ? rhs : buf(L, 1);
-                vd::k_mg_prolong<T><<<grid(p->lv[L].n0, p->lv[L].n1), 128, 0, st>>>(
-                    p->lv[L + 1].n0, p->lv[L + 1].n1, buf(L + 1, 0), (const T*)p->dl[L].divp,
-                    (const T*)p->dl[L].mask, fL, 0);
+                vd::k_mg_prolong<T><<<grid(p->lv[L + 1].n0, p->lv[L + 1].n1), 128, 0, st>>>(
+                    lev(L), p->lv[L + 1].n0, p->lv[L + 1].n1, buf(L + 1, 0), fL, 0);
                 VD_LAUNCH_CHECK();
-                if ((rc = vcycle(fL, rL, L))) return rc;
+                if ((rc = vcycle(fL, rL, L, false))) return rc;
             }
         }
         for (int it = 0; it < p->max_ite; ++it)
-            if ((rc = vcycle(out, rhs, 0))) return rc;
+            if ((rc = vcycle(out, rhs, 0, false))) return rc;
         return VD_OK;
     }
 };
@@ -669,7 +995,7 @@ void helm_apply(const HLevel& L, double lam, const std::vector<double>& f, std::
 
 // The bottom level's K damped Jacobi sweeps (the device formula, in float64)
 // as f_K = M f_0 + N rhs, by sweeping unit vectors; appended to `out` as
-// N then M (zeros when !with_m), each [input k][output m].
+// N then M (zeros when !with_m), each [output m][input k].
 void bottom_sweep_matrices(const HLevel& L, const double* factor, double omega, int K, bool with_m,
                            std::vector<double>& out)
 {
@@ -699,8 +1025,8 @@ void bottom_sweep_matrices(const HLevel& L, const double* factor, double omega, 
                 sweep(f, g);
                 f.swap(g);
             }
-            double* dst = out.data() + base + (size_t)pass * n * n + (size_t)k * n;
-            std::copy(f.begin(), f.end(), dst);
+            double* dst = out.data() + base + (size_t)pass * n * n + k;
+            for (int m = 0; m < n; ++m) dst[(size_t)m * n] = f[m];
         }
 }
 
@@ -726,7 +1052,7 @@ int mg_upload(vd_mg_plan* p, const std::vector<int32_t>& idx, const std::vector<
               const std::vector<double>& bsm)
 {
     Blob bl;
-    struct Off { size_t mask, cu, cv, factor, divr, divp; };
+    struct Off { size_t mask, cu, cv, factor, g, mr, mp; };
     std::vector<Off> off(p->nlev);
     for (int l = 0; l < p->nlev; ++l) {
         const HLevel& L = p->lv[l];
@@ -739,8 +1065,26 @@ int mg_upload(vd_mg_plan* p, const std::vector<int32_t>& idx, const std::vector<
         off[l].cu = bl.addv<T>(cus);
         off[l].cv = bl.addv<T>(cvs);
         off[l].factor = bl.addv<T>(fw);
-        off[l].divr = L.divr.empty() ? 0 : bl.addv<T>(L.divr);
-        off[l].divp = L.divp.empty() ? 0 : bl.addv<T>(L.divp);
+        // the sweep's coefficients towards i+1, i-1, j+1, j-1, times the factor
+        off[l].g = 0;
+        if (vd::mg_scaled<T>) {
+            const size_t n = (size_t)L.n0 * L.n1;
+            std::vector<double> g(4 * p->nsys * n);
+            for (int b = 0; b < p->nsys; ++b)
+                for (int i = 0; i < L.n0; ++i)
+                    for (int j = 0; j < L.n1; ++j) {
+                        const size_t o = (size_t)i * L.n1 + j, ov = (size_t)i * (L.n1 + 1) + j;
+                        const double w = fw[b * n + o], c[4] = {cus[o + L.n1], cus[o], cvs[ov + 1], cvs[ov]};
+                        for (int k = 0; k < 4; ++k) g[(4 * b + k) * n + o] = w * c[k];
+                    }
+            off[l].g = bl.addv<T>(g);
+        }
+        // restriction and prolongation: mask / divisor
+        std::vector<double> mr(L.divr), mp(L.divp);
+        for (size_t k = 0; k < mr.size(); ++k) mr[k] = L.mask[k] / mr[k];
+        for (size_t k = 0; k < mp.size(); ++k) mp[k] = L.mask[k] / mp[k];
+        off[l].mr = mr.empty() ? 0 : bl.addv<T>(mr);
+        off[l].mp = mp.empty() ? 0 : bl.addv<T>(mp);
     }
     const size_t o_lam = bl.addv<T>(p->lambda);
     const size_t o_idx = bl.add(idx.data(), idx.size() * sizeof(int32_t));
@@ -755,8 +1099,9 @@ int mg_upload(vd_mg_plan* p, const std::vector<int32_t>& idx, const std::vector<
         p->dl[l].cu = b + off[l].cu;
         p->dl[l].cv = b + off[l].cv;
         p->dl[l].factor = b + off[l].factor;
-        p->dl[l].divr = p->lv[l].divr.empty() ? nullptr : b + off[l].divr;
-        p->dl[l].divp = p->lv[l].divp.empty() ? nullptr : b + off[l].divp;
+        p->dl[l].g = vd::mg_scaled<T> ? b + off[l].g : nullptr;
+        p->dl[l].mr = p->lv[l].divr.empty() ? nullptr : b + off[l].mr;
+        p->dl[l].mp = p->lv[l].divp.empty() ? nullptr : b + off[l].mp;
     }
     p->lam = b + o_lam;
     p->bot_idx = (const int32_t*)(b + o_idx);
@@ -869,12 +1214,13 @@ extern "C" vd_status vd_mg_plan_create(vd_mg_plan** out, const vd_mg_desc* d)
             std::copy(P.begin(), P.end(), inv.begin() + (size_t)b * p->nb * p->nb);
         }
     }
-    // workspace: per level f, rhs, tmp
+    // workspace: per level f, rhs, tmp and, in float64, the scaled rhs
     size_t offw = 0;
-    p->ws_off.resize(3 * nlev);
+    p->ws_off.resize(4 * nlev);
+    const int nbuf = p->dtype == VD_F64 ? 4 : 3;
     for (int l = 0; l < nlev; ++l)
-        for (int w = 0; w < 3; ++w) {
-            p->ws_off[3 * l + w] = offw;
+        for (int w = 0; w < nbuf; ++w) {
+            p->ws_off[4 * l + w] = offw;
             offw += (size_t)p->nsys * p->lv[l].n0 * p->lv[l].n1;
             offw = (offw + 63) & ~size_t(63);
         }
@@ -888,7 +1234,7 @@ extern "C" vd_status vd_mg_plan_create(vd_mg_plan** out, const vd_mg_desc* d)
     const long long max_cells = p->dtype == VD_F64 ? 1024 : 4096;
     for (int l = 0; l < nlev; ++l) {
         size_t sm = 0;
-        for (int k = l; k < nlev; ++k) sm += 3 * (size_t)p->lv[k].n0 * p->lv[k].n1 * esz;
+        for (int k = l; k < nlev; ++k) sm += nbuf * (size_t)p->lv[k].n0 * p->lv[k].n1 * esz;
         if ((long long)p->lv[l].n0 * p->lv[l].n1 <= max_cells && sm <= 200 * 1024) {
             p->lc = l;
             break;
@@ -897,9 +1243,11 @@ extern "C" vd_status vd_mg_plan_create(vd_mg_plan** out, const vd_mg_desc* d)
     if (nlev > vd::MG_MAXLEV) p->lc = nlev;
     if (p->lc < nlev) {
         const cudaError_t e = p->dtype == VD_F64
-            ? cudaFuncSetAttribute(vd::k_mg_coarse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
-            : cudaFuncSetAttribute(vd::k_mg_coarse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) {
+            ? cudaFuncSetAttribute(vd::k_mg_coarse<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
+            : cudaFuncSetAttribute(vd::k_mg_coarse<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        const cudaError_t e2 = cudaFuncSetAttribute(vd::k_mg_coarse<double, true>,
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess || e2 != cudaSuccess) {
             if (p->dev) cudaFree(p->dev);
             delete p;
             return VD_ERR_CUDA;

@@ -503,6 +503,13 @@ tridiag_global_kernel(T* __restrict__ spec, const T* __restrict__ trim, int my, 
 // and writes y[(j/Ns) Ns R + k + r Ns]; the output is in natural order) with
 // radix 4, 2, 3 and 5 stages and direct stages of other odd radices,
 // ping-ponging between two shared-memory buffers.
+// The oddness halves every stage. After the stages of product Ns the buffer holds
+// rows j < T = L/Ns of the DFTs B[j][k] of the subsequences z_{j + q T}, and
+//   B[T - j][k] = -e^{2 pi i k / Ns} B[j][Ns - k],   B[0][Ns - k] = -B[0][k],
+// so a stage forms rows j <= T/2 alone (of row 0 the first half), and reads a row
+// beyond T/2 as its mirror image, whose factor makes the twiddle another entry of
+// the table: -conj(tw[k (R - r)]). (Even radices come first among the small ones:
+// an odd T has one row that mirrors itself, an even T two.)
 // The orthonormal DST-I is its own inverse, so the inverse pass is the same
 // transform from the parity-split spectral rows to the field.
 // ---------------------------------------------------------------------------
@@ -580,30 +587,75 @@ template <> struct Dft<5> {
     }
 };
 
+// x with its sign flipped where neg (integers: an FP64 negation takes an issue slot)
+__device__ __forceinline__ double flip(double x, bool neg)
+{
+    return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+
+// A stage of a small radix over the rows j <= T/2 (T = L/(Ns R) output rows).
+// 4 x 256^2 (510 = 17 2 3 5): 19.0 us a pass, 27.8 with whole stages.
 template <int R>
 __device__ __forceinline__ void fft_stage(const double2* __restrict__ in, double2* __restrict__ out,
                                           const double2* __restrict__ tw, int L, int Ns, int pp)
 {
-    const int T = L / R;
-    const int tstep = L / (Ns * R);
-    for (int idx = threadIdx.x; idx < pp * T; idx += blockDim.x) {
-        const int q = idx / T;
-        const int j = idx - q * T;
-        const int k = j % Ns;
+    const int T = L / (Ns * R), Ti = T * R;      // output and input rows; tw[m T] = e^{-2 pi i m / (Ns R)}
+    const int n0 = Ns / 2 + 1;                   // butterflies of row 0
+    const int nb = n0 + (T / 2) * Ns;
+    for (int idx = threadIdx.x; idx < pp * nb; idx += blockDim.x) {
+        const int q = idx / nb;
+        int k = idx - q * nb, j = 0;
+        if (k >= n0) {
+            k -= n0;
+            j = k / Ns;
+            k -= j * Ns;
+            ++j;
+        }
         const double2* I = in + (long long)q * L;
         double2* O = out + (long long)q * L;
         double2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = I[j + r * T];
-        if (Ns > 1) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(tw + (long long)k * r * tstep));
+        for (int r = 0; r < R; ++r) {
+            const int row = j + r * T;
+            const bool up = 2 * row > Ti;
+            v[r] = I[up ? (Ti - row) * Ns + (k ? Ns - k : 0) : row * Ns + k];
+            if (r == 0) continue;                // row 0 .. T/2 is never beyond Ti/2
+            if (Ns > 1) {
+                double2 w = __ldg(tw + (long long)k * (up ? R - r : r) * T);
+                w.x = flip(w.x, up);
+                v[r] = cmul(v[r], w);
+            } else {
+                v[r] = make_double2(flip(v[r].x, up), flip(v[r].y, up));
+            }
         }
         Dft<R>::run(v);
-        const int base = (j / Ns) * Ns * R + k;
+        const int base = j * Ns * R + k;
 #pragma unroll
         for (int r = 0; r < R; ++r) O[base + r * Ns] = v[r];
+        if (j == 0) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int m = Ns * R - k - r * Ns;
+                if (m < Ns * R) O[m] = make_double2(flip(v[r].x, true), flip(v[r].y, true));
+            }
+        }
     }
+}
+
+// The rows beyond T/2 from their mirror images, for a direct odd stage that is not
+// the first (it works in place on whole columns).
+__device__ __forceinline__ void fft_expand(double2* __restrict__ in, const double2* __restrict__ tw, int L, int Ns,
+                                           int pp)
+{
+    const int T = L / Ns, nr = T - 1 - T / 2;    // rows T/2 + 1 .. T - 1
+    for (int idx = threadIdx.x; idx < pp * nr * Ns; idx += blockDim.x) {
+        const int qr = idx / Ns, k = idx - qr * Ns;
+        const int row = T / 2 + 1 + qr % nr;
+        double2* I = in + (long long)(qr / nr) * L;
+        const double2 w = __ldg(tw + (long long)k * T);
+        I[row * Ns + k] = cmul(I[(T - row) * Ns + (k ? Ns - k : 0)], make_double2(flip(w.x, true), w.y));
+    }
+    __syncthreads();
 }
 
 // A stage of any odd radix p >= 7 (a prime factor of n + 1), as a direct
@@ -613,11 +665,10 @@ __device__ __forceinline__ void fft_stage(const double2* __restrict__ in, double
 // stage's twiddles); then one thread forms one output pair of one butterfly,
 // 4 FP64 FMAs per q. The pass is bound by the FP64 pipe (2 FMA a clock and
 // SM), not by the shared-memory reads of t and d.
-// FIRST (Ns = 1, the input still the odd extension z_{L-m} = -z_m): butterfly
-// T - j holds minus the reversed inputs of butterfly j, so its outputs are
-// -e^{2 pi i r/p} y_{p-r}: half of the butterflies need no sums.
-// Measured: 4 x 256^2 (n + 1 = 3 5 17) 28 us a pass (dense float32-style tile
-// 300 us), one 512^2 field (7 73) 110 us a solve, 291 us with dense products.
+// FIRST (Ns = 1): butterflies j <= T/2 alone. A later one works on whole columns
+// (fft_expand before it).
+// Measured: 4 x 256^2 (n + 1 = 3 5 17) 19.0 us a pass (dense float32-style tile
+// 300 us), one 512^2 field (7 73) 105 us a solve, 291 us with dense products.
 template <bool FIRST>
 __device__ __forceinline__ void fft_stage_odd(double2* __restrict__ in, double2* __restrict__ out,
                                               const double2* __restrict__ tw, int L, int Ns, int pp, int p)
@@ -665,13 +716,6 @@ __device__ __forceinline__ void fft_stage_odd(double2* __restrict__ in, double2*
         if (FIRST) {
             O[j * p + r] = yr;
             if (r) O[j * p + p - r] = yp;
-            if (j > 0 && j < T / 2) {
-                const double2 w = __ldg(tw + r * T);            // e^{-2 pi i r/p}
-                const double2 a = cmul(yp, make_double2(w.x, -w.y)), b = cmul(yr, w);
-                double2* M = O + (T - j) * p;
-                M[r] = make_double2(-a.x, -a.y);
-                if (r) M[p - r] = make_double2(-b.x, -b.y);
-            }
         } else {
             const int k = j % Ns;
             const int base = (j / Ns) * Ns * p + k;
@@ -733,7 +777,10 @@ dst_fft_kernel(FftGeom g, const double2* __restrict__ tw, const double* __restri
             case 5: fft_stage<5>(b0, b1, tw, L, Ns, g.pp); break;
             default:
                 if (Ns == 1) fft_stage_odd<true>(b0, b1, tw, L, Ns, g.pp, R);
-                else fft_stage_odd<false>(b0, b1, tw, L, Ns, g.pp, R);
+                else {
+                    fft_expand(b0, tw, L, Ns, g.pp);
+                    fft_stage_odd<false>(b0, b1, tw, L, Ns, g.pp, R);
+                }
                 break;
         }
         __syncthreads();
@@ -799,7 +846,9 @@ static int upload(const std::vector<double>& h, void** d)
 // Lengths that factor into 2, 3, 5 always take the FFT. Measured solves, FFT /
 // dense: n + 1 = 63 27 / 24 us, 127 50 / 34, 159 37 / 42, 191 (7 fields) 283 /
 // 140, 255 (4 fields) 69 / 152, 447 156 / 194, 1023 279 / 1839; the rule picks
-// the faster one of each.
+// the faster one of each. (These are with whole small stages, as the costs below
+// count them: half stages take 52 us at 255 and 248 at 1023, and halving the costs
+// would move only lengths of n <= 73, where launches are most of either time.)
 static bool fft_factor(int L, std::vector<int>& rad)
 {
     rad.clear();

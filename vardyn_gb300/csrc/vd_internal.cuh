@@ -76,6 +76,7 @@ struct DSTTables {
     void* Weven;  // [kpad][ldw]  Weven[p][t] = c sin(pi (p+1)(2t+2)/(n+1)) (symmetric)
     void* trim;   // [my][lds] Thomas multipliers m_j per spectral column
     double tri_a; // off-diagonal g/f/dy^2
+    void* tri_tab = nullptr;   // float64: [4][my][lds] multipliers, alphas and their products within a piece
     void* tc;     // tensor-core images and tile table (float32 plans), or nullptr
     // float64 plans whose odd extension 2(n+1) factors into 2, 3, 5: the
     // FFT form of the transform (twiddles e^{-2 pi i m / L}, radix per stage)

@@ -216,25 +216,29 @@ dst_gemm_kernel(GemmGeom g, const T* __restrict__ W1, const T* __restrict__ W2,
 // operands are read straight from L1 / L2 (one W load per R FMAs), and the work
 // is cut finely enough to fill all 608 schedulers even for one 128^2 field.
 // A warp owns 32 output columns of one half (even-k or odd-k sums) of R rows;
-// a CTA's 8 warps are both halves x CWC column groups x 4/CWC row groups over
-// the butterflied rows in shared memory. Measured on one 128^2 field: the whole
-// solve 34 us, against 340 us with the 8 x 8 register tile of the float32 kernel
-// (8 CTAs of two warps a pass); 119 us on one 384^2 field.
-template <int R, int CWC, int MODE, int EPI>
-__global__ void __launch_bounds__(256)
+// a CTA's warps are both halves x CWC column groups x RG row groups over the
+// butterflied rows in shared memory. PF (one row a warp): the next 8 entries of W are
+// loaded while the last 8 are used; with a warp or two on a scheduler nothing else
+// covers an L2 load.
+// Measured on one 128^2 field: a pass 6.3 us forward and 6.6 us inverse (8.0 and 13.2
+// without the prefetch and with CTAs of two rows on 63 SMs); the whole solve 340 us with
+// the 8 x 8 register tile of the float32 kernel (8 CTAs of two warps a pass); 119 us on
+// one 384^2 field.
+template <int R, int CWC, int RG, bool PF, int MODE, int EPI>
+__global__ void __launch_bounds__(64 * CWC * RG)
 dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __restrict__ W2,
                    const double* __restrict__ src, const double* __restrict__ sub, int sub_batches,
                    double* __restrict__ spec, double* __restrict__ out, const double* __restrict__ add,
                    int add_batches, const int8_t* __restrict__ mask)
 {
-    constexpr int RG = 4 / CWC, TR = R * RG, NC = 32 * CWC;
+    constexpr int TR = R * RG, NC = 32 * CWC, NW = CWC * RG, NT = 64 * NW;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* As = reinterpret_cast<double*>(smem_raw);    // [ne][TR]
     double* Bs = As + (size_t)g.ne * TR;                 // [no][TR]
     const int n = g.n, ne = g.ne, no = g.no, my = g.my;
     const int row0 = blockIdx.y * TR, c0 = blockIdx.x * NC;
 
-    for (int idx = threadIdx.x; idx < ne * TR; idx += 256) {
+    for (int idx = threadIdx.x; idx < ne * TR; idx += NT) {
         const int r = idx / ne, p = idx - r * ne;
         const int row = row0 + r;
         double a = 0.0, b = 0.0;
@@ -263,7 +267,7 @@ dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __re
     __syncthreads();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int half = warp >> 2, cw = (warp & 3) % CWC, rg = (warp & 3) / CWC;
+    const int half = warp / NW, wi = warp % NW, cw = wi % CWC, rg = wi / CWC;
     const int t = c0 + cw * 32 + lane;                   // < ldw: the tables' rows are zero-padded
     const int K = half == 0 ? ne : no;
     const double* __restrict__ W = (half == 0 ? W1 : W2) + t;
@@ -271,11 +275,51 @@ dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __re
     double acc[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < K; ++k) {
-        const double w = __ldg(W + (size_t)k * g.ldw);
+    if constexpr (PF) {
+        static_assert(R == 1, "one row a warp");
+        double wc[8], wn[8];
 #pragma unroll
-        for (int i = 0; i < R; ++i) acc[i] = fma(X[k * TR + i], w, acc[i]);
+        for (int u = 0; u < 8; ++u) wc[u] = u < K ? __ldg(W + (size_t)u * g.ldw) : 0.0;
+        for (int k0 = 0; k0 < K; k0 += 8) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) wn[u] = k0 + 8 + u < K ? __ldg(W + (size_t)(k0 + 8 + u) * g.ldw) : 0.0;
+            if (k0 + 8 <= K) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    acc[0] = fma(X[(k0 + u) * TR], wc[u], acc[0]);
+            } else {
+                // the last K % 8 as 4 + 2 + 1 (a predicated-off FMA would take its slot)
+                int k = k0;
+                const int rem = K - k0;
+                if (rem & 4) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        acc[0] = fma(X[(k + u) * TR], wc[u], acc[0]);
+                        wc[u] = wc[u + 4];
+                    }
+                    k += 4;
+                }
+                if (rem & 2) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        acc[0] = fma(X[(k + u) * TR], wc[u], acc[0]);
+                        wc[u] = wc[u + 2];
+                    }
+                    k += 2;
+                }
+                if (rem & 1) acc[0] = fma(X[k * TR], wc[0], acc[0]);
+                break;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) wc[u] = wn[u];
+        }
+    } else {
+#pragma unroll 8
+        for (int k = 0; k < K; ++k) {
+            const double w = __ldg(W + (size_t)k * g.ldw);
+#pragma unroll
+            for (int i = 0; i < R; ++i) acc[i] = fma(X[k * TR + i], w, acc[i]);
+        }
     }
 
     if (MODE == MODE_FWD) {
@@ -288,10 +332,10 @@ dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __re
         }
     } else {
         // y[p] = A + B, y[n-1-p] = A - B: the odd-half warps hand over B
-        __shared__ double ex[4][R][32];
+        __shared__ double ex[NW][R][32];
         if (half == 1) {
 #pragma unroll
-            for (int i = 0; i < R; ++i) ex[warp & 3][i][lane] = acc[i];
+            for (int i = 0; i < R; ++i) ex[wi][i][lane] = acc[i];
         }
         __syncthreads();
         if (half == 0 && t < ne) {
@@ -301,7 +345,7 @@ dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __re
                 if (row >= g.R) break;
                 const int f = row / my, j = row - f * my + 1;
                 const long long base = f * g.fs + (long long)j * g.nx + 1;
-                const double B = t < no ? ex[warp][i][lane] : 0.0;
+                const double B = t < no ? ex[wi][i][lane] : 0.0;
                 const double ys[2] = {acc[i] + B, acc[i] - B};
                 const int ps[2] = {t, n - 1 - t};
 #pragma unroll
@@ -1120,16 +1164,16 @@ static cudaError_t set_smem_attrs()
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, maxb);
 }
 
-template <int R, int CWC>
+template <int R, int CWC, int RG = 4 / CWC, bool PF = false>
 static cudaError_t set_smem_dense64()
 {
     const int maxb = 200 * 1024;   // plus the exchange tile in static shared memory
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, MODE_FWD, EPI_H>,
+    if ((e = cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, RG, PF, MODE_FWD, EPI_H>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, maxb))) return e;
-    if ((e = cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, MODE_INV, EPI_H>,
+    if ((e = cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, RG, PF, MODE_INV, EPI_H>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, maxb))) return e;
-    return cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, MODE_INV, EPI_ADJQ>,
+    return cudaFuncSetAttribute(dst_dense64_kernel<R, CWC, RG, PF, MODE_INV, EPI_ADJQ>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, maxb);
 }
 
@@ -1191,6 +1235,8 @@ static cudaError_t configure_kernels()
         if (!e) e = set_smem_attrs<float, 32>();
         if (!e) e = set_smem_attrs<float, 64>();
         if (!e) e = set_smem_dense64<1, 2>();
+        if (!e) e = set_smem_dense64<1, 2, 2, true>();
+        if (!e) e = set_smem_dense64<1, 2, 1, true>();
         if (!e) e = set_smem_dense64<2, 2>();
         if (!e) e = set_smem_dense64<4, 2>();
         if (!e) e = set_smem_dense64<2, 4>();
@@ -1231,26 +1277,44 @@ static int launch_pair(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs
     return VD_OK;
 }
 
-template <int R, int CWC>
-static int launch_dense64_rc(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs& a, double* spec,
+template <int R, int CWC, int RG, bool PF>
+static int launch_dense64_rg(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs& a, double* spec,
                              cudaStream_t st, bool fwd)
 {
     const DSTTables& t = p->dst;
-    constexpr int TR = R * (4 / CWC), NC = 32 * CWC;
+    constexpr int TR = R * RG, NC = 32 * CWC, NT = 64 * CWC * RG;
     const size_t smem = (size_t)t.n * TR * sizeof(double);
     const dim3 grid((t.ne + NC - 1) / NC, (g.R + TR - 1) / TR);
     const double *Wo = (const double*)t.Wodd, *WoT = (const double*)t.WoddT, *We = (const double*)t.Weven;
     if (fwd)
-        dst_dense64_kernel<R, CWC, MODE_FWD, EPI_H><<<grid, 256, smem, st>>>(
+        dst_dense64_kernel<R, CWC, RG, PF, MODE_FWD, EPI_H><<<grid, NT, smem, st>>>(
             g, Wo, We, (const double*)a.src, (const double*)a.sub, a.sub_batches, spec, nullptr, nullptr, 0, nullptr);
     else if (a.epi == EPI_H)
-        dst_dense64_kernel<R, CWC, MODE_INV, EPI_H><<<grid, 256, smem, st>>>(
+        dst_dense64_kernel<R, CWC, RG, PF, MODE_INV, EPI_H><<<grid, NT, smem, st>>>(
             g, WoT, We, nullptr, nullptr, 0, spec, (double*)a.out, (const double*)a.add, a.add_batches, p->d_mask);
     else
-        dst_dense64_kernel<R, CWC, MODE_INV, EPI_ADJQ><<<grid, 256, smem, st>>>(
+        dst_dense64_kernel<R, CWC, RG, PF, MODE_INV, EPI_ADJQ><<<grid, NT, smem, st>>>(
             g, WoT, We, nullptr, nullptr, 0, spec, (double*)a.out, (const double*)a.add, a.add_batches, p->d_mask);
     VD_LAUNCH_CHECK();
     return VD_OK;
+}
+
+// Row groups a CTA: 4 / CWC (8 warps), or one where that leaves SMs without a CTA and
+// twice the CTAs still fit one wave (a scheduler's time is its warps' FMAs). W is
+// prefetched up to four warps a scheduler: solves of one 126, 190, 222 and 382-mode
+// field with / without: 18.4 / 27.0 us (and one row a CTA), 36.5 / 40.7, 41.2 / 46.1 and
+// 116.3 / 115.1.
+template <int R, int CWC>
+static int launch_dense64_rc(const vd_qg1l_plan* p, const GemmGeom& g, const SolveArgs& a, double* spec,
+                             cudaStream_t st, bool fwd)
+{
+    if constexpr (R == 1) {
+        const long long ctas = (long long)((p->dst.ne + 32 * CWC - 1) / (32 * CWC)) * g.R;   // at one row a CTA
+        if (ctas <= 152) return launch_dense64_rg<R, CWC, 1, true>(p, g, a, spec, st, fwd);
+        if (2LL * ((p->dst.ne + 31) / 32) * g.R <= 4 * 608)
+            return launch_dense64_rg<R, CWC, 4 / CWC, true>(p, g, a, spec, st, fwd);
+    }
+    return launch_dense64_rg<R, CWC, 4 / CWC, false>(p, g, a, spec, st, fwd);
 }
 
 // Rows a warp: as many as leave about four warps to each of the 608 schedulers

@@ -1390,6 +1390,19 @@ static int pick_tr(const vd_qg1l_plan* p, int R)
     return 16;
 }
 
+// Whether a length with an FFT takes the dense form all the same: the rows are so few
+// that it runs as one wave of one-row CTAs, a warp a scheduler, and a half sum of up to
+// 120 FMAs is shorter than the FFT's chain of stages and barriers. Solves of one field,
+// dense / FFT: 40 x 46 11.7 / 21.0 us, 64^2 + 1 13.0 / 20.3, 96^2 16.2 / 23.5, 128^2 + 1
+// 18.4 / 22.9, 52 x 193 22.1 / 24.1, 40 x 241 25.0 / 26.1, 40 x 257 26.0 / 24.9, 24 x 385
+// 34.4 / 28.4.
+static bool dense64_few(const vd_qg1l_plan* p, const GemmGeom& g)
+{
+    if (p->dst.ne > 120) return false;
+    const int cols = (p->dst.ne + 31) / 32, cwc = cols == 1 ? 1 : 2;
+    return (long long)((cols + cwc - 1) / cwc) * g.R <= 152;
+}
+
 // One x-direction pass: float32 on the tensor cores or CUDA-core FMA, float64
 // as FFT or dense products.
 template <typename T>
@@ -1403,7 +1416,7 @@ static int dst_pass(const vd_qg1l_plan* p, int nf, const GemmGeom& g, const Solv
         if (tr == 32) return launch_pair<T, 32>(p, g, a, spec, st, fwd);
         return launch_pair<T, 16>(p, g, a, spec, st, fwd);
     } else {
-        if (p->dst.fft_L) return launch_fft(p, g, a, spec, st, fwd);
+        if (p->dst.fft_L && !dense64_few(p, g)) return launch_fft(p, g, a, spec, st, fwd);
         return launch_dense64(p, g, a, spec, st, fwd);
     }
 }

@@ -266,11 +266,15 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
       stage (forward RK stage, k_stage_fwd)     reads h_s, q_s, q_n, writes q: 4F
       adj-stage (k_adj_stage_fused), s = 1      reads h_s, q_s, G_0, writes adq, adh: 5F
       adj-stage, s = 0 (with the accumulations) reads h_s, q_s, G_1, G_0, G_1: 7F
-      dst-fwd (dst_tc_kernel<0,0>)               reads the field, writes spectra: 2F
-      tridiag (tridiag_chunked_kernel)           spectra in place: 2F
-      dst-inv (dst_tc_kernel<1,0>)               spectra -> SSH: 2F
-      dst-inv-adj (dst_tc_kernel<1,1>)           spectra + addend -> masked PV adjoint: 3F
+      dst-fwd-solve (dst_tc_fwd_kernel)          reads the field, writes solved spectra: 2F
+                                                (the tridiagonal solve runs in its epilogue;
+                                                timed as the inversion, less the inverse pass
+                                                and the step output that vd_qg1l_pv2h adds)
+      dst-inv (dst_tc_inv_kernel)                spectra -> SSH: 2F
+      dst-inv-adj (dst_tc_inv_kernel)            spectra + addend -> masked PV adjoint: 3F
 
+    With the CUDA-core engine dst-fwd (dst_gemm_kernel) and tridiag
+    (tridiag_chunked_kernel, spectra in place: 2F) are launches of their own.
     Per RK2 step of an evaluation with the stored trajectory: 2 stages,
     4 forward / 2 inverse / 2 inverse-adjoint passes, 4 tridiagonal solves
     and the two adjoint stages; ``recompute`` (checkpointed forms) runs the
@@ -292,7 +296,8 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
     _lib.call("vd_qg1l_dst_x", plan.handle, B, P(q), P(spec), 0, None, st())
     # names of the x-DST kernels under the plan's schedule (tensor cores or FMA)
     tc = plan.dtype == torch.float32 and plan.dst_engine == "auto" and plan.schedule()["engine"] != 1
-    dname = (lambda m, e: f"dst_tc_kernel<{m},{e}>") if tc else (lambda m, e: "dst_gemm_kernel")   # noqa: E731
+    dname = (lambda m, e: f"dst_tc_{'inv' if m else 'fwd'}_kernel<{e}>") if tc else (lambda m, e: "dst_gemm_kernel")   # noqa: E731
+    ws = plan.workspace(B)
     calls = {
         "stage": (lambda: _lib.call("vd_qg1l_rk_stage", plan.handle, B, P(h), P(q), P(q0), 0, vp([]), dp([]),
                                     DT, None, P(out1), st()), 2 * nstep, 4, "k_stage_fwd"),
@@ -306,16 +311,18 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
                     dname(0, 0)),
         "tridiag": (lambda: _lib.call("vd_qg1l_tridiag_y", plan.handle, B, P(spec), st()), 4 * nstep, 2,
                     "tridiag_chunked_kernel"),
+        "dst-fwd-solve": (lambda: _lib.call("vd_qg1l_pv2h", plan.handle, B, P(q), None, None, P(out1), P(ws),
+                                            ws.numel(), st()), 4 * nstep, 2, dname(0, 0)),
         "dst-inv": (lambda: _lib.call("vd_qg1l_dst_x", plan.handle, B, None, P(spec), 1, P(out1), st()),
                     2 * nstep, 2, dname(1, 0)),
         "dst-inv-adj": (lambda: _lib.call("vd_qg1l_dst_x", plan.handle, B, P(q0), P(spec), 2, P(out1), st()),
                         2 * nstep, 3, dname(1, 1)),
     }
-    rows = []
-    fwd_extra = {"stage": 2 * nstep, "dst-fwd": 2 * nstep, "tridiag": 2 * nstep, "dst-inv": 2 * nstep}
-    for name, (fn, per_eval, nF, kern) in calls.items():
-        if recompute:
-            per_eval += fwd_extra.get(name, 0)
+
+    def output():
+        _lib.call("vd_qg1l_finalize", plan.handle, B, P(out1), None, None, 0.0, P(out1), st())
+
+    def timed(fn):
         for _ in range(5):
             fn()
         torch.cuda.synchronize()
@@ -325,9 +332,24 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
             fn()
         e1.record()
         torch.cuda.synchronize()
-        us = e0.elapsed_time(e1) / reps * 1e3
+        return e0.elapsed_time(e1) / reps * 1e3
+
+    for name in (("dst-fwd", "tridiag") if tc else ("dst-fwd-solve",)):
+        del calls[name]
+    rows = []
+    fwd_extra = {"stage": 2 * nstep, "dst-fwd": 2 * nstep, "tridiag": 2 * nstep, "dst-fwd-solve": 2 * nstep,
+                 "dst-inv": 2 * nstep}
+    for name, (fn, per_eval, nF, kern) in calls.items():
+        if recompute:
+            per_eval += fwd_extra.get(name, 0)
+        us = timed(fn)
         rows.append({"name": name, "kernel": kern, "us": us, "launches_per_eval": per_eval,
                      "algorithmic_bytes": nF * F, "gbs": nF * F / (us * 1e-6) / 1e9})
+    if tc:   # the inversion is the fused forward pass, the inverse pass and the step output
+        r = {x["name"]: x for x in rows}
+        f = r["dst-fwd-solve"]
+        f["us"] = max(f["us"] - r["dst-inv"]["us"] - timed(output), 1e-3)
+        f["gbs"] = f["algorithmic_bytes"] / (f["us"] * 1e-6) / 1e9
     return rows
 
 

@@ -96,7 +96,8 @@ typedef struct vd_qg1l_schedule {
                             their own rule) */
     int tridiag_rows;    /* rows per thread of the separate tridiagonal
                             solve: 0 rule, 8, 16 or 32 (used when the field
-                            fits, else the rule) */
+                            fits, else the rule); float64 fields of up to 512
+                            interior rows run the form with tables at 0 and 8 */
     int tridiag_lean;    /* 1: the float32 16-row tridiagonal kernel capped at
                             80 registers (three CTAs per SM instead of two);
                             0 the standard kernel */

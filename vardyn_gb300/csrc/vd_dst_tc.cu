@@ -15,6 +15,10 @@
 // The K loop of the largest shape (128 rows, two groups) is bound by the SM's
 // shared-memory port: a chunk's 24 MMAs read 8 KB of operands each, its rows and
 // matrix add 96 KB of writes, 292 KB at 128 bytes a clock = 1.15 us, as measured.
+// Every CTA reads its own matrix chunks (64 KB of them at most, from L2); handing a
+// cluster's CTAs one shared copy took as long or longer (an inverse pass 20.0 us
+// without it and 20.7 with it at 16 x 512^2, 17.0 and 17.8 at 1024^2, 10.8 and 11.3
+// at 6 x 287x410; the fused forward pass within 1 %).
 // Measured inversions (the row-major form with a separate solve in brackets, us): 16 x 512^2 52 (64),
 // 1024^2 43 (54), 6 x 287x410 27 (62), 12 x 192^2 18 (28), 128^2 15 (24).
 // A CTA holds MG = 1 or 2 groups of 128 modes (positions) of one parity of the
@@ -130,29 +134,12 @@ __device__ __forceinline__ uint32_t cluster_rank()
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ uint32_t cluster_size()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
 {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
-// The same copy into every CTA of `mask`, at the same offsets of their shared
-// memory and barriers.
-__device__ __forceinline__ void bulk_g2s_mc(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar,
-                                            uint16_t mask)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster "
-                 "[%0], [%1], %2, [%3], %4;"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "h"(mask)
                  : "memory");
 }
 
@@ -195,14 +182,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t adesc, uint64_
 __device__ __forceinline__ void mma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-// The same arrival on the barrier at this offset in every CTA of `mask`.
-__device__ __forceinline__ void mma_commit_mc(uint32_t bar, uint16_t mask)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(mask)
                  : "memory");
 }
 
@@ -374,23 +353,6 @@ struct TcLoop {
     using Sh = TcShape<RPW, MG>;
     uint32_t sbase, bar0, tmem;
     int stages, kch;
-    // The CTAs of the cluster that take the same matrix rows (mask, count) each
-    // load one slice of every chunk and multicast it to the others, so a stage is
-    // free once all of them have multiplied it. Without it, 128 CTAs each read
-    // the whole 512 KB matrix half: the K loop ran at the L2's bandwidth.
-    uint16_t mask;
-    int share;                       // CTAs in mask
-    uint32_t sl_off, sl_bytes;       // this CTA's slice of a chunk's hi (and lo) part
-
-    __device__ __forceinline__ void set_share(uint16_t m, int count, int index, int wrows)
-    {
-        mask = m;
-        share = count;
-        const int per = (((wrows + 7) / 8 + count - 1) / count) * 8;     // matrix rows a slice, 8 at a time
-        const int r0 = min(wrows, index * per);
-        sl_off = (uint32_t)r0 * KCH * 4;
-        sl_bytes = (uint32_t)(min(wrows, r0 + per) - r0) * KCH * 4;
-    }
 
     __device__ __forceinline__ uint32_t rows_hi(int s) const { return sbase + s * Sh::STAGE; }
     __device__ __forceinline__ uint32_t mat_hi(int s) const { return rows_hi(s) + 2 * Sh::ROWS; }
@@ -404,7 +366,7 @@ struct TcLoop {
         for (int s = 0; s < stages; ++s) {
             mbar_init(full_a(s), NPROD);
             mbar_init(full_b(s), 1);
-            mbar_init(empty(s), share);
+            mbar_init(empty(s), 1);
         }
         mbar_init(accf(), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -473,15 +435,9 @@ struct TcLoop {
             if (c >= stages) mbar_wait(empty(s), (u - 1) & 1, 1);
             if (tid == 0) {
                 mbar_arrive_expect_tx(full_b(s), 2 * b_bytes);
-                const float* blk = img + (size_t)c * 2 * ntot * KCH + sl_off / 4;
-                const uint32_t dst = mat_hi(s) + sl_off;
-                if (share == 1) {
-                    bulk_g2s(dst, blk, sl_bytes, full_b(s));
-                    bulk_g2s(dst + Sh::MAT, blk + (size_t)ntot * KCH, sl_bytes, full_b(s));
-                } else if (sl_bytes) {
-                    bulk_g2s_mc(dst, blk, sl_bytes, full_b(s), mask);
-                    bulk_g2s_mc(dst + Sh::MAT, blk + (size_t)ntot * KCH, sl_bytes, full_b(s), mask);
-                }
+                const float* blk = img + (size_t)c * 2 * ntot * KCH;
+                bulk_g2s(mat_hi(s), blk, b_bytes, full_b(s));
+                bulk_g2s(mat_hi(s) + Sh::MAT, blk + (size_t)ntot * KCH, b_bytes, full_b(s));
             }
             const uint32_t ah = rows_hi(s), al = ah + Sh::ROWS;
 #pragma unroll
@@ -500,7 +456,6 @@ struct TcLoop {
 #pragma unroll
         for (int d = 0; d < DEPTH; ++d)
             if (d < kch) load(d, x1[d], x2[d]);
-        cluster_wait();                  // every CTA's barriers exist (the arrive follows their initialisation)
         for (int c0 = 0; c0 < kch; c0 += DEPTH) {
 #pragma unroll
             for (int d = 0; d < DEPTH; ++d) {
@@ -540,10 +495,7 @@ struct TcLoop {
                 }
             }
             // nobody waits for the last use of a stage
-            if (c + stages < kch) {
-                if (share == 1) mma_commit(empty(s));
-                else mma_commit_mc(empty(s), mask);
-            }
+            if (c + stages < kch) mma_commit(empty(s));
             if (++s == stages) {
                 s = 0;
                 ++u;
@@ -592,10 +544,9 @@ dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
         tmem_alloc(smem_u32(&tmem_base_sh), COLS);
         tmem_relinquish();
     }
-    L.set_share((uint16_t)((1u << (FUSE ? g.nr : 1)) - 1), FUSE ? g.nr : 1, FUSE ? rb : 0, wrows);
     if (tid == 0) L.init_barriers();
     __syncwarp();
-    cluster_arrive();
+    if constexpr (FUSE) cluster_arrive();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -650,9 +601,8 @@ dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
         ok = mbar_wait(L.accf(), 0, 4);
         __syncwarp();
         tc_fence_after();
-    } else {
-        cluster_wait();
-        if (lane == 0) L.issue((wrows + GM - 1) / GM);
+    } else if (lane == 0) {
+        L.issue((wrows + GM - 1) / GM);
     }
     __syncwarp();
 
@@ -685,6 +635,7 @@ dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
         };
         const uint32_t mcol = tcol + TMEM_COLS;
         float d = 0.f, P = 1.f;
+        cluster_wait();                  // every CTA of the cluster has started: its shared memory can be written
         if (warp < NPW) {
 #pragma unroll
             for (int b = 0; b < PC; b += NB) {
@@ -758,9 +709,9 @@ dst_tc_fwd_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
     }
 }
 
-// Inverse pass. Grid: x = fields x row blocks x 2 jobs (pairs of cluster ranks:
-// the even one the odd-k half A of the spectrum, the odd one the even-k half B;
-// two row blocks a cluster, to share the matrix), y = groups of MG * 128 positions. x[p] = A + B and x[n-1-p] = A - B: the A CTA writes the
+// Inverse pass. Grid: x = fields x row blocks x 2 jobs (a cluster of two CTAs:
+// rank 0 the odd-k half A of the spectrum, rank 1 the even-k half B), y = groups
+// of MG * 128 positions. x[p] = A + B and x[n-1-p] = A - B: the A CTA writes the
 // first half of the block's rows, the B CTA the second, each after receiving the
 // other's sums of those rows in its (free) pipeline stages. Rows go through
 // shared memory once more so that they leave as aligned float4s: the interior
@@ -794,14 +745,8 @@ dst_tc_inv_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
         tmem_alloc(smem_u32(&tmem_base_sh), TMEM_COLS);
         tmem_relinquish();
     }
-    // cluster ranks 2 r + job: the CTAs of one job share the matrix
-    const int share = (int)cluster_size() / 2;
-    uint16_t same = 0;
-    for (int r = 0; r < share; ++r) same |= (uint16_t)(1u << (2 * r + job));
-    L.set_share(same, share, (int)(blk % share), wrows);
     if (tid == 0) L.init_barriers();
     __syncwarp();
-    cluster_arrive();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -813,7 +758,6 @@ dst_tc_inv_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
     const int pl = grp * GM + sp * 32 + lane;      // position p_first + pl
     bool ok = true;
     if (warp < NPW) {
-        // (a block behind the last row only pads its cluster)
         const int r0 = blk * RB + warp * RPW, nv = min(RPW, g.rows - r0);
         const unsigned first = (unsigned)(r0 * g.lds + (job == 0 ? 0 : g.ne)), pitch = (unsigned)g.lds;
         L.produce(spec, nullptr, [&](int i) { return first + i * pitch; }, [](int) { return false; }, nv, g.n,
@@ -823,9 +767,8 @@ dst_tc_inv_kernel(TcGeom g, TcTab tab, const float* __restrict__ img, const floa
         ok = mbar_wait(L.accf(), 0, 4);
         __syncwarp();
         tc_fence_after();
-    } else {
-        cluster_wait();
-        if (lane == 0) L.issue((wrows + GM - 1) / GM);
+    } else if (lane == 0) {
+        L.issue((wrows + GM - 1) / GM);
     }
     __syncwarp();
 
@@ -1101,9 +1044,9 @@ struct TcPick { int rb, mg; double us; };
 // Rows and groups of a CTA: the shape with the least estimated time. A CTA's time
 // is a fixed part that grows with the values it stores and its K chunks, whose
 // cost grows with the rows it splits and the products it issues (microseconds,
-// fitted to single-wave launches at 128^2 to 1024^2: a forward pass measured 17.0
-// at 16 x 512^2 with 128 rows and two groups; 16.1 at 1024^2 with 64 rows and one
-// group, 19.4 with 128 and one, 25.9 with 128 and two); clusters beyond those that
+// fitted to single-wave launches at 128^2 to 1024^2: a forward pass measured 16.7
+// at 16 x 512^2 with 128 rows and two groups; 16.0 at 1024^2 with 64 rows and one
+// group, 22.3 with 128 and one, 25.3 with 128 and two); clusters beyond those that
 // run at once take further waves. `fuse`: the blocks of a field are one cluster,
 // and the epilogue also solves.
 static TcPick tc_pick(const vd_qg1l_plan* p, int nf, bool fwd, bool fuse)
@@ -1116,7 +1059,7 @@ static TcPick tc_pick(const vd_qg1l_plan* p, int nf, bool fwd, bool fuse)
     auto cost = [&](int rb, int mg) {
         const int nr = (t.my + rb - 1) / rb, groups = (t.ne + GM * mg - 1) / (GM * mg);
         if (fuse && nr > MAX_NR) return 1e30;
-        const int csz = fuse ? nr : fwd ? 1 : 4;
+        const int csz = fuse ? nr : fwd ? 1 : 2;
         const long long blocks = fuse ? (long long)nf * nr : ((long long)nf * t.my + rb - 1) / rb;
         const long long clusters = (2LL * blocks * groups + csz - 1) / csz;
         const int at_once = std::max(1, g_tc_clusters[dev][csz]);
@@ -1142,8 +1085,8 @@ static TcPick tc_pick(const vd_qg1l_plan* p, int nf, bool fwd, bool fuse)
 // Whether the forward pass also solves the tridiagonal systems: not for fields
 // whose row blocks exceed a cluster, nor where the plain pass with its freer shape
 // and the separate solve (measured 3.5 us and 3.1 us per million points) are
-// cheaper: single tall fields (1024^2: 16 + 6 us against 25 us fused; at
-// 16 x 512^2 20 us fused against 17 + 16).
+// cheaper: single tall fields (1024^2: 16 + 6 us against 27 us fused; at
+// 16 x 512^2 22 us fused against 17 + 16).
 static bool tc_fusable(const vd_qg1l_plan* p, int nf)
 {
     const DSTTables& t = p->dst;
@@ -1207,16 +1150,14 @@ static int tc_launch_inv(const vd_qg1l_plan* p, int nf, const SolveArgs& a, cons
         TcTab tab = d->tab;
         tab.nst = (int)std::min<size_t>(MAX_STAGES, (SMEM_MAX - SMEM_STATIC - 1024) / Sh::STAGE);
         cudaLaunchConfig_t cfg = {};
-        // two row blocks a cluster (clusters of 8 fill only 120 of the SMs), padded
-        const int blocks = (g.rows + Sh::RB - 1) / Sh::RB, share = blocks > 1 ? 2 : 1;
-        cfg.gridDim = dim3(2u * (unsigned)((blocks + share - 1) / share * share), (t.ne + GM * M() - 1) / (GM * M()));
+        cfg.gridDim = dim3(2u * (unsigned)((g.rows + Sh::RB - 1) / Sh::RB), (t.ne + GM * M() - 1) / (GM * M()));
         cfg.blockDim = dim3(NTHREADS);
         cfg.dynamicSmemBytes =
             std::max(SMEM_ONE, std::max<size_t>(tab.nst * (size_t)Sh::STAGE, Sh::INV_EPI) + 1024);
         cfg.stream = st;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 2u * (unsigned)share;
+        at[0].val.clusterDim.x = 2;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;

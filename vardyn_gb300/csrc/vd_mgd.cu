@@ -446,18 +446,26 @@ k_mgd_init(MgdLev<T> A, const T* __restrict__ b, long long ldb, long long fsb, T
 }
 
 // p = z + beta p_old (p = z on the first iteration), q = -A p, p.q. p is read a
-// ring beyond the block's tile: p_old and p are different buffers.
+// ring beyond the block's tile: p_old and p are different buffers. q carries the
+// problem that the iteration solves, so it is formed from differences: with the
+// sweeps' rounded 1/D, c0/D, c1/D, D (2 c0/D + 2 c1/D) + lambda would miss D by 1e-7
+// D in float32, as much as the lowest modes' eigenvalues (511 x 767, lambda = 0: 9e-4
+// of the solution). The V-cycle, which only preconditions, keeps the quotients.
+// (7 FP64 instructions a point for 6: 1 % of a float64 solve, 5.25 -> 5.31 ms on three
+// systems of 1023 x 767.)
+// op[m] = {c0, c1, lambda_m}.
 template <typename T, int TI, int TJ>
 __global__ void __launch_bounds__(MGD_NT)
-k_mgd_pq(MgdLev<T> A, int first, const T* __restrict__ z, const T* __restrict__ pold, T* __restrict__ pnew,
-         T* __restrict__ q, MgdDot D)
+k_mgd_pq(MgdLev<T> A, const T* __restrict__ op, int first, const T* __restrict__ z, const T* __restrict__ pold,
+         T* __restrict__ pnew, T* __restrict__ q, MgdDot D)
 {
     constexpr int P = TJ + 2;
     __shared__ T ps[(TI + 2) * P];
     const int s = blockIdx.z;
     if (A.done[s]) return;
     const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
-    const T* co = A.coef + 4 * (s / A.batch);
+    op += 3 * (s / A.batch);
+    const T c0 = op[0], c1 = op[1], lam = op[2];
     const long long o0 = (long long)s * A.n0 * A.n1;
     const T be = first ? T(0) : (T)D.beta[s];
     for (int idx = threadIdx.x; idx < (TI + 2) * P; idx += MGD_NT) {
@@ -481,7 +489,7 @@ k_mgd_pq(MgdLev<T> A, int first, const T* __restrict__ z, const T* __restrict__ 
         const T pc = ps[l];
         T v = T(0);
         if (A.mask[i * A.n1 + j])
-            v = co[3] * (pc - fma(co[2], ps[l - 1] + ps[l + 1], co[1] * (ps[l - P] + ps[l + P])));
+            v = fma(-c0, fma(T(-2), pc, ps[l - P] + ps[l + P]), fma(-c1, fma(T(-2), pc, ps[l - 1] + ps[l + 1]), lam * pc));
         pnew[o] = pc;
         q[o] = v;
         acc += (double)pc * (double)v;
@@ -556,7 +564,7 @@ using namespace vd;
 struct vd_mgd_plan {
     vd_mgd_desc d;
     std::vector<MgdLevel> lv;
-    void* coef = nullptr;           // [level][nmode][4] plan dtype (MgdLev::coef)
+    void* coef = nullptr;           // [level][nmode][4] plan dtype (MgdLev::coef), then op [nmode][3] (k_mgd_pq)
     int nb = 0;                     // coarsest unknowns
     int32_t* cidx = nullptr;        // [nb]
     double* cinv = nullptr;         // [nmode][nb][nb]
@@ -644,18 +652,24 @@ extern "C" vd_status vd_mgd_plan_create(vd_mgd_plan** out, const vd_mgd_desc* d)
             return fail(VD_ERR_CUDA);
     }
     const size_t es = d->dtype == VD_F64 ? 8 : 4;
-    std::vector<char> co(es * 4 * d->nmode * nlev);
+    std::vector<char> co(es * d->nmode * (4 * (size_t)nlev + 3));
+    auto put = [&](size_t o, double v) {
+        if (es == 8) reinterpret_cast<double*>(co.data())[o] = v;
+        else reinterpret_cast<float*>(co.data())[o] = (float)v;
+    };
     for (int l = 0; l < nlev; ++l)
         for (int m = 0; m < d->nmode; ++m) {
             const double a0 = 1.0 / (d0s[l] * d0s[l]), a1 = 1.0 / (d1s[l] * d1s[l]);
             const double D = 2 * a0 + 2 * a1 + d->lambda_host[m];
             const double v[4] = {1.0 / D, a0 / D, a1 / D, D};
-            for (int k = 0; k < 4; ++k) {
-                const size_t o = 4 * ((size_t)l * d->nmode + m) + k;
-                if (es == 8) reinterpret_cast<double*>(co.data())[o] = v[k];
-                else reinterpret_cast<float*>(co.data())[o] = (float)v[k];
-            }
+            for (int k = 0; k < 4; ++k) put(4 * ((size_t)l * d->nmode + m) + k, v[k]);
         }
+    for (int m = 0; m < d->nmode; ++m) {
+        const size_t o = 4 * (size_t)nlev * d->nmode + 3 * (size_t)m;
+        put(o, 1.0 / (d->d0 * d->d0));
+        put(o + 1, 1.0 / (d->d1 * d->d1));
+        put(o + 2, d->lambda_host[m]);
+    }
     if (cudaMalloc(&p->coef, co.size()) != cudaSuccess ||
         cudaMemcpy(p->coef, co.data(), co.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(VD_ERR_CUDA);
@@ -849,6 +863,7 @@ static int mgd_solve_t(const vd_mgd_plan* p, int batch, const T* b, long long ld
     const bool s0 = small(0);
     const dim3 g0 = grid(0);
     const MgdLev<T> A0 = lev(0);
+    const T* op = (const T*)p->coef + 4 * (size_t)nlev * p->d.nmode;
     k_mgd_fill_int<<<(2 * nsys + 255) / 256, 256, 0, st>>>(2 * nsys, 0, done);
     VD_LAUNCH_CHECK();
     if (lc == nlev) {
@@ -864,8 +879,8 @@ static int mgd_solve_t(const vd_mgd_plan* p, int batch, const T* b, long long ld
     for (int it = 0; it < p->d.max_cycles; ++it) {
         // sc[2] = rho / (p . q) = -alpha
         T *pn = cp[it & 1], *po = cp[1 - (it & 1)];
-        if (s0) k_mgd_pq<T, MGD_SI, MGD_SJ><<<g0, MGD_NT, 0, st>>>(A0, it == 0, cz, po, pn, cq, dot(2));
-        else k_mgd_pq<T, MGD_TI, MGD_TJ><<<g0, MGD_NT, 0, st>>>(A0, it == 0, cz, po, pn, cq, dot(2));
+        if (s0) k_mgd_pq<T, MGD_SI, MGD_SJ><<<g0, MGD_NT, 0, st>>>(A0, op, it == 0, cz, po, pn, cq, dot(2));
+        else k_mgd_pq<T, MGD_TI, MGD_TJ><<<g0, MGD_NT, 0, st>>>(A0, op, it == 0, cz, po, pn, cq, dot(2));
         VD_LAUNCH_CHECK();
         if (s0) k_mgd_xr<T, MGD_SI, MGD_SJ><<<g0, MGD_NT, 0, st>>>(A0, pn, cq, u, ldu, fsu, cr, dot(3));
         else k_mgd_xr<T, MGD_TI, MGD_TJ><<<g0, MGD_NT, 0, st>>>(A0, pn, cq, u, ldu, fsu, cr, dot(3));

@@ -236,7 +236,8 @@ dst_dense64_kernel(GemmGeom g, const double* __restrict__ W1, const double* __re
     double* As = reinterpret_cast<double*>(smem_raw);    // [ne][TR]
     double* Bs = As + (size_t)g.ne * TR;                 // [no][TR]
     const int n = g.n, ne = g.ne, no = g.no, my = g.my;
-    const int row0 = blockIdx.y * TR, c0 = blockIdx.x * NC;
+    const int cg = (ne + NC - 1) / NC;                   // column groups: the CTAs of the same rows follow one another
+    const int row0 = (int)(blockIdx.x / (unsigned)cg) * TR, c0 = (int)(blockIdx.x % (unsigned)cg) * NC;
 
     for (int idx = threadIdx.x; idx < ne * TR; idx += NT) {
         const int r = idx / ne, p = idx - r * ne;
@@ -1284,7 +1285,8 @@ static int launch_dense64_rg(const vd_qg1l_plan* p, const GemmGeom& g, const Sol
     const DSTTables& t = p->dst;
     constexpr int TR = R * RG, NC = 32 * CWC, NT = 64 * CWC * RG;
     const size_t smem = (size_t)t.n * TR * sizeof(double);
-    const dim3 grid((t.ne + NC - 1) / NC, (g.R + TR - 1) / TR);
+    // one dimension: the row tiles of a large batch exceed the 65535 blocks of y and z
+    const dim3 grid((unsigned)((t.ne + NC - 1) / NC) * (unsigned)((g.R + TR - 1) / TR));
     const double *Wo = (const double*)t.Wodd, *WoT = (const double*)t.WoddT, *We = (const double*)t.Weven;
     if (fwd)
         dst_dense64_kernel<R, CWC, RG, PF, MODE_FWD, EPI_H><<<grid, NT, smem, st>>>(

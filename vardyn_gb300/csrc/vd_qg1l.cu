@@ -706,7 +706,14 @@ k_adj_stage_fused(QGGeom G, int nf, const T* __restrict__ hs, const T* __restric
     T lkv[NAL][2], bev[NAL][2];
     bool m3a[NAL][2];
     constexpr bool ORD = PLAIN && sizeof(T) == 8;
-    uint32_t big = 0;   // ORD: largest magnitude of the staged SSH, PV and stage adjoint
+    // ORD: largest magnitude of the staged PV, of the SSH off the wall ring and of the
+    // stage adjoint at tendency points (the ring's SSH and the other points' adjoint are
+    // never written and must not choose the form, whose rounding differs)
+    uint32_t big = 0;
+    auto off_ring = [&](int e) {                     // element of the SSH tile
+        const int a = e / AH_X, j = j0 - 3 + a, i = i0 - 4 + (e - a * AH_X);
+        return j >= 1 && j <= G.ny - 2 && i >= 1 && i <= G.nx - 2;
+    };
     if constexpr (TMA) {
         // ---- bulk tensor copies of every staged tile, one mbarrier ----
         const uint32_t sb = (uint32_t)__cvta_generic_to_shared(smem_raw);
@@ -743,7 +750,7 @@ k_adj_stage_fused(QGGeom G, int nf, const T* __restrict__ hs, const T* __restric
             static_assert(AH_X == AQ_X, "one loop over both tiles");
             for (int e = tid; e < AQ_Y * AQ_X; e += 256) {
                 big = max(big, mag((&S.q[0][0])[e]));
-                if (e < AH_Y * AH_X) big = max(big, mag((&S.h[0][0])[e]));
+                if (e < AH_Y * AH_X && off_ring(e)) big = max(big, mag((&S.h[0][0])[e]));
             }
         }
         const int8_t* mk = reinterpret_cast<const int8_t*>(smem_raw + L.mask);
@@ -790,7 +797,9 @@ k_adj_stage_fused(QGGeom G, int nf, const T* __restrict__ hs, const T* __restric
         for (int k = 0; k < NHL; ++k) {
             const int e = tid + 256 * k;
             if (e < AH_Y * AH_X) (&S.h[0][0])[e] = hv[k];
-            if constexpr (ORD) big = max(big, mag(hv[k]));
+            if constexpr (ORD) {
+                if (off_ring(e)) big = max(big, mag(hv[k]));
+            }
         }
 #pragma unroll
         for (int k = 0; k < NQL; ++k) {
@@ -834,7 +843,8 @@ k_adj_stage_fused(QGGeom G, int nf, const T* __restrict__ hs, const T* __restric
 #pragma unroll
         for (int k = 0; k < NAL; ++k)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) big = max(big, mag(lkv[k][u]));
+            for (int u = 0; u < 2; ++u)
+                if (m3a[k][u]) big = max(big, mag(lkv[k][u]));
         ordinary = __syncthreads_and(moderate(big) && moderate_consts(G));
     } else {
         __syncthreads();

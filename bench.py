@@ -268,13 +268,17 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
       adj-stage, s = 0 (with the accumulations) reads h_s, q_s, G_1, G_0, G_1: 7F
       dst-fwd-solve (dst_tc_fwd_kernel)          reads the field, writes solved spectra: 2F
                                                 (the tridiagonal solve runs in its epilogue;
-                                                timed as the inversion, less the inverse pass
-                                                and the step output that vd_qg1l_pv2h adds)
+                                                no call runs it alone, so its time is derived:
+                                                the inversion, less the inverse pass and the
+                                                step output that vd_qg1l_pv2h adds; null where
+                                                the difference is not positive)
       dst-inv (dst_tc_inv_kernel)                spectra -> SSH: 2F
       dst-inv-adj (dst_tc_inv_kernel)            spectra + addend -> masked PV adjoint: 3F
 
-    With the CUDA-core engine dst-fwd (dst_gemm_kernel) and tridiag
-    (tridiag_chunked_kernel, spectra in place: 2F) are launches of their own.
+    Where the plan's inversion does not fuse the solve for this grid and batch
+    (one launch more), and with the CUDA-core engine, dst-fwd (dst_tc_fwd_kernel
+    or dst_gemm_kernel, 2F) and tridiag (tridiag_chunked_kernel, spectra in
+    place: 2F) are rows of their own.
     Per RK2 step of an evaluation with the stored trajectory: 2 stages,
     4 forward / 2 inverse / 2 inverse-adjoint passes, 4 tridiagonal solves
     and the two adjoint stages; ``recompute`` (checkpointed forms) runs the
@@ -334,7 +338,10 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / reps * 1e3
 
-    for name in (("dst-fwd", "tridiag") if tc else ("dst-fwd-solve",)):
+    n0 = L.vd_launch_count()
+    calls["dst-fwd-solve"][0]()
+    fused = tc and L.vd_launch_count() - n0 == 3     # the forward pass with the solve, the inverse, the output
+    for name in (("dst-fwd", "tridiag") if fused else ("dst-fwd-solve",)):
         del calls[name]
     rows = []
     fwd_extra = {"stage": 2 * nstep, "dst-fwd": 2 * nstep, "tridiag": 2 * nstep, "dst-fwd-solve": 2 * nstep,
@@ -345,11 +352,13 @@ def kernel_table(plan, B, nstep, recompute=False, reps=30):
         us = timed(fn)
         rows.append({"name": name, "kernel": kern, "us": us, "launches_per_eval": per_eval,
                      "algorithmic_bytes": nF * F, "gbs": nF * F / (us * 1e-6) / 1e9})
-    if tc:   # the inversion is the fused forward pass, the inverse pass and the step output
+    if fused:
         r = {x["name"]: x for x in rows}
         f = r["dst-fwd-solve"]
-        f["us"] = max(f["us"] - r["dst-inv"]["us"] - timed(output), 1e-3)
-        f["gbs"] = f["algorithmic_bytes"] / (f["us"] * 1e-6) / 1e9
+        us = f["us"] - r["dst-inv"]["us"] - timed(output)
+        f["derived"] = True
+        f["us"] = us if us > 0 else None
+        f["gbs"] = f["algorithmic_bytes"] / (us * 1e-6) / 1e9 if us > 0 else None
     return rows
 
 
@@ -360,6 +369,8 @@ def roofline_from_table(rows, ms_eval, B, n, peaks):
     hbm_peak = peaks.get("hbm_gbs", 6800.0)
     per = {}
     for r in rows:
+        if r["us"] is None:
+            continue
         k = per.setdefault(r["kernel"], {"kernel": r["kernel"], "time_us": 0.0, "launches": 0, "bytes": 0.0,
                                          "forms": []})
         k["time_us"] += r["us"] * r["launches_per_eval"]

@@ -54,10 +54,12 @@ struct vd_basis_plan {
     int ny = 0, nx = 0, dtype = VD_F32, geographic = 0, host_only = 0;
     int ncomp = 0, ntime = 0;
     long long nbasis = 0;
-    int R = 0;          // lattice rows over all components
-    int KX = 0, KY = 0; // ELL widths of the x and y tables
+    int R = 0;          // lattice rows over all groups
+    int KX = 0;         // ELL width of the x table
     int ngrp = 0;       // groups of components on the same space lattice
     int NA = 0;         // max active time centres per (time, component)
+    int gzT = 1;        // blocks along a row's centres of the transposed x pass
+    bool longY = false, longYT = false;   // y lists of eight entries and more
     std::vector<HostComp> comps;
     std::vector<double> times;
     // time weights [ntime][ncomp][NA]
@@ -66,10 +68,10 @@ struct vd_basis_plan {
     // device tables (one allocation)
     void* dev = nullptr;
     // pointers into dev
-    const int32_t *row_grp, *row_pat, *row_n, *fx_i, *fy_j, *ty_ptr, *ty_row, *tx_ptr, *tx_col,
-        *pat_cbase, *grp_rowoff, *grp_ptr, *grp_comp, *d_tact_n, *d_tact_it;
-    const long long *row_cb, *comp_boff, *comp_Nx;
-    const void *fx_w, *fy_w, *ty_w, *tx_w, *d_tact_g;
+    const int32_t *row_grp, *row_pat, *row_n, *row_lg, *fx_i, *xr, *yl_ptr, *yl_row, *ty_ptr, *ty_row, *tx_ptr,
+        *tx_col, *pat_cbase, *te_ptr;
+    const long long *row_cb, *te_off;
+    const void *fx_w, *yl_w, *ty_w, *tx_w, *te_w;
     const int8_t* land;
 };
 
@@ -77,11 +79,11 @@ namespace vd {
 
 template <typename T>
 struct BasisDev {
-    int ny, nx, R, KX, KY, NA, ncomp, ngrp;
-    const int32_t *row_grp, *row_pat, *row_n, *fx_i, *fy_j, *ty_ptr, *ty_row, *tx_ptr, *tx_col,
-        *pat_cbase, *grp_rowoff, *grp_ptr, *grp_comp, *tact_n, *tact_it;
-    const long long *row_cb, *comp_boff, *comp_Nx;
-    const T *fx_w, *fy_w, *ty_w, *tx_w, *tact_g;
+    int ny, nx, R, KX, ngrp;
+    const int32_t *row_grp, *row_pat, *row_n, *row_lg, *fx_i, *xr, *yl_ptr, *yl_row, *ty_ptr, *ty_row, *tx_ptr,
+        *tx_col, *pat_cbase, *te_ptr;
+    const long long *row_cb, *te_off;
+    const T *fx_w, *yl_w, *ty_w, *tx_w, *te_w;
     const int8_t* land;
 };
 
@@ -89,15 +91,13 @@ template <typename T>
 BasisDev<T> dev_view(const vd_basis_plan* p)
 {
     BasisDev<T> d;
-    d.ny = p->ny; d.nx = p->nx; d.R = p->R; d.KX = p->KX; d.KY = p->KY; d.NA = p->NA;
-    d.ncomp = p->ncomp; d.ngrp = p->ngrp; d.grp_ptr = p->grp_ptr; d.grp_comp = p->grp_comp;
-    d.row_grp = p->row_grp; d.row_pat = p->row_pat; d.row_n = p->row_n;
-    d.fx_i = p->fx_i; d.fy_j = p->fy_j; d.ty_ptr = p->ty_ptr; d.ty_row = p->ty_row;
-    d.tx_ptr = p->tx_ptr; d.tx_col = p->tx_col; d.pat_cbase = p->pat_cbase;
-    d.grp_rowoff = p->grp_rowoff; d.tact_n = p->d_tact_n; d.tact_it = p->d_tact_it;
-    d.row_cb = p->row_cb; d.comp_boff = p->comp_boff; d.comp_Nx = p->comp_Nx;
-    d.fx_w = (const T*)p->fx_w; d.fy_w = (const T*)p->fy_w; d.ty_w = (const T*)p->ty_w;
-    d.tx_w = (const T*)p->tx_w; d.tact_g = (const T*)p->d_tact_g;
+    d.ny = p->ny; d.nx = p->nx; d.R = p->R; d.KX = p->KX; d.ngrp = p->ngrp;
+    d.row_grp = p->row_grp; d.row_pat = p->row_pat; d.row_n = p->row_n; d.row_lg = p->row_lg;
+    d.fx_i = p->fx_i; d.xr = p->xr; d.yl_ptr = p->yl_ptr; d.yl_row = p->yl_row; d.ty_ptr = p->ty_ptr;
+    d.ty_row = p->ty_row; d.tx_ptr = p->tx_ptr; d.tx_col = p->tx_col; d.pat_cbase = p->pat_cbase;
+    d.te_ptr = p->te_ptr; d.row_cb = p->row_cb; d.te_off = p->te_off;
+    d.fx_w = (const T*)p->fx_w; d.yl_w = (const T*)p->yl_w; d.ty_w = (const T*)p->ty_w;
+    d.tx_w = (const T*)p->tx_w; d.te_w = (const T*)p->te_w;
     d.land = p->land;
     return d;
 }
@@ -105,171 +105,222 @@ BasisDev<T> dev_view(const vd_basis_plan* p)
 // Components on the same space lattice (equal sigma_D and facns: the usual set of
 // time scales per space scale) form a group: their coefficients are summed over
 // the active time centres of all of them before the x pass, and G^T's space
-// products are formed once. Rows, y tables and the workspace are per group.
+// products are formed once. Rows, y tables and the workspace are per group; the
+// active (component, time centre) entries of a basis time are one list per group.
+//
+// The passes are bound by load latency (the fields stay in L2), so every list is
+// read eight entries at a time: the index loads (the same for all threads) and then
+// the field loads of a batch are in flight together.
+template <typename T, int U, typename F>
+__device__ __forceinline__ void list_batch(T& acc, int e, int e1, const int32_t* __restrict__ idx,
+                                           const T* __restrict__ w, F&& load)
+{
+    int j[U];
+    T c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const bool on = e + u < e1;
+        j[u] = on ? __ldg(idx + e + u) : -1;
+        c[u] = on ? __ldg(w + e + u) : T(0);
+    }
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = j[u] >= 0 ? load(j[u]) : T(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc += c[u] * v[u];
+}
+// LONG: lists of eight entries and more on average; short ones do with fewer registers
+// (more warps an SM). The rest of a list is padded to four entries in float32; in
+// float64, bound by the FP64 pipe, it is taken as 4 + 2 + 1.
+template <typename T, bool LONG, typename F>
+__device__ __forceinline__ T list_sum(int e, int e1, const int32_t* __restrict__ idx, const T* __restrict__ w, F&& load)
+{
+    T acc = T(0);
+    if constexpr (LONG)
+        for (; e1 - e >= 8; e += 8) list_batch<T, 8>(acc, e, e1, idx, w, load);
+    if constexpr (sizeof(T) == 4) {
+        for (; e < e1; e += 4) list_batch<T, 4>(acc, e, e1, idx, w, load);
+    } else {
+        for (; e1 - e >= 4; e += 4) list_batch<T, 4>(acc, e, e1, idx, w, load);
+        if (e1 - e >= 2) {
+            list_batch<T, 2>(acc, e, e1, idx, w, load);
+            e += 2;
+        }
+        if (e < e1) list_batch<T, 1>(acc, e, e1, idx, w, load);
+    }
+    return acc;
+}
 
 // x pass of G: one thread per (group row r, column x, window b). The block first
-// sums the row's coefficients over (component, time centre) into shared memory,
-// warps taking every fourth entry, 64 centres at a time.
-constexpr int BX_ENT = 128, BX_Z = 64;
+// sums over the group's entries the coefficients of the centres that its columns
+// reach (xr), warps taking every fourth entry, 128 centres at a time. float32, 9
+// components in 3 groups at 1024^2 3.9 us (7.8 a component at a time); 8 windows of
+// 512^2, centres 5.3 km apart on 5 km columns, 22 us (32, and 107 with the sums of whole
+// rows of centres in every block).
+constexpr int BX_NT = 128, BX_Z = 128;
 
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(BX_NT)
 k_basis_xpass(BasisDev<T> d, int k, const T* __restrict__ X, long long ldX, T* __restrict__ Tw)
 {
-    __shared__ long long eo[BX_ENT];
-    __shared__ T eg[BX_ENT], zp[4][BX_Z], zs[BX_Z];
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ T zp[4][BX_Z];
+    const int x = blockIdx.x * BX_NT + threadIdx.x;
     const int r = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = d.row_grp[r], m0 = d.grp_ptr[g], nf = (d.grp_ptr[g + 1] - m0) * d.NA;
+    const int pat = d.row_pat[r], g = d.row_grp[r];
+    const int lo = d.xr[2 * (pat * gridDim.x + blockIdx.x)], hi = d.xr[2 * (pat * gridDim.x + blockIdx.x) + 1];
+    const int f1 = d.te_ptr[k * d.ngrp + g + 1], f0 = d.te_ptr[k * d.ngrp + g];
     const T* Xr = X + (long long)b * ldX + d.row_cb[r];
-    const int nc = d.row_n[r];
-    const long long e0 = x < d.nx ? ((long long)d.row_pat[r] * d.nx + x) * d.KX : 0;
+    const long long e0 = x < d.nx ? ((long long)pat * d.nx + x) * d.KX : 0;
     T acc = T(0);
-    for (int i0 = 0; i0 < nc; i0 += BX_Z) {
-        T z0 = T(0), z1 = T(0);
-        const bool v0 = i0 + lane < nc, v1 = i0 + 32 + lane < nc;
-        for (int f0 = 0; f0 < nf; f0 += BX_ENT) {
-            const int n = min(BX_ENT, nf - f0);
-            __syncthreads();
-            for (int e = threadIdx.x; e < n; e += blockDim.x) {
-                const int c = d.grp_comp[m0 + (f0 + e) / d.NA], a = (f0 + e) % d.NA;
-                const bool on = a < d.tact_n[k * d.ncomp + c];
-                const int ta = (k * d.ncomp + c) * d.NA + a;
-                eo[e] = on ? d.comp_boff[c] + (long long)d.tact_it[ta] * d.comp_Nx[c] : -1;
-                eg[e] = on ? d.tact_g[ta] : T(0);
-            }
-            __syncthreads();
+    for (int i0 = lo; i0 < hi; i0 += BX_Z) {
+        T z[BX_Z / 32] = {};
 #pragma unroll 4
-            for (int e = warp; e < n; e += 4) {
-                if (eo[e] < 0) continue;
-                const T* p = Xr + eo[e] + i0 + lane;
-                if (v0) z0 += eg[e] * p[0];
-                if (v1) z1 += eg[e] * p[32];
-            }
+        for (int f = f0 + warp; f < f1; f += 4) {
+            const T* p = Xr + __ldg(d.te_off + f) + i0 + lane;
+            const T w = __ldg(d.te_w + f);
+#pragma unroll
+            for (int u = 0; u < BX_Z / 32; ++u)
+                if (i0 + 32 * u + lane < hi) z[u] += w * p[32 * u];
         }
-        zp[warp][lane] = z0;
-        zp[warp][lane + 32] = z1;
+        if (i0 > lo) __syncthreads();
+#pragma unroll
+        for (int u = 0; u < BX_Z / 32; ++u) zp[warp][32 * u + lane] = z[u];
         __syncthreads();
-        if (threadIdx.x < BX_Z) zs[threadIdx.x] = (zp[0][threadIdx.x] + zp[1][threadIdx.x]) +
-                                                  (zp[2][threadIdx.x] + zp[3][threadIdx.x]);
-        __syncthreads();
+        auto sum = [&](int i) { return (zp[0][i] + zp[1][i]) + (zp[2][i] + zp[3][i]); };
+        if constexpr (sizeof(T) == 8) {          // once a centre: an FP64 addition costs more than a barrier
+            zp[0][threadIdx.x] = sum(threadIdx.x);
+            __syncthreads();
+        }
         if (x < d.nx)
             for (int e = 0; e < d.KX; ++e) {
-                const int i = d.fx_i[e0 + e];
-                if (i < 0) break;
-                if (i >= i0 && i < i0 + BX_Z) acc += d.fx_w[e0 + e] * zs[i - i0];
+                const int i = d.fx_i[e0 + e] - i0;
+                if (i + i0 < 0) break;
+                if (i >= 0 && i < BX_Z) acc += d.fx_w[e0 + e] * (sizeof(T) == 8 ? zp[0][i] : sum(i));
             }
     }
     if (x < d.nx) Tw[((long long)b * d.R + r) * d.nx + x] = acc;
 }
 
-// (row offset, weight) entries staged in shared memory, a block of them at a
-// time: a thread's field loads then depend on no index load and eight of them
-// are in flight. The passes are bound by that latency (the fields stay in L2).
-// 9 components in 3 groups at 1024^2, float32: y pass 27.9 -> 10.1 us, transposed
-// y pass 15.5 -> 10.3, transposed x pass 24.6 -> 9.1 (one thread a centre before).
-constexpr int BS_ENT = 128;
-
-// y pass of G: one thread per (y, x, b), summing every group in order.
-template <typename T>
-__global__ void __launch_bounds__(128)
+// y pass of G: one thread per (y, x, b), summing every group in order. 9 components at
+// 1024^2 in float32 10.7 us (40 with a loop per component; 11.8 with the list staged in
+// shared memory, whose barriers cost short lists 8 %).
+template <typename T, bool LONG>
+__global__ void __launch_bounds__(BX_NT)
 k_basis_ypass(BasisDev<T> d, const T* __restrict__ Tw, T* __restrict__ phi, int accumulate)
 {
-    __shared__ int off_s[BS_ENT];
-    __shared__ T w_s[BS_ENT];
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x = blockIdx.x * BX_NT + threadIdx.x;
     const int y = blockIdx.y, b = blockIdx.z;
-    const T* Tb = Tw + (long long)b * d.R * d.nx + x;
-    T acc = T(0);
-    for (int f0 = 0; f0 < d.ngrp * d.KY; f0 += BS_ENT) {
-        const int n = min(BS_ENT, d.ngrp * d.KY - f0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < n; e += blockDim.x) {
-            const int c = (f0 + e) / d.KY;
-            const long long o = ((long long)c * d.ny + y) * d.KY + (f0 + e) % d.KY;
-            const int j = d.fy_j[o];                 // < 0 behind a group's last entry
-            off_s[e] = j < 0 ? -1 : d.grp_rowoff[c] + j;
-            w_s[e] = j < 0 ? T(0) : d.fy_w[o];
-        }
-        __syncthreads();
-        if (x < d.nx) {
-#pragma unroll 8
-            for (int e = 0; e < n; ++e) {
-                const int j = off_s[e];
-                const T v = j < 0 ? T(0) : Tb[(long long)j * d.nx];
-                acc += w_s[e] * v;
-            }
-        }
-    }
     if (x >= d.nx) return;
+    const T* Tb = Tw + (long long)b * d.R * d.nx + x;
+    T acc = list_sum<T, LONG>(d.yl_ptr[y], d.yl_ptr[y + 1], d.yl_row, d.yl_w, [&](int j) { return Tb[(long long)j * d.nx]; });
     const long long o = ((long long)b * d.ny + y) * d.nx + x;
     if (d.land && d.land[(long long)y * d.nx + x]) acc = T(0);
     phi[o] = accumulate ? phi[o] + acc : acc;
 }
 
-// y pass of G^T: one thread per (lattice row r, x, b).
-template <typename T>
-__global__ void __launch_bounds__(128)
+// y pass of G^T: U[r][x] = sum_y wy adphi (land masked out). LONG: the block stages the
+// list in shared memory, 128 entries at a time (two loads less an entry and thread: 9
+// components at 1024^2 8.4 us for 11.8; with 8 entries 6.8 for 7.6 at 8 x 512^2, with 3
+// entries 14.5 for 11.0, so that short lists are read directly).
+template <typename T, bool LONG>
+__global__ void __launch_bounds__(BX_NT)
 k_basisT_ypass(BasisDev<T> d, const T* __restrict__ adphi, T* __restrict__ Uw)
 {
-    __shared__ int y_s[BS_ENT];
-    __shared__ T w_s[BS_ENT];
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x = blockIdx.x * BX_NT + threadIdx.x;
     const int r = blockIdx.y, b = blockIdx.z;
     const T* a = adphi + (long long)b * d.ny * d.nx + x;
     const int8_t* land = d.land ? d.land + x : nullptr;
-    const int e1 = d.ty_ptr[r + 1];
+    const int e0 = d.ty_ptr[r], e1 = d.ty_ptr[r + 1];
     T acc = T(0);
-    for (int e0 = d.ty_ptr[r]; e0 < e1; e0 += BS_ENT) {
-        const int n = min(BS_ENT, e1 - e0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < n; e += blockDim.x) {
-            y_s[e] = d.ty_row[e0 + e];
-            w_s[e] = d.ty_w[e0 + e];
-        }
-        __syncthreads();
-        if (x < d.nx) {
-            if (land) {
+    if constexpr (LONG) {
+        __shared__ int y_s[BX_NT];
+        __shared__ T w_s[BX_NT];
+        for (int e = e0; e < e1; e += BX_NT) {
+            const int n = min(BX_NT, e1 - e);
+            __syncthreads();
+            if (threadIdx.x < n) {
+                y_s[threadIdx.x] = d.ty_row[e + threadIdx.x];
+                w_s[threadIdx.x] = d.ty_w[e + threadIdx.x];
+            }
+            __syncthreads();
+            if (x < d.nx) {
+                if (land) {
 #pragma unroll 8
-                for (int e = 0; e < n; ++e) {
-                    const long long o = (long long)y_s[e] * d.nx;
-                    const T v = a[o];
-                    acc += w_s[e] * (land[o] ? T(0) : v);
+                    for (int u = 0; u < n; ++u) {
+                        const long long o = (long long)y_s[u] * d.nx;
+                        const T v = a[o];
+                        acc += w_s[u] * (land[o] ? T(0) : v);
+                    }
+                } else {
+#pragma unroll 8
+                    for (int u = 0; u < n; ++u) acc += w_s[u] * a[(long long)y_s[u] * d.nx];
                 }
-            } else {
-#pragma unroll 8
-                for (int e = 0; e < n; ++e) acc += w_s[e] * a[(long long)y_s[e] * d.nx];
             }
         }
+        if (x >= d.nx) return;
+    } else {
+        if (x >= d.nx) return;
+        if (land)
+            acc = list_sum<T, false>(e0, e1, d.ty_row, d.ty_w, [&](int y) {
+                const long long o = (long long)y * d.nx;
+                const T v = a[o];
+                return land[o] ? T(0) : v;
+            });
+        else
+            acc = list_sum<T, false>(e0, e1, d.ty_row, d.ty_w, [&](int y) { return a[(long long)y * d.nx]; });
     }
-    if (x < d.nx) Uw[((long long)b * d.R + r) * d.nx + x] = acc;
+    Uw[((long long)b * d.R + r) * d.nx + x] = acc;
 }
 
-// x pass of G^T: one CTA per (group row r, window b), one warp per centre
-// (lanes over its columns, which are consecutive), lanes over the time centres
-// of the group's components.
+// x pass of G^T. A block forms the space products of a run of centres of row r, each
+// by 2^lg lanes over the centre's consecutive columns (up to eight a lane), and adds
+// them to the coefficients of every entry, centres along the lanes. With a warp a centre
+// everywhere the few columns of a fine lattice left its lanes idle and its additions
+// were scattered: 8 x 512^2, centres 5.3 km apart on 5 km columns, 315 us, here 24; 9
+// components at 1024^2 9.2 us, here 5.7.
+__host__ __device__ constexpr int bxT_centres(int lg) { return lg < 4 ? BX_NT >> lg : 8; }   // of a block
+
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(BX_NT)
 k_basisT_xpass(BasisDev<T> d, int k, const T* __restrict__ Uw, T* __restrict__ adX, long long ldX)
 {
-    const int r = blockIdx.x, b = blockIdx.y;
-    const int g = d.row_grp[r], m0 = d.grp_ptr[g], nf = (d.grp_ptr[g + 1] - m0) * d.NA;
+    __shared__ T ss[BX_NT];
+    const int r = blockIdx.x, b = blockIdx.y, lg = d.row_lg[r], nc = bxT_centres(lg);
+    const int i0 = blockIdx.z * nc, n = min(nc, d.row_n[r] - i0);
+    if (n <= 0) return;
+    const int g = d.row_grp[r], f0 = d.te_ptr[k * d.ngrp + g], f1 = d.te_ptr[k * d.ngrp + g + 1];
     const T* U = Uw + ((long long)b * d.R + r) * d.nx;
-    T* A = adX + (long long)b * ldX + d.row_cb[r];
-    const int base = d.pat_cbase[d.row_pat[r]];
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int i = blockIdx.z * nw + (threadIdx.x >> 5); i < d.row_n[r]; i += nw * gridDim.z) {
+    T* A = adX + (long long)b * ldX + d.row_cb[r] + i0;
+    const int base = d.pat_cbase[d.row_pat[r]] + i0;
+    const int lanes = 1 << lg, lane = threadIdx.x & (lanes - 1);
+    for (int i = threadIdx.x >> lg; i < nc; i += BX_NT >> lg) {
         T s = T(0);
-        for (int e = d.tx_ptr[base + i] + lane; e < d.tx_ptr[base + i + 1]; e += 32) s += d.tx_w[e] * U[d.tx_col[e]];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        for (int f = lane; f < nf; f += 32) {
-            const int c = d.grp_comp[m0 + f / d.NA], a = f % d.NA;
-            if (a >= d.tact_n[k * d.ncomp + c]) continue;
-            const int ta = (k * d.ncomp + c) * d.NA + a;
-            const long long o = d.comp_boff[c] + (long long)d.tact_it[ta] * d.comp_Nx[c] + i;
-            A[o] += d.tact_g[ta] * s;
+        if (i < n) {
+            const int e1 = d.tx_ptr[base + i + 1];
+#pragma unroll 4
+            for (int e = d.tx_ptr[base + i] + lane; e < e1; e += lanes) s += d.tx_w[e] * U[d.tx_col[e]];
         }
+        for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) ss[i] = s;
+    }
+    __syncthreads();
+    const int i = threadIdx.x & (nc - 1), step = lg < 4 ? 1 << lg : BX_NT / 8;      // = BX_NT / nc
+    if (i >= n) return;
+    A += i;
+    const T s = ss[i];
+    for (int f = f0 + threadIdx.x / nc; f < f1; f += 4 * step) {     // four loads in flight
+        T* o[4];
+        T v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (f + u * step < f1) {
+                o[u] = A + __ldg(d.te_off + f + u * step);
+                v[u] = *o[u] + __ldg(d.te_w + f + u * step) * s;
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (f + u * step < f1) *o[u] = v[u];
     }
 }
 
@@ -278,10 +329,10 @@ k_basisT_xpass(BasisDev<T> d, int k, const T* __restrict__ Uw, T* __restrict__ a
 namespace {
 
 struct Tables {
-    std::vector<int32_t> row_grp, row_pat, row_n, fx_i, fy_j, ty_ptr, ty_row, tx_ptr, tx_col, pat_cbase,
-        grp_rowoff, grp_ptr, grp_comp;
-    std::vector<long long> row_cb, comp_boff, comp_Nx;
-    std::vector<double> fx_w, fy_w, ty_w, tx_w;
+    std::vector<int32_t> row_grp, row_pat, row_n, row_lg, fx_i, xr, yl_ptr, yl_row, ty_ptr, ty_row, tx_ptr, tx_col,
+        pat_cbase, te_ptr;
+    std::vector<long long> row_cb, te_off;
+    std::vector<double> fx_w, yl_w, ty_w, tx_w, te_w;
 };
 
 // Lattice, time weights and banded tables of every component.
@@ -311,7 +362,7 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
 
     long long boff = 0;
     int rowoff = 0;
-    std::vector<int> leads, lead_of;      // leading component of every group / of every component
+    std::vector<int> leads, lead_of, grp_row0;   // leading component of every group / component; first rows
     p->comps.resize(p->ncomp);
     for (int c = 0; c < p->ncomp; ++c) {
         HostComp& hc = p->comps[c];
@@ -342,7 +393,7 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
             if (p->comps[q2].p.sigma_D == q.sigma_D && p->comps[q2].p.facns == q.facns) { lead = q2; break; }
         if (lead == c) {
             leads.push_back(c);
-            tb.grp_rowoff.push_back(rowoff);
+            grp_row0.push_back(rowoff);
             rowoff += (int)hc.rows_lat.size();
         }
         lead_of.push_back(lead);
@@ -392,20 +443,13 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
         hc.enst = np_arange(-q.sigma_T * (1 - 1. / q.facnlt), (TMAX - TMIN) + 1.5 * q.sigma_T / q.facnlt,
                             q.sigma_T / q.facnlt);
         boff += (long long)hc.enst.size() * hc.Nx;
-        tb.comp_boff.push_back(hc.boff);
-        tb.comp_Nx.push_back(hc.Nx);
     }
     p->nbasis = boff;
     p->R = rowoff;
     p->ngrp = (int)leads.size();
-    for (int l : leads) {
-        tb.grp_ptr.push_back((int32_t)tb.grp_comp.size());
-        for (int c = 0; c < p->ncomp; ++c)
-            if (lead_of[c] == l) tb.grp_comp.push_back(c);
-    }
-    tb.grp_ptr.push_back((int32_t)tb.grp_comp.size());
 
-    // x tables (ELL per pattern column, CSR per pattern centre)
+    // x tables (ELL per pattern column, the centres that a block of columns reaches,
+    // CSR per pattern centre)
     int KX = 1;
     for (auto& pc : pat_cols)
         for (auto& col : pc) KX = std::max(KX, (int)col.size());
@@ -419,7 +463,14 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
         std::vector<std::vector<std::pair<int, double>>> by_centre((size_t)pat_n[pt]);
         for (int x = 0; x < nx; ++x) {
             const auto& col = pat_cols[pt][x];
+            if (x % vd::BX_NT == 0) {
+                tb.xr.push_back(INT32_MAX);
+                tb.xr.push_back(0);
+            }
+            int32_t *lo = &tb.xr[tb.xr.size() - 2], *hi = lo + 1;
             for (size_t e = 0; e < col.size(); ++e) {
+                *lo = std::min<int32_t>(*lo, col[e].first);
+                *hi = std::max<int32_t>(*hi, col[e].first + 1);
                 tb.fx_i[((size_t)pt * nx + x) * KX + e] = col[e].first;
                 tb.fx_w[((size_t)pt * nx + x) * KX + e] = col[e].second;
                 by_centre[col[e].first].push_back({x, col[e].second});
@@ -434,9 +485,18 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
         }
     }
 
-    // y tables (ELL per group and grid row, CSR per lattice row)
+    // lanes a centre in the transposed x pass: up to eight columns each
+    for (size_t r = 0; r < tb.row_pat.size(); ++r) {
+        const int pt = tb.row_pat[r], n = tb.row_n[r], cb = tb.pat_cbase[pt];
+        const int cols = n ? (tb.tx_ptr[cb + n] - tb.tx_ptr[cb]) / n : 0;
+        int lg = 0;
+        while (lg < 5 && (8 << lg) < cols) ++lg;
+        tb.row_lg.push_back(lg);
+        p->gzT = std::max(p->gzT, (n + vd::bxT_centres(lg) - 1) / vd::bxT_centres(lg));
+    }
+
+    // y tables (CSR per grid row over all groups, CSR per lattice row)
     std::vector<std::vector<std::vector<std::pair<int, double>>>> ycols((size_t)p->ngrp);
-    int KY = 1;
     for (int c = 0; c < p->ngrp; ++c) {
         const HostComp& hc = p->comps[leads[c]];
         ycols[c].resize((size_t)ny);
@@ -445,22 +505,25 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
                 const double yy = (yc[y] - hc.rows_lat[j]) / k;
                 if (std::fabs(yy) <= hc.p.sigma_D) ycols[c][y].push_back({j, mywindow(yy / hc.p.sigma_D)});
             }
-        for (auto& l : ycols[c]) KY = std::max(KY, (int)l.size());
     }
-    p->KY = KY;
-    tb.fy_j.assign((size_t)p->ngrp * ny * KY, -1);
-    tb.fy_w.assign((size_t)p->ngrp * ny * KY, 0.0);
+    for (int y = 0; y < ny; ++y) {
+        tb.yl_ptr.push_back((int32_t)tb.yl_row.size());
+        for (int c = 0; c < p->ngrp; ++c)
+            for (const auto& e : ycols[c][y]) {
+                tb.yl_row.push_back(grp_row0[c] + e.first);
+                tb.yl_w.push_back(e.second);
+            }
+    }
+    tb.yl_ptr.push_back((int32_t)tb.yl_row.size());
+    p->longY = tb.yl_row.size() >= 8 * (size_t)ny;
+    p->longYT = tb.yl_row.size() >= 8 * (size_t)p->R;
     tb.ty_ptr.push_back(0);
     for (int c = 0; c < p->ngrp; ++c) {
         const int nr = (int)p->comps[leads[c]].rows_lat.size();
         std::vector<std::vector<std::pair<int, double>>> by_row((size_t)nr);
         for (int y = 0; y < ny; ++y) {
             const auto& l = ycols[c][y];
-            for (size_t e = 0; e < l.size(); ++e) {
-                tb.fy_j[((size_t)c * ny + y) * KY + e] = l[e].first;
-                tb.fy_w[((size_t)c * ny + y) * KY + e] = l[e].second;
-                by_row[l[e].first].push_back({y, l[e].second});
-            }
+            for (size_t e = 0; e < l.size(); ++e) by_row[l[e].first].push_back({y, l[e].second});
         }
         for (auto& lst : by_row) {
             for (auto& pr : lst) {
@@ -503,6 +566,18 @@ int build_host(vd_basis_plan* p, const vd_basis_grid* g, const vd_gauss3d_params
             p->tact_g[s * NA + a] = act[s][a].second;
         }
     }
+    // the active entries of (basis time, group): offset of the time centre in X, weight
+    for (int kt = 0; kt < p->ntime; ++kt)
+        for (int l : leads) {
+            tb.te_ptr.push_back((int32_t)tb.te_off.size());
+            for (int c = 0; c < p->ncomp; ++c)
+                if (lead_of[c] == l)
+                    for (const auto& a : act[(size_t)kt * p->ncomp + c]) {
+                        tb.te_off.push_back(p->comps[c].boff + (long long)a.first * p->comps[c].Nx);
+                        tb.te_w.push_back(a.second);
+                    }
+        }
+    tb.te_ptr.push_back((int32_t)tb.te_off.size());
     return VD_OK;
 }
 
@@ -511,14 +586,12 @@ int upload(vd_basis_plan* p, const Tables& tb, const int8_t* land_host)
 {
     Packer pk;
     const size_t o_row_grp = pk.add(tb.row_grp), o_row_pat = pk.add(tb.row_pat), o_row_n = pk.add(tb.row_n),
-                 o_fx_i = pk.add(tb.fx_i), o_fy_j = pk.add(tb.fy_j), o_ty_ptr = pk.add(tb.ty_ptr),
+                 o_row_lg = pk.add(tb.row_lg), o_fx_i = pk.add(tb.fx_i), o_xr = pk.add(tb.xr),
+                 o_yl_ptr = pk.add(tb.yl_ptr), o_yl_row = pk.add(tb.yl_row), o_ty_ptr = pk.add(tb.ty_ptr),
                  o_ty_row = pk.add(tb.ty_row), o_tx_ptr = pk.add(tb.tx_ptr), o_tx_col = pk.add(tb.tx_col),
-                 o_pat_cbase = pk.add(tb.pat_cbase), o_grp_rowoff = pk.add(tb.grp_rowoff),
-                 o_grp_ptr = pk.add(tb.grp_ptr), o_grp_comp = pk.add(tb.grp_comp),
-                 o_tact_n = pk.add(p->tact_n), o_tact_it = pk.add(p->tact_it), o_row_cb = pk.add(tb.row_cb),
-                 o_comp_boff = pk.add(tb.comp_boff), o_comp_Nx = pk.add(tb.comp_Nx),
-                 o_fx_w = pk.add_as<T>(tb.fx_w), o_fy_w = pk.add_as<T>(tb.fy_w), o_ty_w = pk.add_as<T>(tb.ty_w),
-                 o_tx_w = pk.add_as<T>(tb.tx_w), o_tact_g = pk.add_as<T>(p->tact_g);
+                 o_pat_cbase = pk.add(tb.pat_cbase), o_te_ptr = pk.add(tb.te_ptr), o_row_cb = pk.add(tb.row_cb),
+                 o_te_off = pk.add(tb.te_off), o_fx_w = pk.add_as<T>(tb.fx_w), o_yl_w = pk.add_as<T>(tb.yl_w),
+                 o_ty_w = pk.add_as<T>(tb.ty_w), o_tx_w = pk.add_as<T>(tb.tx_w), o_te_w = pk.add_as<T>(tb.te_w);
     size_t o_land = 0;
     bool any_land = false;
     std::vector<int8_t> land;
@@ -533,26 +606,24 @@ int upload(vd_basis_plan* p, const Tables& tb, const int8_t* land_host)
     p->row_grp = (const int32_t*)(b + o_row_grp);
     p->row_pat = (const int32_t*)(b + o_row_pat);
     p->row_n = (const int32_t*)(b + o_row_n);
+    p->row_lg = (const int32_t*)(b + o_row_lg);
     p->fx_i = (const int32_t*)(b + o_fx_i);
-    p->fy_j = (const int32_t*)(b + o_fy_j);
+    p->xr = (const int32_t*)(b + o_xr);
+    p->yl_ptr = (const int32_t*)(b + o_yl_ptr);
+    p->yl_row = (const int32_t*)(b + o_yl_row);
     p->ty_ptr = (const int32_t*)(b + o_ty_ptr);
     p->ty_row = (const int32_t*)(b + o_ty_row);
     p->tx_ptr = (const int32_t*)(b + o_tx_ptr);
     p->tx_col = (const int32_t*)(b + o_tx_col);
     p->pat_cbase = (const int32_t*)(b + o_pat_cbase);
-    p->grp_rowoff = (const int32_t*)(b + o_grp_rowoff);
-    p->grp_ptr = (const int32_t*)(b + o_grp_ptr);
-    p->grp_comp = (const int32_t*)(b + o_grp_comp);
-    p->d_tact_n = (const int32_t*)(b + o_tact_n);
-    p->d_tact_it = (const int32_t*)(b + o_tact_it);
+    p->te_ptr = (const int32_t*)(b + o_te_ptr);
     p->row_cb = (const long long*)(b + o_row_cb);
-    p->comp_boff = (const long long*)(b + o_comp_boff);
-    p->comp_Nx = (const long long*)(b + o_comp_Nx);
+    p->te_off = (const long long*)(b + o_te_off);
     p->fx_w = b + o_fx_w;
-    p->fy_w = b + o_fy_w;
+    p->yl_w = b + o_yl_w;
     p->ty_w = b + o_ty_w;
     p->tx_w = b + o_tx_w;
-    p->d_tact_g = b + o_tact_g;
+    p->te_w = b + o_te_w;
     p->land = any_land ? (const int8_t*)(b + o_land) : nullptr;
     return VD_OK;
 }
@@ -655,10 +726,11 @@ int project(const vd_basis_plan* p, int B, int k, const T* X, long long ldX, T* 
             cudaStream_t st)
 {
     const vd::BasisDev<T> d = vd::dev_view<T>(p);
-    const unsigned gx = (unsigned)((p->nx + 127) / 128);
-    vd::k_basis_xpass<T><<<dim3(gx, p->R, B), 128, 0, st>>>(d, k, X, ldX, ws);
+    const unsigned gx = (unsigned)((p->nx + vd::BX_NT - 1) / vd::BX_NT);
+    vd::k_basis_xpass<T><<<dim3(gx, p->R, B), vd::BX_NT, 0, st>>>(d, k, X, ldX, ws);
     VD_LAUNCH_CHECK();
-    vd::k_basis_ypass<T><<<dim3(gx, p->ny, B), 128, 0, st>>>(d, ws, phi, acc);
+    if (p->longY) vd::k_basis_ypass<T, true><<<dim3(gx, p->ny, B), vd::BX_NT, 0, st>>>(d, ws, phi, acc);
+    else vd::k_basis_ypass<T, false><<<dim3(gx, p->ny, B), vd::BX_NT, 0, st>>>(d, ws, phi, acc);
     VD_LAUNCH_CHECK();
     return VD_OK;
 }
@@ -668,10 +740,11 @@ int project_T(const vd_basis_plan* p, int B, int k, const T* adphi, T* adX, long
               cudaStream_t st)
 {
     const vd::BasisDev<T> d = vd::dev_view<T>(p);
-    const unsigned gx = (unsigned)((p->nx + 127) / 128);
-    vd::k_basisT_ypass<T><<<dim3(gx, p->R, B), 128, 0, st>>>(d, adphi, ws);
+    const unsigned gx = (unsigned)((p->nx + vd::BX_NT - 1) / vd::BX_NT);
+    if (p->longYT) vd::k_basisT_ypass<T, true><<<dim3(gx, p->R, B), vd::BX_NT, 0, st>>>(d, adphi, ws);
+    else vd::k_basisT_ypass<T, false><<<dim3(gx, p->R, B), vd::BX_NT, 0, st>>>(d, adphi, ws);
     VD_LAUNCH_CHECK();
-    vd::k_basisT_xpass<T><<<dim3(p->R, B, 4), 128, 0, st>>>(d, k, ws, adX, ldX);
+    vd::k_basisT_xpass<T><<<dim3(p->R, B, p->gzT), vd::BX_NT, 0, st>>>(d, k, ws, adX, ldX);
     VD_LAUNCH_CHECK();
     return VD_OK;
 }

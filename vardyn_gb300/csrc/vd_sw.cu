@@ -556,6 +556,26 @@ __global__ void k_sw_diag(Tab<T> t, Tri<R> x, W om, W kp, W ht)
     else ht.at(ob * t.sh)(ui, sclamp(hr + hl, t.hmin * ar, t.sharp));
 }
 
+// The vorticity-grid point of a thread: rows of 32 x 8 blocks in float32; in float64 128
+// consecutive points of the whole grid a block. The FP64 pipe sets the pace there (a block
+// of 256 threads saturates its SM: 38 us alone, 77 two, 115 three), so the points are cut
+// into equal blocks without idle lanes at the ends of rows, small enough to spread evenly:
+// a tendency of 16 x 16 cells 38 -> 24 us, 48 x 40 x 3 41 -> 25, 256 x 200 76 -> 55, 16
+// members of 64^2 115 -> 75, 2 of 256^2 x 3 351 -> 338.
+constexpr int TEND64_NT = 128;
+template <typename T>
+__device__ __forceinline__ void sw_point(const Tab<T>& t, int& i, int& j)
+{
+    if constexpr (sizeof(T) == 8) {
+        const int q = blockIdx.x * blockDim.x + threadIdx.x, n1 = t.ny + 1;
+        i = q / n1;
+        j = q - i * n1;
+    } else {
+        j = blockIdx.x * blockDim.x + threadIdx.x;
+        i = blockIdx.y * blockDim.y + threadIdx.y;
+    }
+}
+
 // ------------------------------------------------------------------ k_sw_tend
 // The six cells of a face between cells o and o + s (cell c of 0..last is the
 // first of them): a cell outside the grid is read by no reconstruction (the 4-
@@ -581,8 +601,8 @@ template <typename T, typename S, typename R, typename W>
 __global__ void k_sw_tend(Tab<T> t, Tri<R> x, R om_, R kp_, R ht_, const T* taux, const T* tauy, W tu, W tv, W fx,
                           W fy)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    sw_point(t, i, j);
     const int nx = t.nx, ny = t.ny, nl = t.nl;
     if (i > nx || j > ny) return;
     const long long ob = blockIdx.z;
@@ -2385,6 +2405,18 @@ static Launch lgrid(const vd_sw_plan* p, int z)
     return L;
 }
 
+// launch of k_sw_tend: one thread a point (sw_point)
+template <typename T>
+static Launch tgrid(const vd_sw_plan* p, int z)
+{
+    Launch L = lgrid(p, z);
+    if (sizeof(T) == 8) {
+        L.block = dim3(TEND64_NT, 1, 1);
+        L.grid = dim3((unsigned)(((long long)(p->nx + 1) * (p->ny + 1) + TEND64_NT - 1) / TEND64_NT), 1, (unsigned)z);
+    }
+    return L;
+}
+
 // blocks and attributes of k_sw_tend_adj
 template <typename T>
 static cudaError_t adj_attr()
@@ -2472,10 +2504,10 @@ template <typename T>
 static int tend_fwd(vd_sw_plan* p, int B, Fields<T> cur, Work<T>& wk, const T* taux, const T* tauy, cudaStream_t st)
 {
     Tab<T>& t = tab<T>(p);
-    const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl);
+    const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl), Lt = tgrid<T>(p, B * p->nl);
     k_sw_diag<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(cur), w(wk.om), w(wk.kp), w(wk.ht));
     VD_LAUNCH_CHECK();
-    k_sw_tend<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(cur), r<T>(wk.om), r<T>(wk.kp), r<T>(wk.ht), taux, tauy,
+    k_sw_tend<T, T><<<Lt.grid, Lt.block, 0, st>>>(t, rt(cur), r<T>(wk.om), r<T>(wk.kp), r<T>(wk.ht), taux, tauy,
                                                    w(wk.tuvh.u), w(wk.tuvh.v), w(wk.fx), w(wk.fy));
     VD_LAUNCH_CHECK();
     if (p->bf) {
@@ -2500,12 +2532,12 @@ static int tend_tgl(vd_sw_plan* p, int B, Fields<T> cur, Fields<T> dcur, Work<T>
                     const T* tauy, cudaStream_t st)
 {
     Tab<T>& t = tab<T>(p);
-    const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl);
+    const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl), Lt = tgrid<T>(p, B * p->nl);
     using S = DN<T, 1>;
     k_sw_diag<T, S><<<Ll.grid, Ll.block, 0, st>>>(t, rtd(cur, dcur), WD<T>{wk.om, dk.om}, WD<T>{wk.kp, dk.kp},
                                                    WD<T>{wk.ht, dk.ht});
     VD_LAUNCH_CHECK();
-    k_sw_tend<T, S><<<Ll.grid, Ll.block, 0, st>>>(
+    k_sw_tend<T, S><<<Lt.grid, Lt.block, 0, st>>>(
         t, rtd(cur, dcur), RD<T>{wk.om, dk.om}, RD<T>{wk.kp, dk.kp}, RD<T>{wk.ht, dk.ht}, taux, tauy,
         WD<T>{wk.tuvh.u, dk.tuvh.u}, WD<T>{wk.tuvh.v, dk.tuvh.v}, WD<T>{wk.fx, dk.fx}, WD<T>{wk.fy, dk.fy});
     VD_LAUNCH_CHECK();
@@ -2734,7 +2766,7 @@ static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> a
                    T* adom, T* adkp, T* adht, const UpdAdj<T>& next, const T* taux, const T* tauy, cudaStream_t st)
 {
     Tab<T>& t = tab<T>(p);
-    const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl);
+    const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl), Lt = tgrid<T>(p, B * p->nl);
     if (!have_diag) {
         k_sw_diag<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(x), w(wk.om), w(wk.kp), w(wk.ht));
         VD_LAUNCH_CHECK();
@@ -2743,7 +2775,7 @@ static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> a
     if (p->bf) {
         // the filter's transpose first: it needs the pre-filter tendencies of
         // x, and leaves the cotangents of those tendencies in wk.bau / wk.bav
-        k_sw_tend<T, T><<<Ll.grid, Ll.block, 0, st>>>(t, rt(x), r<T>(wk.om), r<T>(wk.kp), r<T>(wk.ht), taux, tauy,
+        k_sw_tend<T, T><<<Lt.grid, Lt.block, 0, st>>>(t, rt(x), r<T>(wk.om), r<T>(wk.kp), r<T>(wk.ht), taux, tauy,
                                                        w(wk.tuvh.u), w(wk.tuvh.v), w(wk.fx), w(wk.fy));
         VD_LAUNCH_CHECK();
         k_bf_adw<T><<<Ld.grid, Ld.block, 0, st>>>(t, adk.u, adk.v, wk.bf);

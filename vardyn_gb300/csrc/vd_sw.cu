@@ -18,9 +18,9 @@
 // The kernels are templates over the arithmetic type: T for the forward,
 // a one-direction dual number for the tangent-linear (jax.jvp of step,
 // sw.py:906-922). The adjoint (jax.vjp, 924-938) recomputes each step from
-// its stored start and runs hand-written transposes, without atomics: a tile
-// kernel forms the local gradient of every face's WENO flux and gathers what
-// reaches its points (k_sw_tend_adj), then k_sw_diag_adj transposes the
+// its stored start and runs hand-written transposes, without atomics: the local
+// gradient of every face's WENO flux is formed and what reaches a point gathered
+// (k_sw_tend_adj, in float64 two kernels), then k_sw_diag_adj transposes the
 // diagnostics. max(u, 0) takes derivative 1/2 at u = 0, the
 // rule of jax's lax.max.
 #include "vd_internal.cuh"
@@ -984,52 +984,183 @@ __global__ void k_sw_update_adj(Tab<T> t, UpdAdj<T> n, int nf, Fields<T> ad)
 // h_wind table cotangents and by the mass-consistent forcing adjoint.
 template <typename T> __device__ __forceinline__ void aadd(T* p, T v) { atomicAdd(p, v); }
 
-// Adjoint of k_sw_tend and of the divergence / diffusion part of k_sw_update,
-// without atomics: one block owns a tile of ADJ_TI x ADJ_TJ targets of every kind
-// (vorticity, h, u, v) and forms, in four passes, the local gradients of the faces
-// whose stencils reach its targets: u faces' vorticity fluxes (reaching along y),
-// v faces' (along x), and the two thickness fluxes. A pass leaves a face's six
-// cotangents a * dF/dq_k and its velocity term in shared memory, then every target
-// sums those that reach it in a fixed order, so the sums are the same on every run.
-// A pass's halo is 5 faces along its own stencil alone: 20 % more faces than
-// targets at 24 x 32. The sums used to go through memory between two kernels (33
-// values a point written and read again, 620 MB a stage at 3 x 1024 x 768
-// float32): 206 + 169 us; here 245 us, bound by issue and by how many warps
-// cover the faces' loads: tiles of 16 rows with 3, 4 and 5 blocks an SM 322, 257 and
-// 253 us, 24 rows 303, 249 and 241 (48 registers, 10 of them spilled once). The
-// H / h_wind table cotangents (only when registered) accumulate with atomics over
-// the batch, each face in the block that owns it.
+// ---- pieces of the adjoint of k_sw_tend and of the divergence / diffusion part of
+// k_sw_update. Fields are slabs (a layer of one member).
+
+// Cotangents of an interior u (v) face's vorticity flux: ws[k] to the six vorticity
+// points of its stencil, g to each of the four v (u) faces that its velocity averages.
+// a: the face's masked tendency cotangent. (All loads stand before the branch on a: one
+// wait instead of two.)
+template <typename T>
+__device__ __forceinline__ void adj_face_wu(const Tab<T>& t, const T* v, const T* om, int i, int j, T a, T* ws, T& g)
+{
+    const int ny = t.ny, n1 = ny + 1, ui = i * ny + j, vi = i * n1 + j, fl = t.fu[ui];
+    auto Vv = [&](int k) { return v[k] * t.idyv2[k]; };
+    const T Vm = T(0.25) * (Vv(vi + 1) + Vv(vi) + Vv(vi - n1 + 1) + Vv(vi - n1));
+    T q[6], gv;
+    ring6(q, R1<T>{om}, vi, 1, j - 2, ny);
+    if (a != T(0)) {
+        weno_flux_adj<T>(q, Vm, (fl >> 4) & 7, j >= 1 && j <= ny - 2, j >= 2 && j <= ny - 3, a, ws, gv);
+        g = T(0.25) * a * (gv + t.fsu[ui]);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void adj_face_wv(const Tab<T>& t, const T* u, const T* om, int i, int j, T a, T* ws, T& g)
+{
+    const int nx = t.nx, ny = t.ny, n1 = ny + 1, ui = i * ny + j, vi = i * n1 + j, fl = t.fv[vi];
+    auto Uu = [&](int k) { return u[k] * t.idxu2[k]; };
+    const T Um = T(0.25) * (Uu(ui + ny) + Uu(ui + ny - 1) + Uu(ui) + Uu(ui - 1));
+    T q[6], gv;
+    ring6(q, R1<T>{om}, vi, n1, i - 2, nx);
+    if (a != T(0)) {
+        weno_flux_adj<T>(q, Um, (fl >> 4) & 7, i >= 1 && i <= nx - 2, i >= 2 && i <= nx - 3, -a, ws, gv);
+        g = -T(0.25) * a * (gv + t.fsv[vi]);
+    }
+}
+
+// Cotangents of the thickness flux through an interior u (v) face: hs[k] to the six cells,
+// g to the face's own velocity. aF: the flux's cotangent.
+template <typename T>
+__device__ __forceinline__ void adj_face_hu(const Tab<T>& t, const T* u, const T* ht, int i, int j, T aF, T* hs, T& g)
+{
+    const int nx = t.nx, ny = t.ny, ui = i * ny + j, fl = t.fu[ui];
+    const T iu2 = t.idxu2[ui];
+    const T Uf = u[ui] * iu2;
+    T q[6], gv;
+    ring6(q, R1<T>{ht}, ui - ny, ny, i - 3, nx - 1);
+    if (aF != T(0)) {
+        weno_flux_adj<T>(q, Uf, (fl >> 1) & 7, i >= 2 && i <= nx - 2, i >= 3 && i <= nx - 3, aF, hs, gv);
+        g = aF * gv * iu2;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void adj_face_hv(const Tab<T>& t, const T* v, const T* ht, int i, int j, T aF, T* hs, T& g)
+{
+    const int ny = t.ny, vi = i * (ny + 1) + j, fl = t.fv[vi];
+    const T iv2 = t.idyv2[vi];
+    const T Vf = v[vi] * iv2;
+    T q[6], gv;
+    ring6(q, R1<T>{ht}, i * ny + j - 1, 1, j - 3, ny - 1);
+    if (aF != T(0)) {
+        weno_flux_adj<T>(q, Vf, (fl >> 1) & 7, j >= 2 && j <= ny - 2, j >= 3 && j <= ny - 3, aF, hs, gv);
+        g = aF * gv * iv2;
+    }
+}
+
+// Reference pressure gradient and wind factor cotangents of an interior face (only where
+// registered; atomics over the batch).
+template <typename T>
+__device__ __forceinline__ void adj_tab_u(const Tab<T>& t, int l, int ui, T a, const T* taux)
+{
+    if (a == T(0)) return;
+    if (t.ad_dxp && t.hxy_dxp) aadd(&t.ad_dxp[(long long)l * (t.nx - 1) * t.ny + ui - t.ny], -a);
+    if (t.ad_wfu && l == 0) aadd(&t.ad_wfu[ui], a * (taux ? taux : t.taux)[ui - t.ny]);
+}
+template <typename T>
+__device__ __forceinline__ void adj_tab_v(const Tab<T>& t, int l, int i, int j, T a, const T* tauy)
+{
+    if (a == T(0)) return;
+    const int pk = i * (t.ny - 1) + j - 1;
+    if (t.ad_dyp && t.hxy_dyp) aadd(&t.ad_dyp[(long long)l * t.nx * (t.ny - 1) + pk], -a);
+    if (t.ad_wfv && l == 0) aadd(&t.ad_wfv[i * (t.ny + 1) + j], a * (tauy ? tauy : t.tauy)[pk]);
+}
+
+// What reaches a point through the viscosity stencils of the u (v) faces and the diffusion
+// stencil of the cells around it: (p+-1, c), (p, c+-1) clamped to the grid, and (p, c).
+// a(di, dj): the masked cotangent of the face or cell (i + di, j + dj), 0 where it has none.
+template <typename T, typename F>
+__device__ __forceinline__ T adj_visc_u(const Tab<T>& t, int i, int j, F&& a)
+{
+    const int nx = t.nx, ny = t.ny, ui = i * ny + j;
+    auto C = [&](int di, int dj) { return t.dxu[ui + di * ny + dj] * a(di, dj); };
+    // the faces p = 0 and nx, whose a is 0, contribute nothing
+    const T ix2 = t.idxu2[ui], iy2 = t.idyu2[ui];
+    T w = -T(2) * ix2 - T(2) * iy2, c = T(0);
+    if (i >= 1) c += C(-1, 0) * t.idxu2[ui - ny];
+    if (i + 1 <= nx) c += C(1, 0) * t.idxu2[ui + ny];
+    if (j >= 1) c += C(0, -1) * t.idyu2[ui - 1];
+    else w += iy2;
+    if (j + 1 <= ny - 1) c += C(0, 1) * t.idyu2[ui + 1];
+    else w += iy2;
+    c += C(0, 0) * w;
+    return t.visc * t.idxu[ui] * c;
+}
+template <typename T, typename F>
+__device__ __forceinline__ T adj_visc_v(const Tab<T>& t, int i, int j, F&& a)
+{
+    const int nx = t.nx, ny = t.ny, n1 = ny + 1, vi = i * n1 + j;
+    auto C = [&](int di, int dj) { return t.dyv[vi + di * n1 + dj] * a(di, dj); };
+    const T ix2 = t.idxv2[vi], iy2 = t.idyv2[vi];
+    T w = -T(2) * ix2 - T(2) * iy2, c = T(0);
+    if (i >= 1) c += C(-1, 0) * t.idxv2[vi - n1];
+    else w += ix2;
+    if (i + 1 <= nx - 1) c += C(1, 0) * t.idxv2[vi + n1];
+    else w += ix2;
+    if (j >= 1) c += C(0, -1) * t.idyv2[vi - 1];
+    if (j + 1 <= ny) c += C(0, 1) * t.idyv2[vi + 1];
+    c += C(0, 0) * w;
+    return t.visc * t.idyv[vi] * c;
+}
+template <typename T, typename F>
+__device__ __forceinline__ T adj_diff_h(const Tab<T>& t, int i, int j, F&& a)
+{
+    const int nx = t.nx, ny = t.ny, hi = i * ny + j;
+    auto D = [&](int di, int dj) { return a(di, dj) * t.area[hi + di * ny + dj]; };
+    const T ix2 = t.idx2h[hi], iy2 = t.idy2h[hi];
+    T w = -T(2) * ix2 - T(2) * iy2, s = T(0);
+    if (i >= 1) s += D(-1, 0) * t.idx2h[hi - ny];
+    else w += ix2;
+    if (i + 1 <= nx - 1) s += D(1, 0) * t.idx2h[hi + ny];
+    else w += ix2;
+    if (j >= 1) s += D(0, -1) * t.idy2h[hi - 1];
+    else w += iy2;
+    if (j + 1 <= ny - 1) s += D(0, 1) * t.idy2h[hi + 1];
+    else w += iy2;
+    s += D(0, 0) * w;
+    return t.diff * t.iarea[hi] * s;
+}
+
+// The adjoint in float32, without atomics: one block owns a tile of ADJ_TI x ADJ_TJ
+// targets of every kind (vorticity, h, u, v) and forms, in four passes, the local
+// gradients of the faces whose stencils reach its targets: u faces' vorticity fluxes
+// (reaching along y), v faces' (along x), and the two thickness fluxes. A pass leaves a
+// face's six cotangents a * dF/dq_k and its velocity term in shared memory, then every
+// target sums those that reach it in a fixed order, so the sums are the same on every run.
+// A pass's halo is 5 faces along its own stencil alone: 20 % more faces than targets at
+// 24 x 32. Through memory between two kernels (33 values a point written and read again,
+// 620 MB a stage at 3 x 1024 x 768): 206 + 169 us; here 245 us, bound by issue and by how
+// many warps cover the faces' loads: tiles of 16 rows with 3, 4 and 5 blocks an SM 322, 257
+// and 253 us, 24 rows 303, 249 and 241 (48 registers, 10 of them spilled once). The H /
+// h_wind table cotangents (only when registered) accumulate with atomics over the batch,
+// each face in the block that owns it.
+// (float64, bound by the FP64 pipe, where each halo face costs and a tile is long: two
+// kernels, below.)
 #ifdef __CUDACC__
 constexpr int ADJ_NT = 256;
 #else
 constexpr int ADJ_NT = 1;   // host build: one thread runs a block's loops, pass by pass
 #endif
-constexpr int ADJ_TJ = 32;
-// float64 is bound by the FP64 pipe, where each halo face costs: 32 rows (17 % halo)
-// and 98 KB of shared memory a block (4.87 ms; 8 rows, 44 % halo, 5.77; the two
-// kernels 4.83); float32 24 rows and 38 KB
-template <typename T> constexpr int adj_ti = sizeof(T) == 4 ? 24 : 32;
-template <typename T> constexpr int adj_nf =   // faces of the largest pass
-    (adj_ti<T> + 5) * (ADJ_TJ + 1) > (adj_ti<T> + 1) * (ADJ_TJ + 5) ? (adj_ti<T> + 5) * (ADJ_TJ + 1)
-                                                                    : (adj_ti<T> + 1) * (ADJ_TJ + 5);
-template <typename T> constexpr int adj_smem =   // elements of shared memory
-    2 * (adj_ti<T> + 2) * (ADJ_TJ + 2) + (adj_ti<T> + 6) * (ADJ_TJ + 6) + 7 * adj_nf<T>;
+constexpr int ADJ_TI = 24, ADJ_TJ = 32;
+constexpr int ADJ_NF =   // faces of the largest pass
+    (ADJ_TI + 5) * (ADJ_TJ + 1) > (ADJ_TI + 1) * (ADJ_TJ + 5) ? (ADJ_TI + 5) * (ADJ_TJ + 1)
+                                                              : (ADJ_TI + 1) * (ADJ_TJ + 5);
+constexpr int ADJ_SMEM =   // elements of shared memory (38 KB)
+    2 * (ADJ_TI + 2) * (ADJ_TJ + 2) + (ADJ_TI + 6) * (ADJ_TJ + 6) + 7 * ADJ_NF;
 
 template <typename T>
-__global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(Tab<T> t, const T* u, const T* v, const T* om, const T* ht,
-                                                        const T* adk_u, const T* adk_v, const T* adk_h, T* adom,
-                                                        T* adkp, T* adht, T* adu, T* adv, T* adh, const T* taux,
-                                                        const T* tauy)
+__global__ void __launch_bounds__(ADJ_NT, 5)
+k_sw_tend_adj(Tab<T> t, const T* u, const T* v, const T* om, const T* ht, const T* adk_u, const T* adk_v,
+              const T* adk_h, T* adom, T* adkp, T* adht, T* adu, T* adv, T* adh, const T* taux, const T* tauy)
 {
-    constexpr int TI = adj_ti<T>, TJ = ADJ_TJ, RPT = TI * TJ / ADJ_NT;
+    constexpr int TI = ADJ_TI, TJ = ADJ_TJ, RPT = TI * TJ / ADJ_NT;
     constexpr int AC = TJ + 2, HC = TJ + 6;           // row lengths of the tiles of a and of the masked h cotangent
     constexpr int CA = TJ + 5, CB = TJ + 1;           // row lengths of passes A (u faces, omega), B (v faces, omega)
-    constexpr int NF = adj_nf<T>;
+    constexpr int NF = ADJ_NF;
 #ifdef __CUDACC__
     extern __shared__ __align__(16) unsigned char adj_pool[];
     T* const s_au = (T*)adj_pool;
 #else
-    T s_au[adj_smem<T>];
+    T s_au[ADJ_SMEM];
 #endif
     T* const s_av = s_au + (TI + 2) * AC;
     T* const s_hm = s_av + (TI + 2) * AC;
@@ -1076,23 +1207,10 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
 #pragma unroll
         for (int k = 0; k < 6; ++k) ws[k] = T(0);
         if (i >= 1 && i <= nx - 1 && j >= 0 && j < ny) {
-            const int ui = i * ny + j, vi = i * n1 + j;
-            const int fl = t.fu[ui];
-            // (all loads before the branch on a: one wait instead of two)
-            const T a = adk_u[ui] * ((fl & 1) ? T(1) : T(0));
-            auto Vv = [&](int k) { return v[k] * t.idyv2[k]; };
-            const T Vm = T(0.25) * (Vv(vi + 1) + Vv(vi) + Vv(vi - n1 + 1) + Vv(vi - n1));
-            T q[6], gv;
-            ring6(q, R1<T>{om}, vi, 1, j - 2, ny);
-            if (a != T(0)) {
-                weno_flux_adj<T>(q, Vm, (fl >> 4) & 7, j >= 1 && j <= ny - 2, j >= 2 && j <= ny - 3, a, ws, gv);
-                vm = T(0.25) * a * (gv + t.fsu[ui]);
-                // reference pressure gradient and wind factor (H / h_wind cotangents)
-                if (i < i0 + TI && j >= j0 && j < j0 + TJ) {
-                    if (t.ad_dxp && t.hxy_dxp) aadd(&t.ad_dxp[(long long)l * (nx - 1) * ny + ui - ny], -a);
-                    if (t.ad_wfu && l == 0) aadd(&t.ad_wfu[ui], a * (taux ? taux : t.taux)[ui - ny]);
-                }
-            }
+            const int ui = i * ny + j;
+            const T a = adk_u[ui] * ((t.fu[ui] & 1) ? T(1) : T(0));
+            adj_face_wu(t, v, om, i, j, a, ws, vm);
+            if (i < i0 + TI && j >= j0 && j < j0 + TJ) adj_tab_u(t, l, ui, a, taux);
         }
 #pragma unroll
         for (int k = 0; k < 6; ++k) S[k][e] = ws[k];
@@ -1118,22 +1236,7 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
             // KE + pressure: u faces i (-a) and i+1 (+a), v faces j (-a) and j+1 (+a)
             const int hi = i * ny + j;
             adkp[hi] = (-s_au[ea] + s_au[ea + AC]) + (-s_av[ea] + s_av[ea + 1]);
-            if (t.diff > T(0)) {
-                // the diffusion stencil of cell (p, c): (p+-1, c), (p, c+-1) clamped to the grid, and (p, c)
-                auto D = [&](int e2, int k) { return s_hm[e2] * t.area[k]; };
-                const T ix2 = t.idx2h[hi], iy2 = t.idy2h[hi];
-                T w = -T(2) * ix2 - T(2) * iy2, s = T(0);
-                if (i >= 1) s += D(eh - HC, hi - ny) * t.idx2h[hi - ny];
-                else w += ix2;
-                if (i + 1 <= nx - 1) s += D(eh + HC, hi + ny) * t.idx2h[hi + ny];
-                else w += ix2;
-                if (j >= 1) s += D(eh - 1, hi - 1) * t.idy2h[hi - 1];
-                else w += iy2;
-                if (j + 1 <= ny - 1) s += D(eh + 1, hi + 1) * t.idy2h[hi + 1];
-                else w += iy2;
-                s += D(eh, hi) * w;
-                adh[hi] += t.diff * t.iarea[hi] * s;
-            }
+            if (t.diff > T(0)) adh[hi] += adj_diff_h(t, i, j, [&](int di, int dj) { return s_hm[eh + di * HC + dj]; });
         }
     }
     __syncthreads();
@@ -1145,22 +1248,10 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
 #pragma unroll
         for (int k = 0; k < 6; ++k) ws[k] = T(0);
         if (i >= 0 && i < nx && j >= 1 && j <= ny - 1) {
-            const int ui = i * ny + j, vi = i * n1 + j;
-            const int fl = t.fv[vi];
-            const T a = adk_v[vi] * ((fl & 1) ? T(1) : T(0));
-            auto Uu = [&](int k) { return u[k] * t.idxu2[k]; };
-            const T Um = T(0.25) * (Uu(ui + ny) + Uu(ui + ny - 1) + Uu(ui) + Uu(ui - 1));
-            T q[6], gv;
-            ring6(q, R1<T>{om}, vi, n1, i - 2, nx);
-            if (a != T(0)) {
-                weno_flux_adj<T>(q, Um, (fl >> 4) & 7, i >= 1 && i <= nx - 2, i >= 2 && i <= nx - 3, -a, ws, gv);
-                um = -T(0.25) * a * (gv + t.fsv[vi]);
-                if (i >= i0 && i < i0 + TI && j < j0 + TJ) {
-                    const int pk = i * (ny - 1) + j - 1;
-                    if (t.ad_dyp && t.hxy_dyp) aadd(&t.ad_dyp[(long long)l * nx * (ny - 1) + pk], -a);
-                    if (t.ad_wfv && l == 0) aadd(&t.ad_wfv[vi], a * (tauy ? tauy : t.tauy)[pk]);
-                }
-            }
+            const int vi = i * n1 + j;
+            const T a = adk_v[vi] * ((t.fv[vi] & 1) ? T(1) : T(0));
+            adj_face_wv(t, u, om, i, j, a, ws, um);
+            if (i >= i0 && i < i0 + TI && j < j0 + TJ) adj_tab_v(t, l, i, j, a, tauy);
         }
 #pragma unroll
         for (int k = 0; k < 6; ++k) S[k][e] = ws[k];
@@ -1194,15 +1285,7 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
             T aF = T(0);
             if (i - 1 >= 1) aF -= s_hm[r * HC + c + 3];
             if (i <= nx - 2) aF += s_hm[(r + 1) * HC + c + 3];
-            const int ui = i * ny + j, fl = t.fu[ui];
-            const T iu2 = t.idxu2[ui];
-            const T Uf = u[ui] * iu2;
-            T q[6], gv;
-            ring6(q, R1<T>{ht}, ui - ny, ny, i - 3, nx - 1);
-            if (aF != T(0)) {
-                weno_flux_adj<T>(q, Uf, (fl >> 1) & 7, i >= 2 && i <= nx - 2, i >= 3 && i <= nx - 3, aF, hs, gv);
-                f = aF * gv * iu2;
-            }
+            adj_face_hu(t, u, ht, i, j, aF, hs, f);
         }
 #pragma unroll
         for (int k = 0; k < 6; ++k) S[k][e] = hs[k];
@@ -1219,21 +1302,7 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
             const int ui = i * ny + j, ea = (ti + 1) * AC + tj + 1;
             T s = a_u[q];
             if (l == nl - 1) s += -t.drag * s_au[ea];
-            if (t.visc > T(0)) {
-                // viscosity stencil of u face (p, c): (p+-1, c), (p, c+-1) with c clamped, and (p, c);
-                // the faces p = 0 and nx, whose a is 0, contribute nothing
-                auto C = [&](int e2, int k) { return t.dxu[k] * s_au[e2]; };
-                const T ix2 = t.idxu2[ui], iy2 = t.idyu2[ui];
-                T w = -T(2) * ix2 - T(2) * iy2, c = T(0);
-                if (i >= 1) c += C(ea - AC, ui - ny) * t.idxu2[ui - ny];
-                if (i + 1 <= nx) c += C(ea + AC, ui + ny) * t.idxu2[ui + ny];
-                if (j >= 1) c += C(ea - 1, ui - 1) * t.idyu2[ui - 1];
-                else w += iy2;
-                if (j + 1 <= ny - 1) c += C(ea + 1, ui + 1) * t.idyu2[ui + 1];
-                else w += iy2;
-                c += C(ea, ui) * w;
-                s += t.visc * t.idxu[ui] * c;
-            }
+            if (t.visc > T(0)) s += adj_visc_u(t, i, j, [&](int di, int dj) { return s_au[ea + di * AC + dj]; });
             s += S[6][(ti + 2) * TJ + tj];
             adu[ui] += s;
         }
@@ -1250,15 +1319,7 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
             T aF = T(0);
             if (j - 1 >= 1) aF -= s_hm[(r + 3) * HC + c];
             if (j <= ny - 2) aF += s_hm[(r + 3) * HC + c + 1];
-            const int vi = i * n1 + j, fl = t.fv[vi];
-            const T iv2 = t.idyv2[vi];
-            const T Vf = v[vi] * iv2;
-            T q[6], gv;
-            ring6(q, R1<T>{ht}, i * ny + j - 1, 1, j - 3, ny - 1);
-            if (aF != T(0)) {
-                weno_flux_adj<T>(q, Vf, (fl >> 1) & 7, j >= 2 && j <= ny - 2, j >= 3 && j <= ny - 3, aF, hs, gv);
-                f = aF * gv * iv2;
-            }
+            adj_face_hv(t, v, ht, i, j, aF, hs, f);
         }
 #pragma unroll
         for (int k = 0; k < 6; ++k) S[k][e] = hs[k];
@@ -1276,23 +1337,146 @@ __global__ void __launch_bounds__(ADJ_NT, sizeof(T) == 4 ? 5 : 2) k_sw_tend_adj(
             const int vi = i * n1 + j, ea = (ti + 1) * AC + tj + 1;
             T s = a_v[q];
             if (l == nl - 1) s += -t.drag * s_av[ea];
-            if (t.visc > T(0)) {
-                // viscosity stencil of v face (p, c): (p+-1, c) with p clamped, (p, c+-1), and (p, c)
-                auto C = [&](int e2, int k) { return t.dyv[k] * s_av[e2]; };
-                const T ix2 = t.idxv2[vi], iy2 = t.idyv2[vi];
-                T w = -T(2) * ix2 - T(2) * iy2, c = T(0);
-                if (i >= 1) c += C(ea - AC, vi - n1) * t.idxv2[vi - n1];
-                else w += ix2;
-                if (i + 1 <= nx - 1) c += C(ea + AC, vi + n1) * t.idxv2[vi + n1];
-                else w += ix2;
-                if (j >= 1) c += C(ea - 1, vi - 1) * t.idyv2[vi - 1];
-                if (j + 1 <= ny) c += C(ea + 1, vi + 1) * t.idyv2[vi + 1];
-                c += C(ea, vi) * w;
-                s += t.visc * t.idyv[vi] * c;
-            }
+            if (t.visc > T(0)) s += adj_visc_v(t, i, j, [&](int di, int dj) { return s_av[ea + di * AC + dj]; });
             s += S[6][ti * CA + tj + 2];
             adv[vi] += s;
         }
+    }
+}
+
+// The adjoint in float64: k_sw_tend_adj_src forms the gradients of every face once and
+// stores them (seven values a flux), k_sw_tend_adj_gather sums what reaches each target in
+// a fixed order. Both points' loops are cut like k_sw_tend's (sw_point). The tile form's
+// halo faces cost FP64 instructions and its long tiles leave SMs idle: a stage's adjoint
+// in tiles of 32 x 32 and here, 16 x 16 cells 156 / 46 us, 48 x 40 x 3 307 / 47, 256 x 200
+// 320 / 100, 16 members of 64^2 310 / 137, 2 of 256^2 x 3 928 / 619; the step adjoint of
+// 3 x 1024 x 768 51.5 / 46.5 ms.
+template <typename T>
+struct SwSrc {
+    T *wu, *hu;              // [7][bl][su] u faces: six terms, then the velocity's
+    T *wv, *hv;              // [7][bl][sv] v faces
+    long long nu, nv;        // bl * su, bl * sv: stride of the seven
+};
+
+template <typename T>
+__global__ void k_sw_tend_adj_src(Tab<T> t, const T* u, const T* v, const T* om, const T* ht, const T* adk_u,
+                                  const T* adk_v, const T* adk_h, SwSrc<T> S, const T* taux, const T* tauy)
+{
+    int i, j;
+    sw_point(t, i, j);
+    const int nx = t.nx, ny = t.ny, nl = t.nl, n1 = ny + 1;
+    if (i > nx || j > ny) return;
+    const long long ob = blockIdx.z;
+    const int l = (int)(blockIdx.z % (unsigned)nl);
+    const int ui = i * ny + j, vi = i * n1 + j;
+    u += ob * t.su;
+    v += ob * t.sv;
+    om += ob * t.sw;
+    ht += ob * t.sh;
+    const T* const hb = adk_h + ob * t.sh;
+    auto hm = [&](int k) { return hb[k] * ((t.fh[k] & 1) ? T(1) : T(0)); };
+    auto put = [](T* p, long long stride, const T* s, T g) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) p[k * stride] = s[k];
+        p[6 * stride] = g;
+    };
+    if (j < ny) {                                    // u face (zeros where it has no flux)
+        const long long so = ob * t.su + ui;
+        T s[6] = {}, g = T(0), s2[6] = {}, g2 = T(0);
+        if (i >= 1 && i <= nx - 1) {
+            const T a = adk_u[so] * ((t.fu[ui] & 1) ? T(1) : T(0));
+            adj_face_wu(t, v, om, i, j, a, s, g);
+            adj_tab_u(t, l, ui, a, taux);
+            // dt_h[c] = -div_x[c] * mask_h[c], no x contribution in the first and last cells
+            T aF = T(0);
+            if (i - 1 >= 1) aF -= hm(ui - ny);
+            if (i <= nx - 2) aF += hm(ui);
+            adj_face_hu(t, u, ht, i, j, aF, s2, g2);
+        }
+        put(S.wu + so, S.nu, s, g);
+        put(S.hu + so, S.nu, s2, g2);
+    }
+    if (i < nx) {                                    // v face
+        const long long so = ob * t.sv + vi;
+        T s[6] = {}, g = T(0), s2[6] = {}, g2 = T(0);
+        if (j >= 1 && j <= ny - 1) {
+            const T a = adk_v[so] * ((t.fv[vi] & 1) ? T(1) : T(0));
+            adj_face_wv(t, u, om, i, j, a, s, g);
+            adj_tab_v(t, l, i, j, a, tauy);
+            T aF = T(0);
+            if (j - 1 >= 1) aF -= hm(ui - 1);
+            if (j <= ny - 2) aF += hm(ui);
+            adj_face_hv(t, v, ht, i, j, aF, s2, g2);
+        }
+        put(S.wv + so, S.nv, s, g);
+        put(S.hv + so, S.nv, s2, g2);
+    }
+}
+
+template <typename T>
+__global__ void k_sw_tend_adj_gather(Tab<T> t, SwSrc<T> S, const T* adk_u, const T* adk_v, const T* adk_h, T* adom,
+                                     T* adkp, T* adht, T* adu, T* adv, T* adh)
+{
+    int i, j;
+    sw_point(t, i, j);
+    const int nx = t.nx, ny = t.ny, nl = t.nl, n1 = ny + 1;
+    if (i > nx || j > ny) return;
+    const long long ob = blockIdx.z;
+    const int l = (int)(blockIdx.z % (unsigned)nl);
+    const int ui = i * ny + j, vi = i * n1 + j;      // ui: also the h point
+    // term k of the u (v) face (p, c), and the masked tendency cotangents; 0 outside the grid
+    auto inu = [&](int p, int c) { return p >= 0 && p <= nx && c >= 0 && c < ny; };
+    auto inv = [&](int p, int c) { return p >= 0 && p < nx && c >= 0 && c <= ny; };
+    auto U = [&](const T* A, int k, int p, int c) {
+        return inu(p, c) ? A[k * S.nu + ob * t.su + p * ny + c] : T(0);
+    };
+    auto V = [&](const T* A, int k, int p, int c) {
+        return inv(p, c) ? A[k * S.nv + ob * t.sv + p * n1 + c] : T(0);
+    };
+    auto au = [&](int di, int dj) {
+        const int p = i + di, c = j + dj, k = p * ny + c;
+        return p >= 1 && p <= nx - 1 && c >= 0 && c < ny ? adk_u[ob * t.su + k] * ((t.fu[k] & 1) ? T(1) : T(0)) : T(0);
+    };
+    auto av = [&](int di, int dj) {
+        const int p = i + di, c = j + dj, k = p * n1 + c;
+        return p >= 0 && p < nx && c >= 1 && c <= ny - 1 ? adk_v[ob * t.sv + k] * ((t.fv[k] & 1) ? T(1) : T(0)) : T(0);
+    };
+    {   // vorticity point: u face (i, j+2-k) and v face (i+2-k, j) reach it with term k
+        T s = T(0);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += U(S.wu, k, i, j + 2 - k);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += V(S.wv, k, i + 2 - k, j);
+        adom[ob * t.sw + vi] = s;
+    }
+    if (i < nx && j < ny) {   // h point: u face (i+3-k, j) and v face (i, j+3-k) reach it with term k
+        // KE + pressure: u faces i (-a) and i+1 (+a), v faces j (-a) and j+1 (+a)
+        adkp[ob * t.sh + ui] = (-au(0, 0) + au(1, 0)) + (-av(0, 0) + av(0, 1));
+        T s = T(0);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += U(S.hu, k, i + 3 - k, j);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += V(S.hv, k, i, j + 3 - k);
+        adht[ob * t.sh + ui] = s;
+        if (t.diff > T(0))
+            adh[ob * t.sh + ui] += adj_diff_h(t, i, j, [&](int di, int dj) {
+                const int k = ui + di * ny + dj;
+                return adk_h[ob * t.sh + k] * ((t.fh[k] & 1) ? T(1) : T(0));
+            });
+    }
+    if (j < ny) {             // u face: U-average of the v faces (i-1, j), (i-1, j+1), (i, j), (i, j+1)
+        T s = (V(S.wv, 6, i - 1, j) + V(S.wv, 6, i - 1, j + 1) + V(S.wv, 6, i, j) + V(S.wv, 6, i, j + 1)) * t.idxu2[ui];
+        if (l == nl - 1) s += -t.drag * au(0, 0);
+        if (t.visc > T(0)) s += adj_visc_u(t, i, j, au);
+        s += U(S.hu, 6, i, j);
+        adu[ob * t.su + ui] += s;
+    }
+    if (i < nx) {             // v face: V-average of the u faces (i, j-1), (i, j), (i+1, j-1), (i+1, j)
+        T s = (U(S.wu, 6, i, j - 1) + U(S.wu, 6, i, j) + U(S.wu, 6, i + 1, j - 1) + U(S.wu, 6, i + 1, j)) * t.idyv2[vi];
+        if (l == nl - 1) s += -t.drag * av(0, 0);
+        if (t.visc > T(0)) s += adj_visc_v(t, i, j, av);
+        s += V(S.hv, 6, i, j);
+        adv[ob * t.sv + vi] += s;
     }
 }
 
@@ -2417,21 +2601,26 @@ static Launch tgrid(const vd_sw_plan* p, int z)
     return L;
 }
 
-// blocks and attributes of k_sw_tend_adj
-template <typename T>
-static cudaError_t adj_attr()
+static dim3 agrid(const vd_sw_plan* p, int z)   // blocks of k_sw_tend_adj
 {
-    static vd::PerDeviceOnce once;
-    return once.run([] {
-        return cudaFuncSetAttribute(k_sw_tend_adj<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(T) * adj_smem<T>));
-    });
-}
-template <typename T>
-static dim3 agrid(const vd_sw_plan* p, int z)
-{
-    return dim3((unsigned)((p->ny + 1 + ADJ_TJ - 1) / ADJ_TJ), (unsigned)((p->nx + 1 + adj_ti<T> - 1) / adj_ti<T>),
+    return dim3((unsigned)((p->ny + 1 + ADJ_TJ - 1) / ADJ_TJ), (unsigned)((p->nx + 1 + ADJ_TI - 1) / ADJ_TI),
                 (unsigned)z);
+}
+
+// The float64 tendency adjoint's stored terms (every field of the batch).
+static size_t src_elems(const Sizes& s, int B) { return 14 * (size_t)(s.su + s.sv) * B; }
+template <typename T>
+static bool take_src(Arena& ws, const Sizes& s, int B, SwSrc<T>& S)
+{
+    if (sizeof(T) == 4) return true;
+    T* b = (T*)ws.take(sizeof(T) * src_elems(s, B));
+    S.nu = s.su * B;
+    S.nv = s.sv * B;
+    S.wu = b;
+    S.hu = b + 7 * S.nu;
+    S.wv = b + 14 * S.nu;
+    S.hv = b + 14 * S.nu + 7 * S.nv;
+    return b != nullptr;
 }
 
 // One RK3-SSP run of nstep steps in model space, forward (S = T) or
@@ -2701,9 +2890,9 @@ extern "C" size_t vd_sw_workspace_bytes(const vd_sw_plan* p, int batch, int nste
     const size_t wk = (esz == 8 ? work_bytes<double>(s, batch, bfn) : work_bytes<float>(s, batch, bfn));
     // inputs (x, xb, F), their tangents / adjoints, two work sets, adjoint
     // accumulators, the vorticity and thickness of a step's first two stages,
-    // and the per-step trajectory
+    // the stored terms of the float64 tendency adjoint, and the per-step trajectory
     return 14 * F3 + 2 * wk + (size_t)nstep * F3 + esz * (s.sw + 2 * s.sh) * batch +
-           2 * esz * (s.sw + s.sh) * batch + 64 * 256;
+           2 * esz * (s.sw + s.sh) * batch + (esz == 8 ? esz * src_elems(s, batch) : 0) + 64 * 256;
 }
 
 namespace {
@@ -2763,7 +2952,8 @@ static int sw_tgl_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
 // stage combination that follows, or stage -1 for none.
 template <typename T>
 static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> adx, const Work<T>& wk, bool have_diag,
-                   T* adom, T* adkp, T* adht, const UpdAdj<T>& next, const T* taux, const T* tauy, cudaStream_t st)
+                   T* adom, T* adkp, T* adht, const SwSrc<T>& src, const UpdAdj<T>& next, const T* taux,
+                   const T* tauy, cudaStream_t st)
 {
     Tab<T>& t = tab<T>(p);
     const Launch Ld = lgrid(p, B), Ll = lgrid(p, B * p->nl), Lt = tgrid<T>(p, B * p->nl);
@@ -2790,10 +2980,17 @@ static int rhs_adj(vd_sw_plan* p, int B, Fields<T> x, Fields<T> adk, Fields<T> a
         ak.u = wk.bau;
         ak.v = wk.bav;
     }
-    VD_CUDA_TRY(adj_attr<T>());
-    k_sw_tend_adj<T><<<agrid<T>(p, B * p->nl), ADJ_NT, sizeof(T) * adj_smem<T>, st>>>(t, x.u, x.v, wk.om, wk.ht, ak.u, ak.v, ak.h, adom,
-                                                                adkp, adht, adx.u, adx.v, adx.h, taux, tauy);
-    VD_LAUNCH_CHECK();
+    if constexpr (sizeof(T) == 4) {
+        k_sw_tend_adj<T><<<agrid(p, B * p->nl), ADJ_NT, sizeof(T) * ADJ_SMEM, st>>>(
+            t, x.u, x.v, wk.om, wk.ht, ak.u, ak.v, ak.h, adom, adkp, adht, adx.u, adx.v, adx.h, taux, tauy);
+        VD_LAUNCH_CHECK();
+    } else {
+        k_sw_tend_adj_src<T><<<Lt.grid, Lt.block, 0, st>>>(t, x.u, x.v, wk.om, wk.ht, ak.u, ak.v, ak.h, src, taux, tauy);
+        VD_LAUNCH_CHECK();
+        k_sw_tend_adj_gather<T><<<Lt.grid, Lt.block, 0, st>>>(t, src, ak.u, ak.v, ak.h, adom, adkp, adht, adx.u, adx.v,
+                                                              adx.h);
+        VD_LAUNCH_CHECK();
+    }
     k_sw_diag_adj<T><<<Ll.grid, Ll.block, 0, st>>>(t, x.u, x.v, x.h, adom, adkp, adht, adx, next);
     VD_LAUNCH_CHECK();
     return VD_OK;
@@ -2829,7 +3026,9 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
         som[k] = (T*)ws.take(sizeof(T) * s.sw * B);
         sht[k] = (T*)ws.take(sizeof(T) * s.sh * B);
     }
-    if (!adom || !adkp || !adht || !som[0] || !sht[0] || !som[1] || !sht[1]) return VD_ERR_WORKSPACE;
+    SwSrc<T> src;
+    if (!adom || !adkp || !adht || !som[0] || !sht[0] || !som[1] || !sht[1] || !take_src(ws, s, B, src))
+        return VD_ERR_WORKSPACE;
     // forward sweep keeping the state at the start of every step (the last
     // step's own result is not part of the adjoint)
     traj[0] = in.x;
@@ -2899,8 +3098,8 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
             }
             // the filter's transpose forms the pre-filter tendencies again and reads KE + pressure
             const bool have = (stg < 2 || mc) && !p->bf;
-            if ((rc = rhs_adj<T>(p, B, stages[stg], adk, ad, ws2, have, adom, adkp, adht, upd(stg - 1), (const T*)taux,
-                                 (const T*)tauy, st)))
+            if ((rc = rhs_adj<T>(p, B, stages[stg], adk, ad, ws2, have, adom, adkp, adht, src, upd(stg - 1),
+                                 (const T*)taux, (const T*)tauy, st)))
                 return rc;
         }
     }
@@ -3049,9 +3248,10 @@ static int sw_rhs_adj_t(vd_sw_plan* p, int B, const void* u, const void* v, cons
     T* adom = (T*)ws.take(sizeof(T) * s.sw * B);
     T* adkp = (T*)ws.take(sizeof(T) * s.sh * B);
     T* adht = (T*)ws.take(sizeof(T) * s.sh * B);
-    if (!adom || !adkp || !adht) return VD_ERR_WORKSPACE;
+    SwSrc<T> src;
+    if (!adom || !adkp || !adht || !take_src(ws, s, B, src)) return VD_ERR_WORKSPACE;
     Fields<T> x{(T*)u, (T*)v, (T*)h}, ak{(T*)aku, (T*)akv, (T*)akh}, ad{(T*)adu, (T*)adv, (T*)adh};
-    return rhs_adj<T>(p, B, x, ak, ad, wk, false, adom, adkp, adht, UpdAdj<T>{-1}, nullptr, nullptr, st);
+    return rhs_adj<T>(p, B, x, ak, ad, wk, false, adom, adkp, adht, src, UpdAdj<T>{-1}, nullptr, nullptr, st);
 }
 
 // elementwise stage combination: k = rhs + sponge; stage 0/1 store k

@@ -507,9 +507,41 @@ tridiag_chunked_kernel(T* __restrict__ spec, const T* __restrict__ trim, int my,
         if (i < cnt) S[(long long)(j0 + i) * lds] = x[i];
 }
 
+// Rows of a piece of the float64 tridiagonal kernel with tables, and the tallest field
+// it takes (16 warps of 4 pieces, 128 registers a thread).
+constexpr int TRI_TAB_ROWS = 8, TRI_TAB_MAX = 16 * 4 * TRI_TAB_ROWS;
+
+// Those tables, from the Thomas multipliers, at plan creation (columns behind n are never
+// read): [4][my][lds] multipliers, alphas and their products within a piece, from its
+// start and from its end. A 512^2 plan takes 6.7 ms with the tables formed on the host,
+// 3.7 here.
+__global__ void tridiag_tables_kernel(const double* __restrict__ trim, double* __restrict__ tab, int my, int n, int lds,
+                                      double a)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j0 = blockIdx.y * TRI_TAB_ROWS, j1 = min(j0 + TRI_TAB_ROWS, my);
+    if (t >= n) return;
+    const long long pl = (long long)my * lds;
+    double pr = 1.0;
+    for (int j = j0; j < j1; ++j) {
+        const long long o = (long long)j * lds + t;
+        const double m = trim[o], al = -a * m;
+        tab[o] = m;
+        tab[pl + o] = al;
+        pr *= al;
+        tab[2 * pl + o] = pr;
+    }
+    pr = 1.0;
+    for (int j = j1 - 1; j >= j0; --j) {
+        const long long o = (long long)j * lds + t;
+        pr *= -a * trim[o];
+        tab[3 * pl + o] = pr;
+    }
+}
+
 // The float64 form of the chunked kernel with its data-independent products from
 // tables: alpha_j, and the products of the alphas from a piece's start to j (pf) and
-// from j to its end (pb), formed on the host in the order the sweeps form them. 5 FP64
+// from j to its end (pb), formed in the order the sweeps form them. 5 FP64
 // instructions a row instead of 10, in pieces of 8 rows: one SM quarter issues a
 // warp's FP64 instruction in 75 clocks, so a small grid's time is the instructions of
 // one warp. 4 x 256^2: 6.1 us (11.4 without the tables), one 128^2 field 4.3 us (10.9).
@@ -978,10 +1010,6 @@ size_t spec_bytes(const vd_qg1l_plan* p, int nf)
 // form (index arithmetic, barriers between stages).
 constexpr double FFT_OVER_DENSE = 1.3;
 
-// Rows of a piece of the float64 tridiagonal kernel with tables, and the tallest field
-// it takes (16 warps of 4 pieces, 128 registers a thread).
-constexpr int TRI_TAB_ROWS = 8, TRI_TAB_MAX = 16 * 4 * TRI_TAB_ROWS;
-
 template <typename T>
 static int upload(const std::vector<double>& h, void** d)
 {
@@ -1104,30 +1132,6 @@ int build_dst_tables(vd_qg1l_plan* p)
     }
     int rc;
     if (p->d.dtype == VD_F64 && (rc = build_fft_tables(t))) return rc;
-    if (p->d.dtype == VD_F64 && my <= TRI_TAB_MAX) {
-        // multipliers, alphas and their products within a piece, from its start and from its end
-        const size_t pl = trim.size();
-        std::vector<double> tab(4 * pl, 0.0);
-        for (int col = 0; col < n; ++col)
-            for (int j0 = 0; j0 < my; j0 += TRI_TAB_ROWS) {
-                const int j1 = std::min(j0 + TRI_TAB_ROWS, my);
-                double pr = 1.0;
-                for (int j = j0; j < j1; ++j) {
-                    const size_t o = size_t(j) * t.lds + col;
-                    tab[o] = trim[o];
-                    tab[pl + o] = -a * trim[o];
-                    pr *= tab[pl + o];
-                    tab[2 * pl + o] = pr;
-                }
-                pr = 1.0;
-                for (int j = j1 - 1; j >= j0; --j) {
-                    const size_t o = size_t(j) * t.lds + col;
-                    pr *= tab[pl + o];
-                    tab[3 * pl + o] = pr;
-                }
-            }
-        if ((rc = upload<double>(tab, &t.tri_tab))) return rc;
-    }
     if (p->d.dtype == VD_F32) {
         if ((rc = upload<float>(wodd, &t.Wodd))) return rc;
         if ((rc = upload<float>(woddT, &t.WoddT))) return rc;
@@ -1138,6 +1142,13 @@ int build_dst_tables(vd_qg1l_plan* p)
         if ((rc = upload<double>(woddT, &t.WoddT))) return rc;
         if ((rc = upload<double>(weven, &t.Weven))) return rc;
         if ((rc = upload<double>(trim, &t.trim))) return rc;
+        if (my <= TRI_TAB_MAX) {
+            VD_CUDA_TRY(cudaMalloc(&t.tri_tab, 4 * trim.size() * sizeof(double)));
+            tridiag_tables_kernel<<<dim3((n + 127) / 128, (my + TRI_TAB_ROWS - 1) / TRI_TAB_ROWS), 128>>>(
+                (const double*)t.trim, (double*)t.tri_tab, my, n, t.lds, a);
+            VD_LAUNCH_CHECK();
+            VD_CUDA_TRY(cudaStreamSynchronize(0));
+        }
     }
     return VD_OK;
 }

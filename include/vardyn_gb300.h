@@ -92,8 +92,9 @@ typedef struct vd_qg1l_schedule {
                             cluster) */
     int tc_group_inv;    /* the same for the inverse pass */
     int fma_rows;        /* rows per CTA of the float32 FMA pass: 0 rule, 16,
-                            32 or 64 (float64 plans accept 16 and 32 and keep
-                            their own rule) */
+                            32 or 64 as far as its tile fits shared memory
+                            (float64 plans accept 16 and 32 by the same
+                            measure of 8-byte tiles and keep their own rule) */
     int tridiag_rows;    /* rows per thread of the separate tridiagonal
                             solve: 0 rule, 8, 16 or 32 (used when the field
                             fits, else the rule); float64 fields of up to 512

@@ -3,9 +3,12 @@
 Batches of windows of uneven grid sizes (one plan per size, as the reference
 runs one assimilation per window, ``run_assimilation.py:27-349``) do not all
 run fastest with one fixed rule: whether the x-DST pass runs on the tensor
-cores or on CUDA-core FMA, how many 32-column tiles a tensor-core CTA owns,
-how many rows an FMA CTA owns and how many rows a tridiagonal thread owns
-depend on the grid and on the number of windows. ``tune(plan, batch)`` times
+cores or on CUDA-core FMA, how many rows and groups of 128 modes a tensor-core
+CTA owns, how many rows an FMA CTA owns and how many rows a tridiagonal thread
+owns depend on the grid and on the number of windows. (Where a tensor-core
+shape solves the tridiagonal systems in its epilogue, the tridiagonal choices
+are the same launches; float64 plans keep their own rule whatever the rows of
+an FMA CTA.) ``tune(plan, batch)`` times
 the PV -> SSH inversion (forward x-DST, y tridiagonal solve, inverse x-DST:
 the pass every model stage and adjoint stage runs) under each candidate
 schedule on the plan's device, outside any graph capture, keeps the fastest
@@ -25,7 +28,7 @@ _cache = {}
 def candidates(plan):
     """Schedules worth timing for this plan: the built-in rule, FMA with each
     row tile, and (float32 plans with tensor-core images) tensor cores with
-    each tile group; each with the three tridiagonal row counts and, in float32,
+    each CTA shape; each with the three tridiagonal row counts and, in float32,
     the register-capped tridiagonal kernel."""
     out = [{}]
     f32 = plan.dtype == torch.float32

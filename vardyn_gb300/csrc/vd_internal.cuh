@@ -78,8 +78,8 @@ struct DSTTables {
     double tri_a; // off-diagonal g/f/dy^2
     void* tri_tab = nullptr;   // float64: [4][my][lds] multipliers, alphas and their products within a piece
     void* tc;     // tensor-core images and tile table (float32 plans), or nullptr
-    // float64 plans whose odd extension 2(n+1) factors into 2, 3, 5: the
-    // FFT form of the transform (twiddles e^{-2 pi i m / L}, radix per stage)
+    // float64 plans whose length takes the FFT form of the transform (fft_factor):
+    // twiddles e^{-2 pi i m / L} of the odd extension L = 2(n+1), radix per stage
     void* fft_tw = nullptr;
     int fft_L = 0, fft_nst = 0;
     int fft_rad[24] = {};

@@ -981,7 +981,7 @@ __global__ void k_sw_update_adj(Tab<T> t, UpdAdj<T> n, int nf, Fields<T> ad)
 }
 
 // Atomic accumulation, used only where sums run over the batch into the H /
-// h_wind table cotangents and by the mass-consistent forcing adjoint.
+// h_wind table cotangents.
 template <typename T> __device__ __forceinline__ void aadd(T* p, T v) { atomicAdd(p, v); }
 
 // ---- pieces of the adjoint of k_sw_tend and of the divergence / diffusion part of
@@ -1541,13 +1541,10 @@ __global__ void k_sw_diag_adj(Tab<T> t, const T* u, const T* v, const T* h, cons
     }
 }
 
-// Adjoint of k_sw_force_mc (scatter to the thickness and Fh of the replicate
-// padding stencil, atomics). adn: adjoint of the output (in place: becomes the
-// adjoint of the input u, v, h direct paths).
-// Adjoint of the mass-consistent forcing (sw.py:880-898), without atomics:
-// the face terms (the cotangents the face's thickness and forcing averages
-// hand to each of their two padded cells) are recomputed where they are
-// gathered. mc_face_u / mc_face_v give them for one face from the face's
+// Adjoint of k_sw_force_mc, the mass-consistent forcing (sw.py:880-898), without
+// atomics: the face terms (the cotangents the face's thickness and forcing
+// averages hand to each of their two padded cells) are recomputed where they are
+// gathered. The adjoint of the output becomes that of the input's direct path in place. mc_face_u / mc_face_v give them for one face from the face's
 // incoming velocity cotangent.
 template <typename T>
 __device__ __forceinline__ void mc_face_u(const Tab<T>& t, const T* u, const T* h, const T* Fh, const T* adu,

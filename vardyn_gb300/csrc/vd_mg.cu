@@ -868,14 +868,20 @@ struct MgRun {
         // blocks a system: one in float32 (a phase is shorter than a cluster barrier);
         // in float64, where one SM's FP64 rate is the bound, a cluster of up to 8 while
         // the systems' clusters fit the GPU at once (15 of 8). Levels of 768 and 192 cells:
-        // 43.5 us a V-cycle with one block, 31.8 with 8, now bound by the barriers. It is the
-        // bottom's matrix (its cells squared) that gains: 17 us at 144 cells, 8 at 96, 4 at
-        // 64, and each level above loses 10 to 14 us of sweeps to the barriers. Solves with
-        // one block / 8: one level of 60 cells 332 / 256 us; 24^2 + 12^2 724 / 603, 24x16 +
-        // 12x8 451 / 561, 16^2 + 8^2 349 / 535, 32^2 + 16^2 + 8^2 906 / 1044.
+        // 43.5 us a V-cycle with one block, 31.8 with 8, now bound by the barriers. What
+        // gains is the bottom solve, by its cells squared as a matrix or an exact inverse;
+        // each level above loses 10 to 14 us of sweeps to the barriers. Solves with one
+        // block / 8, by the cells of these levels:
+        //   bottom sweeps as a matrix (up to 512 cells): 60 332 / 256 us, 384 3031 / 1901,
+        //   480 + 120 1562 / 1515, 384 + 96 1381 / 1502, 1024 + 256 + 64 1550 / 1697
+        //   bottom sweeps one by one: 672 5433 / 6248, 896 6606 / 6443
+        //   exact bottom: 288 3620 / 3626, 384 2574 / 2367, 768 + 192 1928 / 1996
         const int above = p->nlev - 1 - l0, cells = p->lv.back().n0 * p->lv.back().n1;
+        const bool wide = p->niter_bottom <= 0 ? above == 0 && cells >= 320
+                          : p->bot_sm          ? cells >= 32 + 80 * above
+                                               : cells >= 864;
         int nc = 1;
-        if (vd::mg_scaled<T> && p->bot_sm && cells >= 32 + 96 * above)
+        if (vd::mg_scaled<T> && wide)
             while (nc < 8 && (long long)p->nsys * 2 * nc <= 120) nc *= 2;
         if (nc == 1) {
             vd::k_mg_coarse<T, false><<<(unsigned)p->nsys, 1024, smem, st>>>(A);

@@ -3023,7 +3023,7 @@ static int sw_adj_t(vd_sw_plan* p, int B, const void* u0, const void* v0, const 
         som[k] = (T*)ws.take(sizeof(T) * s.sw * B);
         sht[k] = (T*)ws.take(sizeof(T) * s.sh * B);
     }
-    SwSrc<T> src;
+    SwSrc<T> src{};
     if (!adom || !adkp || !adht || !som[0] || !sht[0] || !som[1] || !sht[1] || !take_src(ws, s, B, src))
         return VD_ERR_WORKSPACE;
     // forward sweep keeping the state at the start of every step (the last
@@ -3245,7 +3245,7 @@ static int sw_rhs_adj_t(vd_sw_plan* p, int B, const void* u, const void* v, cons
     T* adom = (T*)ws.take(sizeof(T) * s.sw * B);
     T* adkp = (T*)ws.take(sizeof(T) * s.sh * B);
     T* adht = (T*)ws.take(sizeof(T) * s.sh * B);
-    SwSrc<T> src;
+    SwSrc<T> src{};
     if (!adom || !adkp || !adht || !take_src(ws, s, B, src)) return VD_ERR_WORKSPACE;
     Fields<T> x{(T*)u, (T*)v, (T*)h}, ak{(T*)aku, (T*)akv, (T*)akh}, ad{(T*)adu, (T*)adv, (T*)adh};
     return rhs_adj<T>(p, B, x, ak, ad, wk, false, adom, adkp, adht, src, UpdAdj<T>{-1}, nullptr, nullptr, st);
